@@ -22,6 +22,7 @@ namespace tri {
 namespace {
 
 constexpr int kLvThreads = 512;
+constexpr int kSortThreads = 1024;
 constexpr int kPre = 4;                          // dependencies per row prefetched into registers
 constexpr int kMerge = 8;                        // ILU(0): update pairs per batch of loads
 // Every wait ends after kWaitNs of GPU time (%globaltimer) at the latest.
@@ -158,11 +159,6 @@ __device__ __forceinline__ void wait_levels(volatile int* done, int l, int lane,
 }
 
 // ---- analysis -------------------------------------------------------------
-// column c is a dependency on another tile (c >= 0: a dependency at all)
-__device__ __forceinline__ int is_ext(int32_t c, int32_t base, int32_t m) {
-    return c >= 0 && (c < base || c >= base + m) ? 1 : 0;
-}
-
 // Per row: validate the structure (row pointers monotone and within nnz,
 // columns in range and strictly increasing), locate the diagonal, and the
 // dependency range: strictly lower part [rp[i], first column >= i) or
@@ -196,8 +192,7 @@ __global__ void k_tri_rows(int32_t n, int64_t nnz, int upper, const int32_t* __r
 }
 
 // Per tile (one block): the global level of each row -- the longest chain
-// of dependencies ending at it over the whole triangle -- and the tile's rows
-// sorted by it.  Tiles are taken by ticket in the solve's order (ascending
+// of dependencies ending at it over the whole triangle.  Tiles are taken by ticket in the solve's order (ascending
 // for a lower, descending for an upper triangle) and each waits (bounded)
 // for the previous one to publish its levels, so the levels of every
 // other-tile dependency are final when read.  In the tile: start from
@@ -205,26 +200,17 @@ __global__ void k_tri_rows(int32_t n, int64_t nnz, int upper, const int32_t* __r
 // contiguous per-thread segments walked in dependency order until a sweep
 // changes nothing (a sweep that changes something brings one more row of
 // the longest in-tile chain to its final value, so at most m + 1 sweeps).
-// Then a bitonic sort of (level, row) and a dense renumbering of the
-// distinct levels: the solve's levels of the tile, in global order.  Rows
-// of the tile then never wait on an other-tile row that is late in its own
-// tile merely because of where the tile boundary falls.
 template <bool UPPER>
 __global__ void __launch_bounds__(kLvThreads)
 k_tri_levels(int32_t n, int32_t ntiles, const int32_t* __restrict__ ci, const int32_t* __restrict__ beg,
-             const int32_t* __restrict__ cnt, const int32_t* __restrict__ dpos, int32_t* glev,
-             int4* __restrict__ desc, int4* __restrict__ dcol, int32_t* __restrict__ lvlptr,
-             int32_t* __restrict__ nlev, int32_t* __restrict__ hcount, unsigned* chain, int* err) {
+             const int32_t* __restrict__ cnt, int32_t* glev, unsigned* chain, int* err) {
     extern __shared__ __align__(16) unsigned char shraw[];
-    unsigned long long* key = reinterpret_cast<unsigned long long*>(shraw);  // kTriTile
-    volatile int* lev = reinterpret_cast<volatile int*>(key + kTriTile);      // kTriTile
-    int* ext = reinterpret_cast<int*>(key);  // aliases key until the sort
-    __shared__ int part[kLvThreads];
-    __shared__ int s_tile, s_ext;
+    volatile int* lev = reinterpret_cast<volatile int*>(shraw);  // kTriTile
+    int* ext = reinterpret_cast<int*>(shraw) + kTriTile;          // kTriTile
+    __shared__ int s_tile;
     if (threadIdx.x == 0) {
         const int tk = int(atomicAdd(chain + ntiles, 1u));
         s_tile = UPPER ? ntiles - 1 - tk : tk;
-        s_ext = 0;
     }
     __syncthreads();
     const int t = s_tile;
@@ -281,104 +267,112 @@ k_tri_levels(int32_t n, int32_t ntiles, const int32_t* __restrict__ ci, const in
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) st_release(chain + t, 1u);
+}
 
-    // sort the tile's rows by (level, row): bitonic over kTriTile keys
-    for (int r = threadIdx.x; r < kTriTile; r += blockDim.x)
-        key[r] = r < m ? (static_cast<unsigned long long>(lev[r]) << 13) | static_cast<unsigned long long>(r)
+// Per tile (one block): the tile's rows in (level, row) order -- the order in
+// which the solve takes them -- by a bitonic sort in shared memory.  For
+// position p of the tile: desc (row, first dependency, dependency count,
+// diagonal position) and dsrc, where the first four dependencies are found:
+// >= 0 the tile's own position of that row, <= -2 row -(c + 2) of another
+// tile, -1 none.  pos is the inverse (position of each row in its tile),
+// bit k of lmask[q] says that position 32 q + k starts a new level, and
+// lvlptr / nlev hold the level starts.  Levels are global, so rows of the
+// tile never wait on an other-tile row that is late in its own tile merely
+// because of where the tile boundary falls.
+__global__ void __launch_bounds__(kSortThreads)
+k_tri_sort(int32_t n, const int32_t* __restrict__ ci, const int32_t* __restrict__ beg,
+           const int32_t* __restrict__ cnt, const int32_t* __restrict__ dpos, const int32_t* __restrict__ glev,
+           int4* __restrict__ desc, int4* __restrict__ dsrc, uint16_t* __restrict__ pos, uint32_t* __restrict__ lmask,
+           int32_t* __restrict__ lvlptr, int32_t* __restrict__ nlev) {
+    extern __shared__ __align__(16) unsigned char shraw[];
+    unsigned long long* key = reinterpret_cast<unsigned long long*>(shraw);  // kTriTile
+    uint16_t* inv = reinterpret_cast<uint16_t*>(key + kTriTile);             // kTriTile
+    __shared__ int first[kTriChunks + 1];  // level starts before each chunk of 32 positions
+    const int t = blockIdx.x;
+    const int32_t base = int32_t(t) * kTriTile;
+    const int32_t m = min(kTriTile, n - base);
+    int size = 32;  // the power of two the sort runs over
+    while (size < m) size <<= 1;
+    for (int r = threadIdx.x; r < size; r += blockDim.x)
+        key[r] = r < m ? (static_cast<unsigned long long>(glev[base + r]) << 13) | static_cast<unsigned long long>(r)
                        : ~0ull;
     __syncthreads();
-    for (int k = 2; k <= kTriTile; k <<= 1)
+    for (int k = 2; k <= size; k <<= 1)
         for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < kTriTile; i += blockDim.x) {
-                const int ixj = i ^ j;
-                if (ixj > i) {
-                    const unsigned long long a = key[i], b = key[ixj];
-                    if ((a > b) == ((i & k) == 0)) {
-                        key[i] = b;
-                        key[ixj] = a;
-                    }
+            for (int q = threadIdx.x; q < size / 2; q += blockDim.x) {
+                const int i = ((q & ~(j - 1)) << 1) | (q & (j - 1)), ixj = i | j;
+                const unsigned long long a = key[i], b = key[ixj];
+                if ((a > b) == ((i & k) == 0)) {
+                    key[i] = b;
+                    key[ixj] = a;
                 }
             }
             __syncthreads();
         }
-    // dense level numbers: a new level starts where the level value changes
-    int nf = 0;
-    for (int i = s0; i < s1; ++i) nf += (i == 0 || (key[i] >> 13) != (key[i - 1] >> 13)) ? 1 : 0;
-    part[threadIdx.x] = nf;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int w = 0; w < int(blockDim.x); ++w) {
-            const int v = part[w];
-            part[w] = acc;
-            acc += v;
+    for (int p = threadIdx.x; p < m; p += blockDim.x) {
+        const int r = int(key[p] & 8191ull);
+        inv[r] = uint16_t(p);
+        pos[base + r] = uint16_t(p);
+    }
+    // level starts: one ballot per chunk, then a scan of their counts
+    const int nc = (m + 31) >> 5, lane = threadIdx.x & 31;
+    for (int c = threadIdx.x >> 5; c < kTriChunks; c += blockDim.x >> 5) {
+        const int p = 32 * c + lane;
+        const bool st = p < m && (p == 0 || (key[p] >> 13) != (key[p - 1] >> 13));
+        const uint32_t w = __ballot_sync(0xffffffffu, st);
+        if (lane == 0) {
+            if (c < nc) lmask[size_t(t) * kTriChunks + c] = w;
+            first[c] = __popc(w);
         }
-        nlev[t] = acc;
-        lvlptr[size_t(t) * (kTriTile + 1) + acc] = m;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {  // exclusive scan of the kTriChunks counts, kTriChunks / 32 per lane
+        int v[kTriChunks / 32], s = 0;
+#pragma unroll
+        for (int k = 0; k < kTriChunks / 32; ++k) {
+            v[k] = first[lane * (kTriChunks / 32) + k];
+            s += v[k];
+        }
+        int x = s;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= d) x += y;
+        }
+        int acc = x - s;
+#pragma unroll
+        for (int k = 0; k < kTriChunks / 32; ++k) {
+            first[lane * (kTriChunks / 32) + k] = acc;
+            acc += v[k];
+        }
+        if (lane == 31) first[kTriChunks] = acc;
     }
     __syncthreads();
     int32_t* lp = lvlptr + size_t(t) * (kTriTile + 1);
-    int d = part[threadIdx.x];
-    int ext_n = 0;
-    for (int i = s0; i < s1; ++i) {
-        if (i == 0 || (key[i] >> 13) != (key[i - 1] >> 13)) lp[d++] = i;
-        const int32_t row = base + int32_t(key[i] & 8191ull);
-        const int32_t b = __ldg(beg + row), c = __ldg(cnt + row);
-        desc[base + i] = make_int4(row, b, c, __ldg(dpos + row));
-        const int4 c4 = make_int4(c > 0 ? __ldg(ci + b) : -1, c > 1 ? __ldg(ci + b + 1) : -1,
-                                  c > 2 ? __ldg(ci + b + 2) : -1, c > 3 ? __ldg(ci + b + 3) : -1);
-        dcol[base + i] = c4;
-        ext_n += is_ext(c4.x, base, m) + is_ext(c4.y, base, m) + is_ext(c4.z, base, m) + is_ext(c4.w, base, m);
-    }
-    atomicAdd(&s_ext, ext_n);
-    __syncthreads();
-    if (threadIdx.x == 0) hcount[t] = s_ext;
-}
-
-// Per tile (one block): number, in level order, the tile's dependencies on
-// other tiles among each row's first kPre (the rows whose values the solve's
-// receiver warp fetches): dslot holds the slot of each such dependency (-1:
-// none, in the tile, or past kPre), hrow the row each slot is filled from.
-__global__ void __launch_bounds__(kLvThreads)
-k_tri_halo(int32_t n, const int4* __restrict__ dcol, const int32_t* __restrict__ hoff, int4* __restrict__ dslot,
-           int32_t* __restrict__ hrow) {
-    __shared__ int part[kLvThreads];
-    const int t = blockIdx.x;
-    const int32_t base = int32_t(t) * kTriTile;
-    const int32_t m = min(kTriTile, n - base);
-    const int seg = (m + blockDim.x - 1) / blockDim.x;
-    const int s0 = min(m, int(threadIdx.x) * seg), s1 = min(m, s0 + seg);
-    int cnt = 0;
-    for (int p = s0; p < s1; ++p) {
-        const int4 c4 = dcol[base + p];
-        cnt += is_ext(c4.x, base, m) + is_ext(c4.y, base, m) + is_ext(c4.z, base, m) + is_ext(c4.w, base, m);
-    }
-    part[threadIdx.x] = cnt;
-    __syncthreads();
     if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int w = 0; w < int(blockDim.x); ++w) {
-            const int v = part[w];
-            part[w] = acc;
-            acc += v;
-        }
+        nlev[t] = first[kTriChunks];
+        lp[first[kTriChunks]] = m;
     }
-    __syncthreads();
-    int slot = part[threadIdx.x];
-    int32_t* hr = hrow + hoff[t];
-    for (int p = s0; p < s1; ++p) {
-        const int4 c4 = dcol[base + p];
-        const int c[4] = {c4.x, c4.y, c4.z, c4.w};
-        int o[4];
+    for (int c = threadIdx.x >> 5; c < nc; c += blockDim.x >> 5) {
+        const int p = 32 * c + lane;
+        const bool st = p < m && (p == 0 || (key[p] >> 13) != (key[p - 1] >> 13));
+        const uint32_t w = __ballot_sync(0xffffffffu, st);
+        if (p >= m) continue;
+        if (st) lp[first[c] + __popc(w & ((1u << lane) - 1u))] = p;
+        const int32_t row = base + int32_t(key[p] & 8191ull);
+        const int32_t b = __ldg(beg + row), d = __ldg(cnt + row);
+        desc[base + p] = make_int4(row, b, d, __ldg(dpos + row));
+        int sc[kPre];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            o[k] = -1;
-            if (is_ext(c[k], base, m)) {
-                hr[slot] = c[k];
-                o[k] = slot++;
+        for (int k = 0; k < kPre; ++k) {
+            sc[k] = -1;
+            if (k < d) {
+                const int32_t j = __ldg(ci + b + k), jl = j - base;
+                // (columns outside [0, n) are reported by k_tri_rows)
+                if (j >= 0 && j < n) sc[k] = (jl >= 0 && jl < m) ? int(inv[jl]) : -(j + 2);
             }
         }
-        dslot[base + p] = make_int4(o[0], o[1], o[2], o[3]);
+        dsrc[base + p] = make_int4(sc[0], sc[1], sc[2], sc[3]);
     }
 }
 
@@ -491,308 +485,268 @@ __global__ void k_tri_fill(int32_t n, E* __restrict__ x, unsigned* ticket) {
         Pub<E>::fill(x, i);
 }
 
-// Cross-tile values come through a receiver warp: the block's last warp
-// polls the tile's other-tile dependencies (numbered in level order by the
-// analysis, kHalo<E> of them at most) from x, 128 in flight, and stores each
-// arrived value into a shared-memory slot.  The slots are pre-filled with
-// the sentinel, so -- as for x in global memory -- a slot that no longer
-// holds it holds the final value (component-wise single-copy stores), and a
-// row waits on shared memory with neither a flag nor a fence, instead of an
-// L2 round trip; the producing tile runs only a few levels ahead, so that
-// round trip would otherwise sit on the critical path of nearly every level.
-template <class E> struct kHalo { static constexpr int value = 12288; };
-template <> struct kHalo<float> { static constexpr int value = 24576; };
-template <> struct kHalo<cd> { static constexpr int value = 5632; };
-constexpr int kRecv = 8;  // slots in flight per receiver lane
+// One tile.  What bounds a solve is the chain of levels, so a tile's rows are
+// taken in level order, 32 positions (a chunk) at a time with one row per
+// lane: a warp steps through the levels its chunk spans and passes every
+// value to the next level through shared memory with a __syncwarp.  The
+// block's warps take the chunks round-robin and hand the chain on from chunk
+// to chunk through a named barrier (bar.arrive / bar.sync of the two warps: it
+// orders the shared-memory accesses, with no fence).  All that does not
+// depend on the chain a warp has done before its turn: descriptors and values
+// loaded one and two turns ahead, the values of other tiles' rows polled from
+// x, the division by the diagonal prepared.  A level costs a shared load, the
+// row's FMAs and a shared store (and, at a non-unit diagonal, a division),
+// whatever the number of rows up to 32; wider levels take several chunks.
+// Measured on B200 (f64, ILU(0) factors of the 1024^2 5-point operator, 2047
+// levels in 128 tiles): lower / upper solve 378-384 / 590-616 us, against
+// 1140 / 1320 us for levels handed round 15 warps one by one (0.22 us a level
+// in a single tile, here 0.04: 78 cycles, 180 with the division) with a
+// receiver warp for the other tiles' values; 96^3 7-point 330 / 345 against
+// 846 / 821 us.  What is left is the chain itself and, at each of the 127
+// tile boundaries, about 1.5 us for a value to go out to L2 and be polled.
+// (A solver warp fed through a shared-memory ring by the others was slower,
+// 480 / 719 us: about 500 cycles a chunk went into taking over the records.)
+// A division by the diagonal sits on the chain, so the loader prepares it:
+// the reciprocal of d to twice the working precision, y + z.  With it the
+// correctly rounded quotient takes four dependent operations: q = a y + a z,
+// which is a / d but for its last rounding, and one correction
+// q += (a - d q) y with the residual exact in an FMA, which from a q within
+// one ulp gives the rounded a / d (Markstein, Computation of elementary
+// functions on the IBM RISC System/6000 processor, 1990) as long as nothing
+// over- or underflows on the way: the diagonal's exponent within +-DivRange::d
+// (checked by the loader) and the numerator's within +-DivRange::n; otherwise the
+// plain division is taken.
+template <class R> struct DivRange;
+template <> struct DivRange<double> { static constexpr int d = 100, n = 880; };
+template <> struct DivRange<float> { static constexpr int d = 30, n = 80; };
+__device__ __forceinline__ int exponent(double v) { return ((__double2hiint(v) >> 20) & 0x7ff) - 1023; }
+__device__ __forceinline__ int exponent(float v) { return int((__float_as_uint(v) >> 23) & 0xffu) - 127; }
+template <class R>
+__device__ __forceinline__ bool within(R v, int e) { return unsigned(exponent(v) + e) <= unsigned(2 * e); }
+__device__ __forceinline__ double rcp_rn(double d) { return __drcp_rn(d); }
+__device__ __forceinline__ float rcp_rn(float d) { return __frcp_rn(d); }
+// A row's prepared diagonal: the divisor (complex: |d|^2) and its reciprocal
+// (y = 0 when the plain division has to be taken).
+template <class E> struct Prep { typename real_of<E>::type den, y, z; };
+template <class E, class R>
+__device__ __forceinline__ R div_prepared(R a, const Prep<E>& p) {
+    const R q = fma_rn(a, p.y, mul_rn(a, p.z));
+    return fma_rn(fma_rn(-p.den, q, a), p.y, q);
+}
+__device__ __forceinline__ double divisor(double d) { return d; }
+__device__ __forceinline__ float divisor(float d) { return d; }
+__device__ __forceinline__ float divisor(cf d) { return __fmaf_rn(d.re, d.re, __fmul_rn(d.im, d.im)); }
+__device__ __forceinline__ double divisor(cd d) { return __fma_rn(d.re, d.re, __dmul_rn(d.im, d.im)); }
+template <class E>
+__device__ __forceinline__ Prep<E> prepare_div(E d) {
+    using R = typename real_of<E>::type;
+    const R den = divisor(d);
+    if (!within(den, DivRange<R>::d)) return Prep<E>{den, R(0), R(0)};
+    const R y = rcp_rn(den);
+    return Prep<E>{den, y, mul_rn(fma_rn(-den, y, R(1)), y)};  // 1/d - y = (1 - d y) / d
+}
+// a / d = quot(a, d); `on`: the lane's result is used (others skip the plain division)
+template <class R>
+__device__ __forceinline__ R quot_prepared(R a, R, const Prep<R>& p, bool on) {
+    R q = div_prepared(a, p);
+    if (on && (p.y == R(0) || !within(a, DivRange<R>::n))) q = quot(a, p.den);
+    return q;
+}
+__device__ __forceinline__ cf quot_prepared(cf a, cf d, const Prep<cf>& p, bool on) {
+    const float re = __fmaf_rn(a.re, d.re, __fmul_rn(a.im, d.im)), im = __fmaf_rn(a.im, d.re, -__fmul_rn(a.re, d.im));
+    cf q{div_prepared(re, p), div_prepared(im, p)};
+    if (on && (p.y == 0.f || !within(re, DivRange<float>::n) || !within(im, DivRange<float>::n))) q = quot(a, d);
+    return q;
+}
+__device__ __forceinline__ cd quot_prepared(cd a, cd d, const Prep<cd>& p, bool on) {
+    const double re = __fma_rn(a.re, d.re, __dmul_rn(a.im, d.im)), im = __fma_rn(a.im, d.re, -__dmul_rn(a.re, d.im));
+    cd q{div_prepared(re, p), div_prepared(im, p)};
+    if (on && (p.y == 0.0 || !within(re, DivRange<double>::n) || !within(im, DivRange<double>::n))) q = quot(a, d);
+    return q;
+}
+
+constexpr int kSolveWarps = 15;  // one named barrier (1..15) behind each warp
+constexpr int kSolveThreads = 32 * kSolveWarps;
 
 template <class E>
-constexpr size_t trsv_smem() {
-    return size_t(kTriTile + kHalo<E>::value) * sizeof(E);
+struct TileValues {
+    E xs[kTriTile];                        // the tile's solution by position
+    E ext[kSolveWarps][kPre][32];          // each warp's current other-tile values
+};
+
+__device__ __forceinline__ void chunk_arrive(int w) {
+    asm volatile("bar.arrive %0, 64;" ::"r"(1 + w) : "memory");
+}
+__device__ __forceinline__ void chunk_sync(int w) {
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + w) : "memory");
 }
 
-// Shared-memory slot access, one volatile access per component.
-__device__ __forceinline__ float vload(const float* p) { return *reinterpret_cast<const volatile float*>(p); }
-__device__ __forceinline__ double vload(const double* p) { return *reinterpret_cast<const volatile double*>(p); }
-__device__ __forceinline__ cf vload(const cf* p) {
-    const volatile float* q = reinterpret_cast<const volatile float*>(p);
-    return cf{q[0], q[1]};
-}
-__device__ __forceinline__ cd vload(const cd* p) {
-    const volatile double* q = reinterpret_cast<const volatile double*>(p);
-    return cd{q[0], q[1]};
-}
-__device__ __forceinline__ void vstore(float* p, float v) { *reinterpret_cast<volatile float*>(p) = v; }
-__device__ __forceinline__ void vstore(double* p, double v) { *reinterpret_cast<volatile double*>(p) = v; }
-__device__ __forceinline__ void vstore(cf* p, cf v) {
-    volatile float* q = reinterpret_cast<volatile float*>(p);
-    q[0] = v.re;
-    q[1] = v.im;
-}
-__device__ __forceinline__ void vstore(cd* p, cd v) {
-    volatile double* q = reinterpret_cast<volatile double*>(p);
-    q[0] = v.re;
-    q[1] = v.im;
-}
+__device__ __forceinline__ int at4(const int4& s, int k) { return k == 0 ? s.x : k == 1 ? s.y : k == 2 ? s.z : s.w; }
 
-// Level handoff inside a tile: the warp that finishes level l arrives on
-// named barrier 1 + l % kSolveWarps, the warp of level l + 1 syncs on it
-// (64 threads: the two warps).  A barrier orders the shared-memory writes
-// of the arriving warp before the reads of the syncing one, with no
-// separate fence; the pair of warps behind each barrier id is fixed because
-// levels go round-robin over kSolveWarps warps.
-constexpr int kSolveWarps = kTriThreads / 32 - 1;  // 15; the 16th warp receives
-__device__ __forceinline__ void level_arrive(int l) {
-    asm volatile("bar.arrive %0, 64;" ::"r"(1 + l % kSolveWarps) : "memory");
-}
-__device__ __forceinline__ void level_sync(int l) {
-    asm volatile("bar.sync %0, 64;" ::"r"(1 + l % kSolveWarps) : "memory");
-}
-
-// One row of a chunk, gathered before it can be solved: its index, the
-// source of each of its first kPre dependencies (>= 0: position in the
-// tile's shared-memory solution; <= -2: halo slot -(src + 2); -1: another
-// tile's row without a slot, read from x), alpha b_i, the diagonal and the
-// dependency values.
+// A row as its lane holds it before the warp's turn.
 template <class E>
 struct RowData {
-    int32_t row, e0, nd;  // row index, first dependency entry, dependency count (-1 row: inactive)
-    int32_t src[kPre];
+    int4 d;          // row, first dependency entry, dependency count, diagonal entry
+    int4 s;          // dependency sources (dsrc)
+    uint32_t starts; // the chunk's level starts
     E rhs, dg, v[kPre];
 };
-
-// A row's descriptors (first gather stage): desc, dependency columns and
-// halo slots at level-order position p (p >= p1: inactive).
-struct RowIdx {
-    int4 d, c4, s4;
-};
-__device__ __forceinline__ void gather_idx(RowIdx& g, int32_t p, int32_t p1, int32_t base,
-                                           const int4* __restrict__ desc, const int4* __restrict__ dcol,
-                                           const int4* __restrict__ dslot) {
-    g.d = make_int4(-1, 0, 0, -1);
-    g.c4 = make_int4(-1, -1, -1, -1);
-    g.s4 = make_int4(-1, -1, -1, -1);
-    if (p < p1) {
-        g.d = desc[base + p];
-        g.c4 = dcol[base + p];
-        g.s4 = dslot[base + p];
+template <class E>
+__device__ __forceinline__ void gather_idx(RowData<E>& r, int c, int nc, int lane, int32_t m, const int4* __restrict__ desc,
+                                           const int4* __restrict__ dsrc, const uint32_t* __restrict__ lmask) {
+    const int32_t p = 32 * c + lane;
+    r.d = make_int4(-1, 0, 0, -1);
+    r.s = make_int4(-1, -1, -1, -1);
+    r.starts = 0u;
+    if (p < m) {
+        r.d = __ldg(desc + p);
+        r.s = __ldg(dsrc + p);
     }
+    if (c < nc) r.starts = __ldg(lmask + c);
 }
-
-// Second gather stage: resolve the dependency sources, load alpha b_i, the
-// diagonal and the dependency values.
 template <class E, bool UNIT>
-__device__ __forceinline__ void gather_val(RowData<E>& r, const RowIdx& g, int32_t base, int32_t m,
-                                           const E* __restrict__ val, E alpha, const E* __restrict__ b) {
-    constexpr int H = kHalo<E>::value;
-    const int4 d = g.d;
-    r.row = d.x;
-    r.e0 = d.y;
-    r.nd = d.z;
-    const int32_t c[kPre] = {g.c4.x, g.c4.y, g.c4.z, g.c4.w};
-    const int32_t sl[kPre] = {g.s4.x, g.s4.y, g.s4.z, g.s4.w};
-#pragma unroll
-    for (int k = 0; k < kPre; ++k) {
-        const int32_t jl = c[k] - base;
-        r.src[k] = (jl >= 0 && jl < m) ? jl : (sl[k] >= 0 && sl[k] < H ? -(sl[k] + 2) : -1);
-        r.v[k] = E{};
-    }
-    r.rhs = E{};
-    r.dg = E{};
-    if (d.x < 0) return;
-    r.rhs = scale(alpha, ldE(b, d.x));
-    if (!UNIT) r.dg = ldE(val, d.w);
+__device__ __forceinline__ void gather_val(RowData<E>& r, const E* __restrict__ val, const E* __restrict__ b) {
+    if (r.d.x < 0) return;
+    r.rhs = ldE(b, r.d.x);
+    if (!UNIT) r.dg = ldE(val, r.d.w);
 #pragma unroll
     for (int k = 0; k < kPre; ++k)
-        if (k < d.z) r.v[k] = ldE(val, d.y + k);
+        if (k < r.d.z) r.v[k] = ldE(val, int64_t(r.d.y) + k);
 }
 
-template <class E, bool UNIT>
-__device__ __forceinline__ void gather_row(RowData<E>& r, int32_t p, int32_t p1, int32_t base, int32_t m,
-                                           const int4* __restrict__ desc, const int4* __restrict__ dcol,
-                                           const int4* __restrict__ dslot, const E* __restrict__ val, E alpha,
-                                           const E* __restrict__ b) {
-    RowIdx g;
-    gather_idx(g, p, p1, base, desc, dcol, dslot);
-    gather_val<E, UNIT>(r, g, base, m, val, alpha, b);
-}
-
-// Solve one gathered row; returns x_row.
-template <class E, bool UNIT>
-__device__ __forceinline__ E solve_row(const RowData<E>& r, int32_t base, int32_t m, const E* xs, const E* halo,
-                                       const int32_t* __restrict__ ci, const E* __restrict__ val, const E* x,
-                                       int* err, unsigned long long lim) {
-    E acc = r.rhs;
+// The chain of one chunk whose rows have at most ND dependencies: `steps`
+// levels, this lane's row in level `mine` (0: no row).  Every lane computes
+// in every step and only the level's lanes store, so a step has no divergent
+// branch: a lane's term past its own count has a zero value and a source that
+// holds a value already (complex: it is left out, since adding +0 to -0 would
+// change the sign of a zero).
+template <class E, bool UNIT, int ND>
+__device__ __forceinline__ void solve_steps(const RowData<E>& r, const Prep<E>& prep, const E* const (&src)[kPre], E* out,
+                                            int steps, int mine, bool publish, E* xo) {
+#pragma unroll 1
+    for (int l = 1; l <= steps; ++l) {
+        const bool on = mine == l;
+        E xj[ND > 0 ? ND : 1];
 #pragma unroll
-    for (int k = 0; k < kPre; ++k)
-        if (k < r.nd) {
-            const int32_t sk = r.src[k];
-            E xj;
-            if (sk >= 0) {
-                xj = xs[sk];
-            } else if (sk <= -2) {
-                const E* slot = halo + (-sk - 2);
-                xj = vload(slot);
-                if (Pub<E>::pending(xj)) {
-                    Waiter w(lim);
-                    do {
-                        if (w.check(err, 255)) break;
-                        xj = vload(slot);
-                    } while (Pub<E>::pending(xj));
-                }
-            } else {
-                const int32_t j = __ldg(ci + r.e0 + k);
-                xj = await_value(x, j, Pub<E>::load(x, j), err, lim);
-            }
-            acc = fms(acc, r.v[k], xj);
+        for (int k = 0; k < ND; ++k) xj[k] = *src[k];
+        E acc = r.rhs;
+#pragma unroll
+        for (int k = 0; k < ND; ++k) {
+            const E f = fms(acc, r.v[k], xj[k]);
+            acc = (!is_cplx<E>::value || k < r.d.z) ? f : acc;
         }
-    for (int32_t e = r.e0 + kPre; e < r.e0 + r.nd; ++e) {
-        const int32_t j = __ldg(ci + e), jl = j - base;
-        const E xj = (jl >= 0 && jl < m) ? xs[jl] : await_value(x, j, Pub<E>::load(x, j), err, lim);
-        acc = fms(acc, ldE(val, e), xj);
+        if (!UNIT) acc = quot_prepared(acc, r.dg, prep, on);
+        if (on) *out = acc;
+        __syncwarp();
+        if (on && publish) Pub<E>::store(xo, 0, acc);
     }
-    if (!UNIT) acc = quot(acc, r.dg);
-    return acc;
 }
 
 template <class E, bool UPPER, bool UNIT>
-__global__ void __launch_bounds__(kTriThreads)
-k_trsv(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int4* __restrict__ dcol,
-       const int4* __restrict__ dslot, const int32_t* __restrict__ hoff, const int32_t* __restrict__ hrow,
-       const int32_t* __restrict__ lvlptr, const int32_t* __restrict__ nlev, const int32_t* __restrict__ ci,
+__global__ void __launch_bounds__(kSolveThreads, 1)
+k_trsv(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int4* __restrict__ dsrc,
+       const uint32_t* __restrict__ lmask, const uint16_t* __restrict__ pos, const int32_t* __restrict__ ci,
        const E* __restrict__ val, E alpha, const E* __restrict__ b, E* x, unsigned* ticket, int* err,
        unsigned long long lim, int32_t withhold) {
-    constexpr int H = kHalo<E>::value;
     extern __shared__ __align__(16) unsigned char smraw[];
-    E* xs = reinterpret_cast<E*>(smraw);
-    E* halo = xs + kTriTile;
+    TileValues<E>& T = *reinterpret_cast<TileValues<E>*>(smraw);
     __shared__ int s_tile;
     if (threadIdx.x == 0) {
         const int tk = int(atomicAdd(ticket, 1u));
         s_tile = UPPER ? ntiles - 1 - tk : tk;
     }
-    for (int i = threadIdx.x; i < H; i += blockDim.x) Pub<E>::fill(halo, i);
     __syncthreads();
     const int t = s_tile;
     if (t < 0 || t >= ntiles) return;
     const int32_t base = int32_t(t) * kTriTile;
     const int32_t m = min(kTriTile, n - base);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int W = kSolveWarps;
+    const int nc = (m + 31) >> 5;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    desc += base;
+    dsrc += base;
+    lmask += size_t(t) * kTriChunks;
 
-    if (warp == W) {  // ---- receiver warp
-        // Lane k takes slots k, k + 32, k + 64, ... in order, kRecv of its
-        // own slots in flight at a time; lanes advance independently (no
-        // warp-wide window), so one late value holds back only its lane.
-        constexpr int K = kRecv;
-        const int32_t h0 = hoff[t];
-        const int32_t nsl = min(hoff[t + 1] - h0, H);
-        const int32_t* hr = hrow + h0;
-        int32_t j0 = 0;  // own index of the window's first slot: slot = lane + 32 (j0 + k)
+    RowData<E> r{}, nx{};
+    gather_idx(r, w, nc, lane, m, desc, dsrc, lmask);
+    gather_idx(nx, w + kSolveWarps, nc, lane, m, desc, dsrc, lmask);
+    gather_val<E, UNIT>(r, val, b);
+    for (int c = w; c < nc; c += kSolveWarps) {
+        // in flight meanwhile: the next chunk's values, the descriptors of the one after it
+        RowData<E> nn{};
+        gather_val<E, UNIT>(nx, val, b);
+        gather_idx(nn, c + 2 * kSolveWarps, nc, lane, m, desc, dsrc, lmask);
+        // sources in shared memory: the tile's own positions, or (another
+        // tile's value; a zero where there is no dependency) the warp's own places
+        const E* src[kPre];
         unsigned pend = 0;
-        int32_t row[K];
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const int32_t sl = lane + 32 * k;
-            row[k] = sl < nsl ? hr[sl] : 0;
-            if (sl < nsl) pend |= 1u << k;
+        for (int k = 0; k < kPre; ++k) {
+            const int sk = at4(r.s, k);
+            src[k] = sk >= 0 ? T.xs + sk : &T.ext[w][k][lane];
+            if (sk == -1) T.ext[w][k][lane] = E{};
+            if (sk <= -2) pend |= 1u << k;
+            if (k >= r.d.z) r.v[k] = E{};
         }
-        Waiter w(lim);
-        while (pend != 0u) {
-            E v[K];
+        r.rhs = scale(alpha, r.rhs);
+        const Prep<E> prep = UNIT ? Prep<E>{} : prepare_div(r.dg);
+        const uint32_t starts = r.starts | 1u;
+        const int steps = __popc(starts);
+        const int mine = r.d.x >= 0 ? __popc(starts & ((2u << lane) - 1u)) : 0;  // this lane's level within the chunk
+        const int most = __reduce_max_sync(0xffffffffu, r.d.z);
+        const bool publish = r.d.x != withhold;
+        E* const out = T.xs + 32 * c + lane;
+        E* const xo = x + (r.d.x >= 0 ? r.d.x : 0);
+        // the other tiles' values, last: nothing but the turn comes after their arrival
+        if (pend != 0u) {
+            Waiter wt(lim);
+            for (;;) {
+                E xe[kPre];
 #pragma unroll
-            for (int k = 0; k < K; ++k)
-                if ((pend >> k) & 1u) v[k] = Pub<E>::load(x, row[k]);
-            bool got = false;
+                for (int k = 0; k < kPre; ++k)
+                    if ((pend >> k) & 1u) xe[k] = Pub<E>::load(x, -at4(r.s, k) - 2);
+                const bool stop = wt.check(err, 63);  // the values go in as they are then
 #pragma unroll
-            for (int k = 0; k < K; ++k)
-                if (((pend >> k) & 1u) && !Pub<E>::pending(v[k])) {
-                    vstore(halo + lane + 32 * (j0 + k), v[k]);
-                    pend &= ~(1u << k);
-                    got = true;
-                }
-            // slide over the delivered front of the window
-            for (int g = 0; g < K && (pend & 1u) == 0u && lane + 32 * j0 < nsl; ++g) {
-                ++j0;
-                pend >>= 1;
-#pragma unroll
-                for (int k = 0; k + 1 < K; ++k) row[k] = row[k + 1];
-                const int32_t sl = lane + 32 * (j0 + K - 1);
-                row[K - 1] = sl < nsl ? hr[sl] : 0;
-                if (sl < nsl) pend |= 1u << (K - 1);
+                for (int k = 0; k < kPre; ++k)
+                    if (((pend >> k) & 1u) && (stop || !Pub<E>::pending(xe[k]))) {
+                        T.ext[w][k][lane] = xe[k];
+                        pend &= ~(1u << k);
+                    }
+                if (pend == 0u) break;
             }
-            if (got) {
-                w = Waiter(lim);
-            } else {
-                // nothing arrived in this pass: back off before polling the same
-                // lines again, so waiting receivers do not flood the L2 slices
-                // their producers store to
-                if (w.check(err, 15)) break;
-                __nanosleep(100);
-            }
-        }
-        return;
-    }
-
-    // ---- solve warps: levels round-robin.  The first chunk (32 rows) of a
-    // warp's coming levels is gathered in a three-stage software pipeline
-    // across the warp's visits -- level bounds for level l + 3W, descriptors
-    // for l + 2W, values for l + W -- so each stage uses only registers that
-    // arrived during an earlier visit and a visit never stalls on a chain of
-    // dependent loads.  Within a level, the next chunk is gathered while the
-    // current one is solved.
-    const int L = nlev[t];
-    const int32_t* lp = lvlptr + size_t(t) * (kTriTile + 1);
-    auto bounds = [&](int lj, int32_t& a0, int32_t& a1) {
-        a0 = lj < L ? lp[lj] : 0;
-        a1 = lj < L ? lp[lj + 1] : 0;
-    };
-    int32_t pa0, pa1;          // stage 1: bounds of level l + 2W (l + 3W after the shift below)
-    RowIdx gb;                 // stage 2: descriptors of level l + W (l + 2W after the shift)
-    int32_t gb0, gb1;
-    RowData<E> rc;             // stage 3: gathered rows of level l (l + W after the shift)
-    int32_t rc0, rc1;
-    bounds(warp, rc0, rc1);
-    gather_row<E, UNIT>(rc, rc0 + lane, rc1, base, m, desc, dcol, dslot, val, alpha, b);
-    bounds(warp + W, gb0, gb1);
-    gather_idx(gb, gb0 + lane, gb1, base, desc, dcol, dslot);
-    bounds(warp + 2 * W, pa0, pa1);
-    for (int l = warp; l < L; l += W) {
-        const int32_t p0 = rc0, p1 = rc1;
-        RowData<E> cur = rc;
-        gather_val<E, UNIT>(rc, gb, base, m, val, alpha, b);        // level l + W
-        rc0 = gb0;
-        rc1 = gb1;
-        gather_idx(gb, pa0 + lane, pa1, base, desc, dcol, dslot);   // level l + 2W
-        gb0 = pa0;
-        gb1 = pa1;
-        bounds(l + 3 * W, pa0, pa1);                                 // level l + 3W
-        int32_t pub_row = -1;
-        E pub_val{};
-        if (l > 0) level_sync(l - 1);  // levels < l of the tile are complete
-        for (int32_t q = p0; q < p1; q += 32) {
-            const bool more = q + 32 < p1;
-            RowData<E> nxt;
-            if (more) gather_row<E, UNIT>(nxt, q + 32 + lane, p1, base, m, desc, dcol, dslot, val, alpha, b);
-            if (cur.row >= 0) {
-                const E acc = solve_row<E, UNIT>(cur, base, m, xs, halo, ci, val, x, err, lim);
-                xs[cur.row - base] = acc;
-                if (more) {
-                    if (cur.row != withhold) Pub<E>::store(x, cur.row, acc);  // more chunks follow in this level
-                } else {
-                    pub_row = cur.row;
-                    pub_val = acc;
-                }
-            }
-            if (more) cur = nxt;
         }
         __syncwarp();
-        level_arrive(l);
-        // the global store after the in-tile announcement
-        if (pub_row >= 0 && pub_row != withhold) Pub<E>::store(x, pub_row, pub_val);
+        if (c > 0) chunk_sync(w == 0 ? kSolveWarps - 1 : w - 1);  // the chunks before this one are complete
+        switch (most) {
+            case 0: solve_steps<E, UNIT, 0>(r, prep, src, out, steps, mine, publish, xo); break;
+            case 1: solve_steps<E, UNIT, 1>(r, prep, src, out, steps, mine, publish, xo); break;
+            case 2: solve_steps<E, UNIT, 2>(r, prep, src, out, steps, mine, publish, xo); break;
+            case 3: solve_steps<E, UNIT, 3>(r, prep, src, out, steps, mine, publish, xo); break;
+            case 4: solve_steps<E, UNIT, 4>(r, prep, src, out, steps, mine, publish, xo); break;
+            default:  // rows with more than kPre dependencies among them
+                for (int l = 1; l <= steps; ++l) {
+                    if (mine == l) {
+                        E acc = r.rhs;
+#pragma unroll
+                        for (int k = 0; k < kPre; ++k)
+                            if (k < r.d.z) acc = fms(acc, r.v[k], *src[k]);
+                        for (int32_t e = r.d.y + kPre; e < r.d.y + r.d.z; ++e) {
+                            const int32_t j = __ldg(ci + e), jl = j - base;
+                            const E xv = (jl >= 0 && jl < m) ? T.xs[__ldg(pos + j)]
+                                                             : await_value(x, j, Pub<E>::load(x, j), err, lim);
+                            acc = fms(acc, ldE(val, e), xv);
+                        }
+                        if (!UNIT) acc = quot(acc, r.dg);
+                        *out = acc;
+                        if (publish) Pub<E>::store(xo, 0, acc);
+                    }
+                    __syncwarp();
+                }
+        }
+        __syncwarp();
+        if (c + 1 < nc) chunk_arrive(w);
+        r = nx;
+        nx = nn;
     }
-    // the warp that would take level L syncs on the last arrival, so that no
-    // barrier is left half-arrived when the block ends
-    if (L > 0 && warp == L % W) level_sync(L - 1);
 }
 
 // ---- approximate solves: Jacobi sweeps ------------------------------------
@@ -955,11 +909,11 @@ int analyse(hpb_context* ctx, int upper, int32_t n, int64_t nnz, const int32_t* 
         return set_error(ctx, status, "hpb_csr_tri_create: %s", what);
     };
     const size_t nn = size_t(n);
-    if (cudaMalloc(&P->desc, nn * sizeof(int4)) != cudaSuccess || cudaMalloc(&P->dcol, nn * sizeof(int4)) != cudaSuccess ||
+    if (cudaMalloc(&P->desc, nn * sizeof(int4)) != cudaSuccess || cudaMalloc(&P->dsrc, nn * sizeof(int4)) != cudaSuccess ||
+        cudaMalloc(&P->pos, nn * sizeof(uint16_t)) != cudaSuccess ||
+        cudaMalloc(&P->lmask, size_t(P->ntiles) * kTriChunks * sizeof(uint32_t)) != cudaSuccess ||
         cudaMalloc(&P->lvlptr, size_t(P->ntiles) * (kTriTile + 1) * sizeof(int32_t)) != cudaSuccess ||
         cudaMalloc(&P->nlev, size_t(P->ntiles) * sizeof(int32_t)) != cudaSuccess ||
-        cudaMalloc(&P->hoff, (size_t(P->ntiles) + 1) * sizeof(int32_t)) != cudaSuccess ||
-        cudaMalloc(&P->dslot, nn * sizeof(int4)) != cudaSuccess ||
         cudaMalloc(&P->dpos, nn * sizeof(int32_t)) != cudaSuccess ||
         cudaMalloc(&P->flags, (nn + 1) * sizeof(unsigned)) != cudaSuccess ||
         cudaMalloc(&P->err, 2 * sizeof(int)) != cudaSuccess || cudaMalloc(&beg, nn * sizeof(int32_t)) != cudaSuccess ||
@@ -974,50 +928,28 @@ int analyse(hpb_context* ctx, int upper, int32_t n, int64_t nnz, const int32_t* 
     cudaMemcpyAsync(P->err, init, sizeof(init), cudaMemcpyHostToDevice, s);
     cudaMemsetAsync(missing, 0, sizeof(int), s);
     k_tri_rows<<<(n + 255) / 256, 256, 0, s>>>(n, nnz, P->upper, rp, ci, beg, cnt, P->dpos, P->err, missing);
-    const size_t lv_smem = size_t(kTriTile) * (sizeof(unsigned long long) + sizeof(int));
+    const size_t lv_smem = size_t(kTriTile) * 2 * sizeof(int);
     cudaMemsetAsync(chain, 0, (size_t(P->ntiles) + 1) * sizeof(unsigned), s);
     if (P->upper) {
         allow_smem(k_tri_levels<true>, lv_smem);
-        k_tri_levels<true><<<P->ntiles, kLvThreads, lv_smem, s>>>(n, P->ntiles, ci, beg, cnt, P->dpos, glev,
-                                                                   P->desc, P->dcol, P->lvlptr, P->nlev, P->hoff,
-                                                                   chain, P->err);
+        k_tri_levels<true><<<P->ntiles, kLvThreads, lv_smem, s>>>(n, P->ntiles, ci, beg, cnt, glev, chain, P->err);
     } else {
         allow_smem(k_tri_levels<false>, lv_smem);
-        k_tri_levels<false><<<P->ntiles, kLvThreads, lv_smem, s>>>(n, P->ntiles, ci, beg, cnt, P->dpos, glev,
-                                                                    P->desc, P->dcol, P->lvlptr, P->nlev, P->hoff,
-                                                                    chain, P->err);
+        k_tri_levels<false><<<P->ntiles, kLvThreads, lv_smem, s>>>(n, P->ntiles, ci, beg, cnt, glev, chain, P->err);
     }
-    count_launch(2);
+    const size_t sort_smem = size_t(kTriTile) * (sizeof(unsigned long long) + sizeof(uint16_t));
+    allow_smem(k_tri_sort, sort_smem);
+    k_tri_sort<<<P->ntiles, kSortThreads, sort_smem, s>>>(n, ci, beg, cnt, P->dpos, glev, P->desc, P->dsrc, P->pos,
+                                                          P->lmask, P->lvlptr, P->nlev);
+    count_launch(3);
     if (cudaGetLastError() != cudaSuccess) return fail(HPB_ERROR_CUDA, "analysis launch failed");
     int host_err = 0, host_missing = 0;
-    std::vector<int32_t> lev(size_t(P->ntiles)), hc(size_t(P->ntiles) + 1, 0);
-    // the per-tile halo counts were written into hoff[0, ntiles)
+    std::vector<int32_t> lev(size_t(P->ntiles));
     if (cudaMemcpyAsync(&host_err, P->err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaMemcpyAsync(&host_missing, missing, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaMemcpyAsync(lev.data(), P->nlev, lev.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, s) !=
             cudaSuccess ||
-        cudaMemcpyAsync(hc.data(), P->hoff, size_t(P->ntiles) * sizeof(int32_t), cudaMemcpyDeviceToHost, s) !=
-            cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
-        return fail(HPB_ERROR_CUDA, "analysis failed");
-    // counts -> offsets; slots of other-tile dependencies in level order
-    int64_t total = 0;
-    for (int32_t t = 0; t < P->ntiles; ++t) {
-        const int32_t c = hc[size_t(t)];
-        hc[size_t(t)] = int32_t(total);
-        total += c;
-    }
-    if (total > INT32_MAX) return fail(HPB_ERROR_INVALID_VALUE, "too many dependencies between row tiles");
-    hc[size_t(P->ntiles)] = int32_t(total);
-    if (cudaMalloc(&P->hrow, size_t(total > 0 ? total : 1) * sizeof(int32_t)) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(HPB_ERROR_OUT_OF_MEMORY, "device allocation failed");
-    }
-    if (cudaMemcpyAsync(P->hoff, hc.data(), hc.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s) != cudaSuccess)
-        return fail(HPB_ERROR_CUDA, "analysis failed");
-    k_tri_halo<<<P->ntiles, kLvThreads, 0, s>>>(n, P->dcol, P->hoff, P->dslot, P->hrow);
-    count_launch();
-    if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess)
         return fail(HPB_ERROR_CUDA, "analysis failed");
     cudaFree(beg);
     cudaFree(cnt);
@@ -1040,12 +972,12 @@ int analyse(hpb_context* ctx, int upper, int32_t n, int64_t nnz, const int32_t* 
 
 void release(Plan* P) {
     cudaFree(P->desc);
-    cudaFree(P->dcol);
-    cudaFree(P->dslot);
-    cudaFree(P->hoff);
-    cudaFree(P->hrow);
-    P->dcol = P->dslot = nullptr;
-    P->hoff = P->hrow = nullptr;
+    cudaFree(P->dsrc);
+    cudaFree(P->pos);
+    cudaFree(P->lmask);
+    P->dsrc = nullptr;
+    P->pos = nullptr;
+    P->lmask = nullptr;
     cudaFree(P->lvlptr);
     cudaFree(P->nlev);
     cudaFree(P->dpos);
@@ -1064,7 +996,8 @@ cudaError_t launch_trsv(const Plan& P, int unit, const E* val, E alpha, const E*
     if (P.n == 0) return cudaSuccess;
     const int fill_grid = int(std::min<int64_t>((int64_t(P.n) + 255) / 256, 148 * 8));
     k_tri_fill<E><<<fill_grid, 256, 0, s>>>(P.n, x, P.flags + P.n);
-    constexpr size_t sm = trsv_smem<E>();
+    constexpr size_t sm = sizeof(TileValues<E>);
+    static_assert(sm <= 226 * 1024, "shared memory of a tile");
     // the shared-memory limit is a per-device function attribute: raise it
     // once for every device this process launches on
     static std::atomic<uint64_t> done_mask{0};
@@ -1080,9 +1013,8 @@ cudaError_t launch_trsv(const Plan& P, int unit, const E* val, E alpha, const E*
     }
     auto k = P.upper ? (unit ? k_trsv<E, true, true> : k_trsv<E, true, false>)
                      : (unit ? k_trsv<E, false, true> : k_trsv<E, false, false>);
-    k<<<P.ntiles, kTriThreads, sm, s>>>(P.n, P.ntiles, P.desc, P.dcol, P.dslot, P.hoff, P.hrow, P.lvlptr,
-                                             P.nlev, P.ci, val, alpha, b, x, P.flags + P.n, P.err,
-                                             P.wait_ns ? P.wait_ns : kWaitNs, P.withhold_row);
+    k<<<P.ntiles, kSolveThreads, sm, s>>>(P.n, P.ntiles, P.desc, P.dsrc, P.lmask, P.pos, P.ci, val, alpha, b, x,
+                                        P.flags + P.n, P.err, P.wait_ns ? P.wait_ns : kWaitNs, P.withhold_row);
     count_launch(2);
     return cudaGetLastError();
 }

@@ -7,19 +7,17 @@
 // (common/csr/gpu_ilu0_preconditioner.h:32-80) their factors.
 //
 // An analysis (hpb_csr_tri) is made once per sparsity pattern and triangle:
-// rows are cut into tiles of kTriTile consecutive rows; inside a tile each
-// row gets its level (longest chain of in-tile dependencies), and the tile's
-// rows are stored in level order as packed descriptors.  A solve is one
-// kernel: each block takes the next tile by ticket (ascending for a lower,
-// descending for an upper triangle), keeps the tile's solution in shared
-// memory, and its warps take the tile's levels round-robin, so a warp loads
-// the rows of its next level while earlier levels finish.  Dependencies on
-// other tiles are read from x itself (x is pre-filled with a signalling-NaN
-// sentinel), by a receiver warp per block that streams them into shared
-// memory ahead of need; the factorization, whose rows are read as a whole,
-// uses per-row flags (release/acquire at GPU scope).  Every wait has a time
-// limit after which the kernel records a timeout and carries on, so a
-// launch always ends.
+// rows are cut into tiles of kTriTile consecutive rows; every row gets its
+// level (longest chain of dependencies over the whole triangle), and the
+// tile's rows are stored in level order as packed descriptors.  A solve is
+// one kernel: each block takes the next tile by ticket (ascending for a
+// lower, descending for an upper triangle), keeps the tile's solution in
+// shared memory, and its warps take the tile's rows round-robin in level
+// order, 32 at a time.  Dependencies on other tiles are polled from x itself
+// (x is pre-filled with a signalling-NaN sentinel); the factorization, whose
+// rows are read as a whole, uses per-row flags (release/acquire at GPU
+// scope).  Every wait has a time limit after which the kernel records a
+// timeout and carries on, so a launch always ends.
 #pragma once
 
 #include "hpb_common.cuh"
@@ -28,7 +26,8 @@ namespace hpb {
 namespace tri {
 
 constexpr int kTriTile = 8192;      // rows per tile
-constexpr int kTriThreads = 512;    // threads per solve block (16 warps)
+constexpr int kTriThreads = 512;    // threads per factorization block (16 warps)
+constexpr int kTriChunks = kTriTile / 32;  // chunks of 32 positions of a tile
 
 // Error bits of Plan::err (device).
 constexpr int kErrUnsorted = 1;     // column indices of a row not strictly increasing
@@ -48,10 +47,9 @@ struct Plan {
     const int32_t* rp = nullptr;    // caller's structure; must stay valid and unchanged
     const int32_t* ci = nullptr;
     int4* desc = nullptr;           // n: (row, first dependency, dependency count, diagonal position) in level order
-    int4* dcol = nullptr;           // n: columns of the first four dependencies (-1: none), in level order
-    int4* dslot = nullptr;          // n: halo slot of each of those that lies in another tile (-1: none)
-    int32_t* hoff = nullptr;        // ntiles + 1: first halo slot of each tile in hrow
-    int32_t* hrow = nullptr;        // halo slots: the other-tile row each one is filled from
+    int4* dsrc = nullptr;           // n: where each of the first four dependencies is found, in level order
+    uint16_t* pos = nullptr;        // n: position of each row in its tile's level order
+    uint32_t* lmask = nullptr;      // ntiles * kTriChunks: positions of a chunk that start a level
     int32_t* lvlptr = nullptr;      // ntiles * (kTriTile + 1): level starts within the tile
     int32_t* nlev = nullptr;        // ntiles
     int32_t* dpos = nullptr;        // n: position of the diagonal entry of each row, -1 if absent
