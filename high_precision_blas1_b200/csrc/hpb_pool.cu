@@ -19,24 +19,45 @@ namespace fused {
 namespace {
 
 constexpr int kMaxDevices = 64;
+// The analyses' pool holds on to freed memory while it has at most this much
+// in all, in use or not (about 58 bytes a row and triangle: both triangles of
+// nine million rows); what is beyond goes back to the device when a stream or
+// the device is next synchronised.  (With 256 MB, callers that hold three
+// matrices' analyses of a million rows paid 15 ms a set-up for memory going
+// back and forth.)
+constexpr uint64_t kAnalysisKeep = uint64_t(1) << 30;
 std::mutex g_pool_mutex;
-cudaMemPool_t g_pools[kMaxDevices] = {};
+enum PoolKind { POOL_WORKSPACE = 0, POOL_ANALYSIS = 1 };
+cudaMemPool_t g_pools[2][kMaxDevices] = {};
 
-cudaMemPool_t pool_for(int device) {
+cudaMemPool_t pool_for(int device, PoolKind kind) {
     if (device < 0 || device >= kMaxDevices) return nullptr;
     std::lock_guard<std::mutex> lock(g_pool_mutex);
-    if (g_pools[device] == nullptr) {
+    if (g_pools[kind][device] == nullptr) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = device;
         cudaMemPool_t pool = nullptr;
         if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) return nullptr;
-        uint64_t keep = ~uint64_t(0);
+        uint64_t keep = kind == POOL_WORKSPACE ? ~uint64_t(0) : kAnalysisKeep;
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        g_pools[device] = pool;
+        g_pools[kind][device] = pool;
     }
-    return g_pools[device];
+    return g_pools[kind][device];
+}
+
+void* alloc_from(PoolKind kind, size_t bytes, cudaStream_t stream) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return nullptr;
+    cudaMemPool_t pool = pool_for(device, kind);
+    if (!pool) return nullptr;
+    void* p = nullptr;
+    if (cudaMallocFromPoolAsync(&p, bytes ? bytes : 16, pool, stream) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return p;
 }
 
 constexpr size_t kPinnedSlot = 4096;
@@ -51,17 +72,10 @@ thread_local PinnedCache t_pinned;
 
 }  // namespace
 
-void* pool_alloc(size_t bytes, cudaStream_t stream) {
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess) return nullptr;
-    cudaMemPool_t pool = pool_for(device);
-    if (!pool) return nullptr;
-    void* p = nullptr;
-    if (cudaMallocFromPoolAsync(&p, bytes ? bytes : 16, pool, stream) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    return p;
+void* pool_alloc(size_t bytes, cudaStream_t stream) { return alloc_from(POOL_WORKSPACE, bytes, stream); }
+void* analysis_alloc(size_t bytes, cudaStream_t stream) { return alloc_from(POOL_ANALYSIS, bytes, stream); }
+void analysis_free(void* p, cudaStream_t stream) {
+    if (p) cudaFreeAsync(p, stream);
 }
 
 void pool_free(void* p, cudaStream_t stream) {
@@ -114,7 +128,8 @@ SolverWorkspace::~SolverWorkspace() {
 extern "C" int hpb_solver_memory_release(void) {
     std::lock_guard<std::mutex> lock(hpb::fused::g_pool_mutex);
     int status = HPB_SUCCESS;
-    for (cudaMemPool_t pool : hpb::fused::g_pools)
-        if (pool && cudaMemPoolTrimTo(pool, 0) != cudaSuccess) status = HPB_ERROR_CUDA;
+    for (auto& kind : hpb::fused::g_pools)
+        for (cudaMemPool_t pool : kind)
+            if (pool && cudaMemPoolTrimTo(pool, 0) != cudaSuccess) status = HPB_ERROR_CUDA;
     return status;
 }

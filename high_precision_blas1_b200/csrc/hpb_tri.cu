@@ -15,13 +15,13 @@
 #include <mutex>
 #include <vector>
 
+#include "hpb_fused.cuh"
 #include "hpb_tri.cuh"
 
 namespace hpb {
 namespace tri {
 namespace {
 
-constexpr int kLvThreads = 512;
 constexpr int kSortThreads = 1024;
 constexpr int kPre = 4;                          // dependencies per row prefetched into registers
 constexpr int kMerge = 8;                        // ILU(0): update pairs per batch of loads
@@ -100,6 +100,23 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 }
 __device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+__device__ __forceinline__ unsigned long long ld_relaxed64(const void* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned ld_relaxed32(const void* p) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_relaxed64(void* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ void st_relaxed32(void* p, unsigned v) {
+    asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 // A timeout is sticky: once one wait has given up, every later wait of the
@@ -191,82 +208,357 @@ __global__ void k_tri_rows(int32_t n, int64_t nnz, int upper, const int32_t* __r
     dpos[i] = dp;
 }
 
-// Per tile (one block): the global level of each row -- the longest chain
-// of dependencies ending at it over the whole triangle.  Tiles are taken by ticket in the solve's order (ascending
-// for a lower, descending for an upper triangle) and each waits (bounded)
-// for the previous one to publish its levels, so the levels of every
-// other-tile dependency are final when read.  In the tile: start from
-// 1 + the largest other-tile dependency level, then relaxation sweeps over
-// contiguous per-thread segments walked in dependency order until a sweep
-// changes nothing (a sweep that changes something brings one more row of
-// the longest in-tile chain to its final value, so at most m + 1 sweeps).
+// Levels: the level of a row is the length of the longest chain of
+// dependencies ending at it over the whole triangle.  One block per tile,
+// tiles taken by ticket in the solve's order (ascending for a lower,
+// descending for an upper triangle), all of them at work at once.  A block
+// first lists, for each of its rows, the rows of the tile that depend on it
+// (counts, a scan and a fill in shared memory) and how many dependencies each
+// row waits for.  Then one warp takes the rows whose dependencies are all
+// known from a queue, 32 at a time, publishes their levels to glev and
+// hands them on to their dependents, whose last dependency puts them on the
+// queue; the other warps poll the levels of other tiles' rows (glev holds -1
+// until a level is published) and hand them on the same way.  Each edge is
+// touched once, in whatever order the levels become known, so the time is
+// the chain's and no tile waits for another to finish.
+// Measured on B200: 1.0 ms a triangle for the 1024^2 5-point operator (2047
+// levels, 128 tiles), against 23.4 ms for relaxation sweeps over the tiles
+// one after another; about 0.3 us a level and 5 us a tile boundary.  The
+// polling lanes hold all of a 7-point tile's dependencies on other tiles at
+// once (10 each): with 4 or 8 a lane waits for one that comes late while
+// others are there already (96^3: 6 and 2 ms instead of 0.6).
+// A tile with more than kMaxEdges dependencies inside it takes the sweeps,
+// once all levels from outside are known.
+constexpr int kGlThreads = 1024;
+constexpr int kMaxEdges = 7 * kTriTile;  // in-tile dependencies of a tile
+constexpr int kGlSlots = 10;             // other-tile levels in flight per polling lane
+struct LevelTile {
+    int lev[kTriTile + 1];       // the largest level + 1 of the dependencies met so far (last: no row)
+    int left[kTriTile + 1];      // dependencies not met yet
+    uint16_t queue[kTriTile];    // rows in the order they became ready (kNoRow: not yet)
+    int off[kTriTile];           // dependents met while listing; general list: end of each row's part of `to`
+    union {
+        uint16_t to4[kTriTile][4];  // up to four dependents of each row (kTriTile: none)
+        uint16_t to[kMaxEdges];     // general list of dependents
+    };
+    int tail, edges, more, scan[kGlThreads / 32];
+};
+constexpr uint16_t kNoRow = 0xFFFFu;
+
+// Dependency j of row i of the tile [base, base + m): does it count at all
+// (within range and in the solve's direction, so the graph has no cycle even
+// before the structure checks are read)?
 template <bool UPPER>
-__global__ void __launch_bounds__(kLvThreads)
+__device__ __forceinline__ bool is_dep(int32_t n, int32_t i, int32_t j) {
+    return j >= 0 && j < n && (UPPER ? j > i : j < i);
+}
+
+// Row d has met a dependency of level lv - 1; its last one puts it on the
+// queue.  The count is taken down only after the maximum has returned (the
+// decrement's operand depends on it), so whoever takes the row off the queue
+// finds its final level.
+__device__ __forceinline__ void meet(LevelTile& T, int d, int lv) {
+    int old, left;
+    asm volatile("atom.shared::cta.max.s32 %0, [%1], %2;"
+                 : "=r"(old)
+                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&T.lev[d]))), "r"(lv)
+                 : "memory");
+    asm volatile("atom.shared::cta.add.s32 %0, [%1], %2;"
+                 : "=r"(left)
+                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&T.left[d]))), "r"((old >> 31) - 1)
+                 : "memory");
+    if (left == 1) {
+        int at;
+        asm volatile("atom.shared::cta.add.s32 %0, [%1], 1;"
+                     : "=r"(at)
+                     : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&T.tail)))
+                     : "memory");
+        *reinterpret_cast<volatile uint16_t*>(&T.queue[at]) = uint16_t(d);
+    }
+}
+
+template <bool UPPER>
+__global__ void __launch_bounds__(kGlThreads, 1)
 k_tri_levels(int32_t n, int32_t ntiles, const int32_t* __restrict__ ci, const int32_t* __restrict__ beg,
-             const int32_t* __restrict__ cnt, int32_t* glev, unsigned* chain, int* err) {
+             const int32_t* __restrict__ cnt, int32_t* glev, unsigned* ticket, int* err) {
     extern __shared__ __align__(16) unsigned char shraw[];
-    volatile int* lev = reinterpret_cast<volatile int*>(shraw);  // kTriTile
-    int* ext = reinterpret_cast<int*>(shraw) + kTriTile;          // kTriTile
+    LevelTile& T = *reinterpret_cast<LevelTile*>(shraw);
     __shared__ int s_tile;
-    if (threadIdx.x == 0) {
-        const int tk = int(atomicAdd(chain + ntiles, 1u));
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) {
+        const int tk = int(atomicAdd(ticket, 1u));
         s_tile = UPPER ? ntiles - 1 - tk : tk;
+        T.tail = 0;
     }
     __syncthreads();
     const int t = s_tile;
     if (t < 0 || t >= ntiles) return;
     const int32_t base = int32_t(t) * kTriTile;
     const int32_t m = min(kTriTile, n - base);
-    const int prev = UPPER ? t + 1 : t - 1;
-    if (prev >= 0 && prev < ntiles) {
-        if (threadIdx.x == 0) {
-            Waiter w;
-            while (ld_acquire(chain + prev) == 0u)
-                if (w.check(err, 63)) break;
-        }
-        __syncthreads();
+    if (tid == 0) {
+        T.more = 0;
+        T.lev[kTriTile] = 0;
+        T.left[kTriTile] = INT_MAX;  // "no dependent" never becomes ready
     }
-    // lower bound from the other-tile dependencies (final levels)
-    for (int r = threadIdx.x; r < m; r += blockDim.x) {
-        const int32_t i = base + r;
-        const int32_t b = __ldg(beg + i), c = __ldg(cnt + i);
-        int e = 0;
+    for (int r = tid; r < kTriTile; r += kGlThreads) {
+        T.lev[r] = 0;
+        T.off[r] = 0;
+        T.queue[r] = kNoRow;
+        *reinterpret_cast<uint2*>(T.to4[r]) = make_uint2(kTriTile * 0x10001u, kTriTile * 0x10001u);
+    }
+    __syncthreads();
+    // ---- who depends on each row: up to four dependents in one go
+    bool more = false;
+    for (int r = tid; r < m; r += kGlThreads) {
+        const int32_t i = base + r, b = __ldg(beg + i), c = __ldg(cnt + i);
+        int left = 0;
         for (int32_t k = b; k < b + c; ++k) {
             const int32_t j = __ldg(ci + k), jl = j - base;
-            // (a column outside [0, n) is reported by k_tri_rows; never read through it)
-            if (!(jl >= 0 && jl < m) && j >= 0 && j < n) e = max(e, __ldcg(glev + j) + 1);
+            if (!is_dep<UPPER>(n, i, j)) continue;
+            ++left;
+            if (jl >= 0 && jl < m) {
+                const int at = atomicAdd(&T.off[jl], 1);
+                if (at < 4) T.to4[jl][at] = uint16_t(r);
+                more |= at >= 4;
+            }
         }
-        ext[r] = e;
-        lev[r] = e;
+        T.left[r] = left;
+        if (left == 0) T.queue[atomicAdd(&T.tail, 1)] = uint16_t(r);
+    }
+    more = __syncthreads_or(more);
+    if (more) {  // ---- rows with more dependents: a list by offsets
+    // exclusive scan of off: kTriTile / kGlThreads entries per thread
+    {
+        constexpr int P = kTriTile / kGlThreads;
+        int v[P], s = 0;
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+            v[k] = T.off[tid * P + k];
+            s += v[k];
+        }
+        int x = s;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= d) x += y;
+        }
+        if (lane == 31) T.scan[warp] = x;
+        __syncthreads();
+        if (warp == 0) {
+            const int ws = T.scan[lane];
+            int y = ws;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int z = __shfl_up_sync(0xffffffffu, y, d);
+                if (lane >= d) y += z;
+            }
+            T.scan[lane] = y - ws;
+            if (lane == 31) T.edges = y;
+        }
+        __syncthreads();
+        int acc = T.scan[warp] + x - s;
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+            T.off[tid * P + k] = acc;
+            acc += v[k];
+        }
     }
     __syncthreads();
-    const int seg = (m + blockDim.x - 1) / blockDim.x;
-    const int s0 = min(m, int(threadIdx.x) * seg), s1 = min(m, s0 + seg);
-    int changed, sweeps = 0;
-    do {
-        changed = 0;
-        for (int k = 0; k < s1 - s0; ++k) {
-            const int r = UPPER ? s1 - 1 - k : s0 + k;
-            const int32_t i = base + r;
-            const int32_t b = __ldg(beg + i), c = __ldg(cnt + i);
-            int lv = ext[r];
-            for (int32_t e = b; e < b + c; ++e) {
-                const int32_t j = __ldg(ci + e) - base;
-                // only dependencies in the solve's direction: the graph stays acyclic
-                // (and the sweeps finite) even before the structure checks are read
-                if (j >= 0 && j < m && (UPPER ? j > r : j < r)) lv = max(lv, lev[j] + 1);
+    if (T.edges > kMaxEdges) {  // ---- relaxation sweeps
+        volatile int* lev = T.lev;
+        int* ext = T.left;
+        for (int r = tid; r < m; r += kGlThreads) {  // 1 + the largest level from outside the tile
+            const int32_t i = base + r, b = __ldg(beg + i), c = __ldg(cnt + i);
+            int e = 0;
+            for (int32_t k = b; k < b + c; ++k) {
+                const int32_t j = __ldg(ci + k), jl = j - base;
+                if (!is_dep<UPPER>(n, i, j) || (jl >= 0 && jl < m)) continue;
+                Waiter w;
+                int v;
+                while ((v = int(ld_relaxed32(glev + j))) < 0)
+                    if (w.check(err, 63)) break;
+                e = max(e, v + 1);
             }
-            if (lv > lev[r]) {
-                lev[r] = lv;
-                changed = 1;
+            ext[r] = e;
+            lev[r] = e;
+        }
+        __syncthreads();
+        // contiguous segments walked in dependency order until a sweep
+        // changes nothing (a sweep that changes something brings one more row
+        // of the longest in-tile chain to its final value)
+        const int seg = (m + kGlThreads - 1) / kGlThreads;
+        const int s0 = min(m, tid * seg), s1 = min(m, s0 + seg);
+        int changed, sweeps = 0;
+        do {
+            changed = 0;
+            for (int k = 0; k < s1 - s0; ++k) {
+                const int r = UPPER ? s1 - 1 - k : s0 + k;
+                const int32_t i = base + r, b = __ldg(beg + i), c = __ldg(cnt + i);
+                int lv = ext[r];
+                for (int32_t e = b; e < b + c; ++e) {
+                    const int32_t j = __ldg(ci + e), jl = j - base;
+                    if (is_dep<UPPER>(n, i, j) && jl >= 0 && jl < m) lv = max(lv, lev[jl] + 1);
+                }
+                if (lv > lev[r]) {
+                    lev[r] = lv;
+                    changed = 1;
+                }
+            }
+        } while (__syncthreads_or(changed) && ++sweeps <= m);
+        for (int r = tid; r < m; r += kGlThreads) st_relaxed32(glev + base + r, unsigned(lev[r]));
+        return;
+    }
+    for (int r = tid; r < m; r += kGlThreads) {
+        const int32_t i = base + r, b = __ldg(beg + i), c = __ldg(cnt + i);
+        for (int32_t k = b; k < b + c; ++k) {
+            const int32_t j = __ldg(ci + k), jl = j - base;
+            if (is_dep<UPPER>(n, i, j) && jl >= 0 && jl < m) T.to[atomicAdd(&T.off[jl], 1)] = uint16_t(r);
+        }
+    }
+    __syncthreads();  // off[r] is now the end of row r's part, its start the end of row r - 1's
+    }
+
+    if (warp == 0) {  // ---- the queue
+        // Up to eight ready rows: four lanes each, a dependent per lane; more
+        // of them: a lane each, its dependents one after another.  This chain
+        // of shared loads and atomics is what a level costs, so it is kept
+        // short (one warp issues it; every instruction counts).
+        const volatile uint16_t* queue = T.queue;
+        int head = 0, spins = 0;
+        const int grp = lane >> 2, sub = lane & 3;
+        unsigned long long t0 = 0;
+        while (head < m) {
+            // (the second read, by the whole warp after the first, finds all that the first found)
+            const int wide = head + lane < m ? int(queue[head + lane]) : int(kNoRow);
+            int row = head + grp < m ? int(queue[head + grp]) : int(kNoRow);
+            const unsigned none = __ballot_sync(0xffffffffu, wide == int(kNoRow));
+            const int k = none ? __ffs(int(none)) - 1 : 32;  // rows ready without a gap
+            if (k == 0) {
+                if ((++spins & 255) != 0) continue;
+                const unsigned long long now = gtimer();
+                if (t0 == 0) t0 = now;
+                if (now - t0 > 2 * kWaitNs) {  // the polls below give up earlier: never expected
+                    if (lane == 0) atomicOr(err, kErrTimeout);
+                    return;
+                }
+                continue;
+            }
+            t0 = 0;
+            head += k;
+            const bool few = k <= 8;
+            if (!few) row = wide;
+            if ((few ? grp : lane) < k) {
+                const int lv = *reinterpret_cast<volatile int*>(&T.lev[row]);
+                if (!more && few) {
+                    const int d = T.to4[row][sub];
+                    if (d < kTriTile) meet(T, d, lv + 1);
+                } else if (!more) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int d = T.to4[row][q];
+                        if (d < kTriTile) meet(T, d, lv + 1);
+                    }
+                } else {
+                    const int e1 = T.off[row];
+                    for (int e = (row > 0 ? T.off[row - 1] : 0) + (few ? sub : 0); e < e1; e += few ? 4 : 1)
+                        meet(T, T.to[e], lv + 1);
+                }
+                if (!few || sub == 0) st_relaxed32(glev + base + row, unsigned(lv));
+            }
+            __syncwarp();
+        }
+        return;
+    }
+    // ---- levels from other tiles: each lane walks its rows' dependencies,
+    // kGlSlots of them in flight
+    constexpr int kStride = kGlThreads - 32;
+    int r = UPPER ? m - 1 - (tid - 32) : tid - 32;  // in the order the solve needs them
+    int32_t b = 0, c = 0, k = 0;
+    auto open_row = [&]() {
+        k = 0;
+        c = 0;
+        if (r >= 0 && r < m) {
+            b = __ldg(beg + base + r);
+            c = __ldg(cnt + base + r);
+        }
+    };
+    open_row();
+    int sr[kGlSlots];
+    int32_t sj[kGlSlots];
+    auto refill = [&](int& row, int32_t& from) {  // the lane's next other-tile dependency, -1: none left
+        row = -1;
+        from = 0;
+        while (r >= 0 && r < m) {
+            if (k >= c) {
+                r += UPPER ? -kStride : kStride;
+                open_row();
+                continue;
+            }
+            const int32_t j = __ldg(ci + b + k), jl = j - base;
+            ++k;
+            if (is_dep<UPPER>(n, base + r, j) && !(jl >= 0 && jl < m)) {
+                row = r;
+                from = j;
+                return;
             }
         }
-    } while (__syncthreads_or(changed) && ++sweeps <= m);
-    // publish the tile's levels for the tiles after it
-    for (int r = threadIdx.x; r < m; r += blockDim.x) __stcg(glev + base + r, lev[r]);
-    __threadfence();
+    };
+#pragma unroll
+    for (int q = 0; q < kGlSlots; ++q) refill(sr[q], sj[q]);
+    Waiter w;
+    int pause = 20;
+    for (;;) {
+        int v[kGlSlots];
+        bool any = false, got = false;
+#pragma unroll
+        for (int q = 0; q < kGlSlots; ++q)
+            if (sr[q] >= 0) {
+                v[q] = int(ld_relaxed32(glev + sj[q]));
+                any = true;
+            }
+        if (!any) break;
+        const bool stop = w.check(err, 63);
+        unsigned met = 0;
+#pragma unroll
+        for (int q = 0; q < kGlSlots; ++q)
+            if (sr[q] >= 0 && (v[q] >= 0 || stop)) {
+                meet(T, sr[q], max(v[q], 0) + 1);
+                met |= 1u << q;
+                got = true;
+            }
+        if (met != 0u)
+#pragma unroll
+            for (int q = 0; q < kGlSlots; ++q)
+                if ((met >> q) & 1u) refill(sr[q], sj[q]);
+        if (got) {
+            w = Waiter();
+            pause = 20;
+        } else {  // a tile far behind the front polls less often
+            __nanosleep(pause);
+            pause = min(2 * pause, 320);
+        }
+    }
+}
+
+// Bitonic sort of get(0..m-1) (distinct keys) into key[0, m) by the block.
+template <class K, class F>
+__device__ __forceinline__ void sort_tile(K* key, int m, F get) {
+    int size = 32;  // the power of two the sort runs over
+    while (size < m) size <<= 1;
+    for (int r = threadIdx.x; r < size; r += blockDim.x) key[r] = r < m ? get(r) : ~K(0);
     __syncthreads();
-    if (threadIdx.x == 0) st_release(chain + t, 1u);
+    for (int k = 2; k <= size; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int q = threadIdx.x; q < size / 2; q += blockDim.x) {
+                const int i = ((q & ~(j - 1)) << 1) | (q & (j - 1)), ixj = i | j;
+                const K a = key[i], b = key[ixj];
+                if ((a > b) == ((i & k) == 0)) {
+                    key[i] = b;
+                    key[ixj] = a;
+                }
+            }
+            __syncthreads();
+        }
 }
 
 // Per tile (one block): the tile's rows in (level, row) order -- the order in
@@ -288,27 +580,55 @@ k_tri_sort(int32_t n, const int32_t* __restrict__ ci, const int32_t* __restrict_
     unsigned long long* key = reinterpret_cast<unsigned long long*>(shraw);  // kTriTile
     uint16_t* inv = reinterpret_cast<uint16_t*>(key + kTriTile);             // kTriTile
     __shared__ int first[kTriChunks + 1];  // level starts before each chunk of 32 positions
+    __shared__ int s_lo, s_hi;
     const int t = blockIdx.x;
     const int32_t base = int32_t(t) * kTriTile;
     const int32_t m = min(kTriTile, n - base);
-    int size = 32;  // the power of two the sort runs over
-    while (size < m) size <<= 1;
-    for (int r = threadIdx.x; r < size; r += blockDim.x)
-        key[r] = r < m ? (static_cast<unsigned long long>(glev[base + r]) << 13) | static_cast<unsigned long long>(r)
-                       : ~0ull;
+    if (threadIdx.x == 0) {
+        s_lo = INT_MAX;
+        s_hi = 0;
+    }
     __syncthreads();
-    for (int k = 2; k <= size; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int q = threadIdx.x; q < size / 2; q += blockDim.x) {
-                const int i = ((q & ~(j - 1)) << 1) | (q & (j - 1)), ixj = i | j;
-                const unsigned long long a = key[i], b = key[ixj];
-                if ((a > b) == ((i & k) == 0)) {
-                    key[i] = b;
-                    key[ixj] = a;
-                }
-            }
-            __syncthreads();
+    {
+        int lo = INT_MAX, hi = 0;
+        for (int r = threadIdx.x; r < m; r += blockDim.x) {
+            const int v = glev[base + r];
+            lo = min(lo, v);
+            hi = max(hi, v);
         }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(&s_lo, lo);
+            atomicMax(&s_hi, hi);
+        }
+    }
+    __syncthreads();
+    // the tile's levels span less than 2^18 unless its chains are very long
+    // elsewhere: 32-bit keys then, half the shared-memory traffic
+    const int lo = s_lo;
+    if (s_hi - lo < (1 << 18)) {
+        unsigned* k32 = reinterpret_cast<unsigned*>(key);
+        sort_tile(k32, m, [&](int r) { return (unsigned(glev[base + r] - lo) << 13) | unsigned(r); });
+        // widened in place
+        unsigned v[kTriTile / kSortThreads];
+#pragma unroll
+        for (int k = 0; k < kTriTile / kSortThreads; ++k) {
+            const int p = threadIdx.x + k * kSortThreads;
+            v[k] = p < m ? k32[p] : 0u;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kTriTile / kSortThreads; ++k) {
+            const int p = threadIdx.x + k * kSortThreads;
+            if (p < m) key[p] = v[k];
+        }
+        __syncthreads();
+    } else {
+        sort_tile(key, m, [&](int r) {
+            return (static_cast<unsigned long long>(glev[base + r] - lo) << 13) | static_cast<unsigned long long>(r);
+        });
+    }
     for (int p = threadIdx.x; p < m; p += blockDim.x) {
         const int r = int(key[p] & 8191ull);
         inv[r] = uint16_t(p);
@@ -386,23 +706,6 @@ k_tri_sort(int32_t n, const int32_t* __restrict__ ci, const int32_t* __restrict_
 // warp waits for its level, instead of a flag acquire followed by the load.
 constexpr unsigned long long kSent64 = 0x7FF0DEAD0000BEEFull;  // exponent all ones, quiet bit 0
 constexpr unsigned kSent32 = 0x7F80BEEFu;
-
-__device__ __forceinline__ unsigned long long ld_relaxed64(const void* p) {
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ unsigned ld_relaxed32(const void* p) {
-    unsigned v;
-    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_relaxed64(void* p, unsigned long long v) {
-    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ void st_relaxed32(void* p, unsigned v) {
-    asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 
 // Published values: load / store / fill / "still the sentinel" per element
 // type (complex: per component; a component is final once it is not the
@@ -896,96 +1199,94 @@ int analyse(hpb_context* ctx, int upper, int32_t n, int64_t nnz, const int32_t* 
     P->ntiles = int32_t((int64_t(n) + kTriTile - 1) / kTriTile);
     cudaGetDevice(&P->device);
     cudaStream_t s = ctx->stream;
-    int32_t *beg = nullptr, *cnt = nullptr, *glev = nullptr;
-    unsigned* chain = nullptr;
-    int* missing = nullptr;
+    // Two allocations from the analyses' pool: what the plan keeps, and the
+    // analysis' own work arrays.  The stream is synchronised before they are
+    // used or given back elsewhere.
+    size_t keep = 0, tmp = 0;
+    auto part = [](size_t& total, size_t bytes) {
+        const size_t at = total;
+        total += (bytes + 255) & ~size_t(255);
+        return at;
+    };
+    const size_t nn = size_t(n), nt = size_t(P->ntiles);
+    const size_t o_desc = part(keep, nn * sizeof(int4)), o_dsrc = part(keep, nn * sizeof(int4));
+    const size_t o_pos = part(keep, nn * sizeof(uint16_t)), o_lmask = part(keep, nt * kTriChunks * sizeof(uint32_t));
+    const size_t o_lvl = part(keep, nt * (kTriTile + 1) * sizeof(int32_t)), o_dpos = part(keep, nn * sizeof(int32_t));
+    const size_t o_flags = part(keep, (nn + 1) * sizeof(unsigned));
+    const size_t o_err = part(keep, (4 + nt) * sizeof(int));  // err, err_row, rows without a diagonal, -, nlev
+    const size_t o_beg = part(tmp, nn * sizeof(int32_t)), o_cnt = part(tmp, nn * sizeof(int32_t));
+    const size_t o_glev = part(tmp, nn * sizeof(int32_t)), o_tick = part(tmp, sizeof(unsigned));
+    char* work = nullptr;
     auto fail = [&](int status, const char* what) {
-        cudaFree(beg);
-        cudaFree(cnt);
-        cudaFree(glev);
-        cudaFree(chain);
-        cudaFree(missing);
+        cudaStreamSynchronize(s);
+        fused::analysis_free(work, s);
         release(P);
         return set_error(ctx, status, "hpb_csr_tri_create: %s", what);
     };
-    const size_t nn = size_t(n);
-    if (cudaMalloc(&P->desc, nn * sizeof(int4)) != cudaSuccess || cudaMalloc(&P->dsrc, nn * sizeof(int4)) != cudaSuccess ||
-        cudaMalloc(&P->pos, nn * sizeof(uint16_t)) != cudaSuccess ||
-        cudaMalloc(&P->lmask, size_t(P->ntiles) * kTriChunks * sizeof(uint32_t)) != cudaSuccess ||
-        cudaMalloc(&P->lvlptr, size_t(P->ntiles) * (kTriTile + 1) * sizeof(int32_t)) != cudaSuccess ||
-        cudaMalloc(&P->nlev, size_t(P->ntiles) * sizeof(int32_t)) != cudaSuccess ||
-        cudaMalloc(&P->dpos, nn * sizeof(int32_t)) != cudaSuccess ||
-        cudaMalloc(&P->flags, (nn + 1) * sizeof(unsigned)) != cudaSuccess ||
-        cudaMalloc(&P->err, 2 * sizeof(int)) != cudaSuccess || cudaMalloc(&beg, nn * sizeof(int32_t)) != cudaSuccess ||
-        cudaMalloc(&cnt, nn * sizeof(int32_t)) != cudaSuccess || cudaMalloc(&missing, sizeof(int)) != cudaSuccess ||
-        cudaMalloc(&glev, nn * sizeof(int32_t)) != cudaSuccess ||
-        cudaMalloc(&chain, (size_t(P->ntiles) + 1) * sizeof(unsigned)) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(HPB_ERROR_OUT_OF_MEMORY, "device allocation failed");
-    }
+    P->block = fused::analysis_alloc(keep, s);
+    work = static_cast<char*>(fused::analysis_alloc(tmp, s));
+    if (P->block == nullptr || work == nullptr) return fail(HPB_ERROR_OUT_OF_MEMORY, "device allocation failed");
+    char* blk = static_cast<char*>(P->block);
+    P->desc = reinterpret_cast<int4*>(blk + o_desc);
+    P->dsrc = reinterpret_cast<int4*>(blk + o_dsrc);
+    P->pos = reinterpret_cast<uint16_t*>(blk + o_pos);
+    P->lmask = reinterpret_cast<uint32_t*>(blk + o_lmask);
+    P->lvlptr = reinterpret_cast<int32_t*>(blk + o_lvl);
+    P->dpos = reinterpret_cast<int32_t*>(blk + o_dpos);
+    P->flags = reinterpret_cast<unsigned*>(blk + o_flags);
+    P->err = reinterpret_cast<int*>(blk + o_err);
     P->err_row = P->err + 1;
-    const int init[2] = {0, INT_MAX};
+    P->nlev = P->err + 4;
+    int* missing = P->err + 2;
+    int32_t* beg = reinterpret_cast<int32_t*>(work + o_beg);
+    int32_t* cnt = reinterpret_cast<int32_t*>(work + o_cnt);
+    int32_t* glev = reinterpret_cast<int32_t*>(work + o_glev);
+    unsigned* ticket = reinterpret_cast<unsigned*>(work + o_tick);
+    const int init[4] = {0, INT_MAX, 0, 0};
     cudaMemcpyAsync(P->err, init, sizeof(init), cudaMemcpyHostToDevice, s);
-    cudaMemsetAsync(missing, 0, sizeof(int), s);
+    cudaMemsetAsync(glev, 0xFF, nn * sizeof(int32_t), s);
+    cudaMemsetAsync(ticket, 0, sizeof(unsigned), s);
     k_tri_rows<<<(n + 255) / 256, 256, 0, s>>>(n, nnz, P->upper, rp, ci, beg, cnt, P->dpos, P->err, missing);
-    const size_t lv_smem = size_t(kTriTile) * 2 * sizeof(int);
-    cudaMemsetAsync(chain, 0, (size_t(P->ntiles) + 1) * sizeof(unsigned), s);
-    if (P->upper) {
-        allow_smem(k_tri_levels<true>, lv_smem);
-        k_tri_levels<true><<<P->ntiles, kLvThreads, lv_smem, s>>>(n, P->ntiles, ci, beg, cnt, glev, chain, P->err);
-    } else {
-        allow_smem(k_tri_levels<false>, lv_smem);
-        k_tri_levels<false><<<P->ntiles, kLvThreads, lv_smem, s>>>(n, P->ntiles, ci, beg, cnt, glev, chain, P->err);
-    }
+    auto levels = P->upper ? k_tri_levels<true> : k_tri_levels<false>;
+    allow_smem(levels, sizeof(LevelTile));
+    levels<<<P->ntiles, kGlThreads, sizeof(LevelTile), s>>>(n, P->ntiles, ci, beg, cnt, glev, ticket, P->err);
     const size_t sort_smem = size_t(kTriTile) * (sizeof(unsigned long long) + sizeof(uint16_t));
     allow_smem(k_tri_sort, sort_smem);
     k_tri_sort<<<P->ntiles, kSortThreads, sort_smem, s>>>(n, ci, beg, cnt, P->dpos, glev, P->desc, P->dsrc, P->pos,
                                                           P->lmask, P->lvlptr, P->nlev);
     count_launch(3);
     if (cudaGetLastError() != cudaSuccess) return fail(HPB_ERROR_CUDA, "analysis launch failed");
-    int host_err = 0, host_missing = 0;
-    std::vector<int32_t> lev(size_t(P->ntiles));
-    if (cudaMemcpyAsync(&host_err, P->err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemcpyAsync(&host_missing, missing, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemcpyAsync(lev.data(), P->nlev, lev.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, s) !=
-            cudaSuccess ||
+    std::vector<int32_t> got(4 + nt);  // err, err_row, missing, -, nlev
+    if (cudaMemcpyAsync(got.data(), P->err, got.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
         return fail(HPB_ERROR_CUDA, "analysis failed");
-    cudaFree(beg);
-    cudaFree(cnt);
-    cudaFree(glev);
-    cudaFree(chain);
-    cudaFree(missing);
-    beg = cnt = glev = nullptr;
-    chain = nullptr;
-    missing = nullptr;
-    if (host_err & kErrColumn) return fail(HPB_ERROR_INVALID_VALUE, "row pointer or column index out of range");
-    if (host_err & kErrUnsorted)
+    if (got[0] & kErrColumn) return fail(HPB_ERROR_INVALID_VALUE, "row pointer or column index out of range");
+    if (got[0] & kErrUnsorted)
         return fail(HPB_ERROR_INVALID_VALUE, "column indices of a row are not strictly increasing");
-    P->all_diag = host_missing == 0;
-    for (int32_t v : lev) {
-        P->max_levels = std::max(P->max_levels, v);
-        P->sum_levels += v;
+    if (got[0] & kErrTimeout) return fail(HPB_ERROR_TIMEOUT, "a bounded device-side wait gave up");
+    fused::analysis_free(work, s);
+    P->all_diag = got[2] == 0;
+    for (size_t t = 0; t < nt; ++t) {
+        P->max_levels = std::max(P->max_levels, got[4 + t]);
+        P->sum_levels += got[4 + t];
     }
     return HPB_SUCCESS;
 }
 
+// As cudaFree would, this waits for the device: solves with the analysis may
+// still be running on any stream.
 void release(Plan* P) {
-    cudaFree(P->desc);
-    cudaFree(P->dsrc);
-    cudaFree(P->pos);
-    cudaFree(P->lmask);
-    P->dsrc = nullptr;
+    int dev = 0;
+    const bool other = cudaGetDevice(&dev) == cudaSuccess && dev != P->device;
+    if (other) cudaSetDevice(P->device);
+    if (P->block != nullptr || P->scratch != nullptr) cudaDeviceSynchronize();
+    fused::analysis_free(P->block, nullptr);
+    cudaFree(P->scratch);
+    if (other) cudaSetDevice(dev);
+    P->block = P->scratch = nullptr;
+    P->desc = P->dsrc = nullptr;
     P->pos = nullptr;
     P->lmask = nullptr;
-    cudaFree(P->lvlptr);
-    cudaFree(P->nlev);
-    cudaFree(P->dpos);
-    cudaFree(P->flags);
-    cudaFree(P->err);
-    cudaFree(P->scratch);
-    P->scratch = nullptr;
-    P->desc = nullptr;
     P->lvlptr = P->nlev = P->dpos = nullptr;
     P->flags = nullptr;
     P->err = P->err_row = nullptr;

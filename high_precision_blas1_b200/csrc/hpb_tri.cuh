@@ -46,6 +46,7 @@ struct Plan {
     int64_t sum_levels = 0;         // levels summed over tiles
     const int32_t* rp = nullptr;    // caller's structure; must stay valid and unchanged
     const int32_t* ci = nullptr;
+    void* block = nullptr;          // the allocation that holds the arrays below, up to err_row
     int4* desc = nullptr;           // n: (row, first dependency, dependency count, diagonal position) in level order
     int4* dsrc = nullptr;           // n: where each of the first four dependencies is found, in level order
     uint16_t* pos = nullptr;        // n: position of each row in its tile's level order
@@ -54,9 +55,9 @@ struct Plan {
     int32_t* nlev = nullptr;        // ntiles
     int32_t* dpos = nullptr;        // n: position of the diagonal entry of each row, -1 if absent
     unsigned* flags = nullptr;      // n + 1: per-row done flags (factorization), then the tile ticket
-    void* scratch = nullptr;        // n * 16 bytes, allocated on the first in-place solve
     int* err = nullptr;             // error bits
     int* err_row = nullptr;         // ILU(0): first row with a zero pivot
+    void* scratch = nullptr;        // n * 16 bytes, allocated on the first in-place solve
     unsigned long long wait_ns = 0; // solve: limit of each bounded wait (0: the default, 4 s)
     int32_t withhold_row = -1;      // solve, testing aid: this row's value is never published to x
 };

@@ -552,7 +552,9 @@ int hpb_csr_solve_c128_host(const hpb_solver_params* p, int32_t rows, int64_t nn
  * (Krylov vectors: (l + 1) or (m + 1) vectors of n elements, plus a few)
  * from a library-owned stream-ordered memory pool per device that keeps
  * freed blocks for the next solve, so repeated solves neither call
- * cudaMalloc/cudaFree nor synchronise the device.  This returns the pool's
+ * cudaMalloc/cudaFree nor synchronise the device.  The triangular analyses
+ * (hpb_csr_tri_create) take their arrays from a second pool of that kind,
+ * which gives freed memory back once it has more than 1 GiB in all.  This returns both pools'
  * unused memory to the device (no counterpart in the reference, whose
  * vector objects allocate and free their own buffers). */
 int hpb_solver_memory_release(void);
