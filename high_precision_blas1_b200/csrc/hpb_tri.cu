@@ -1090,7 +1090,212 @@ k_tri_sweep(int32_t n, const int32_t* __restrict__ rp, const int32_t* __restrict
     }
 }
 
-// ---- ILU(0) ---------------------------------------------------------------
+// ---- ILU(0), diagonal updates only ----------------------------------------
+// Where no entry of row i beside its diagonal lies in the pattern of a row k
+// it eliminates (a graph without triangles, as that of every 5- and 7-point
+// stencil), eliminating k from row i changes a_ii alone:
+//     l_ik = a_ik / d_k,   d_i = a_ii - sum_k l_ik a_ki  (k ascending),
+// with a_ik, a_ki still the matrix' own values.  The factorization is then a
+// recurrence in one value per row, run like a triangular solve: the same
+// chunks of the level order, d by position in shared memory and published
+// once to a sentinel-filled array for the other tiles.  The operations are
+// those of the general kernel (k_ilu0) in the same order, so the same bits.
+// Measured on B200 (f64, 1024^2 5-point operator): 1.45 ms with its pattern
+// check, against 15.6 ms for the general kernel, whose every level (7.6 us) is a chain of
+// dependent loads from L2 and fences.
+// k_ilu0_pattern finds for each of a row's first kPre dependencies where row
+// k holds column i (wpos, in level order; -1: nowhere) and sets *general if
+// the matrix is not of that kind or a row has more dependencies.
+__global__ void k_ilu0_pattern(int32_t n, const int4* __restrict__ desc, const int32_t* __restrict__ rp,
+                               const int32_t* __restrict__ ci, const int32_t* __restrict__ dpos,
+                               int4* __restrict__ wpos, int* general) {
+    const int32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    const int4 d = desc[p];
+    int w[kPre] = {-1, -1, -1, -1};
+    bool gen = d.z > kPre;
+    const int32_t end = __ldg(rp + d.x + 1);
+#pragma unroll
+    for (int q = 0; q < kPre; ++q) {
+        if (q >= d.z || gen) continue;
+        const int32_t k = __ldg(ci + d.y + q);
+        int32_t a = d.y + q + 1, b = __ldg(dpos + k) + 1;
+        const int32_t bend = __ldg(rp + k + 1);
+        while (a < end && b < bend) {  // the common columns past k
+            const int32_t ca = __ldg(ci + a), cb = __ldg(ci + b);
+            if (ca == cb) {
+                if (ca == d.x)
+                    w[q] = b;
+                else
+                    gen = true;
+                ++a;
+                ++b;
+            } else if (ca < cb) {
+                ++a;
+            } else {
+                ++b;
+            }
+        }
+    }
+    wpos[p] = make_int4(w[0], w[1], w[2], w[3]);
+    if (gen) *general = 1;
+}
+
+// A diagonal value that happens to be the sentinel (only a signalling NaN in
+// the input can be) is published as a quiet one.
+__device__ __forceinline__ double publishable(double v) {
+    return Pub<double>::pending(v) ? __longlong_as_double(0x7FF8000000000000ll) : v;
+}
+__device__ __forceinline__ float publishable(float v) { return Pub<float>::pending(v) ? __int_as_float(0x7FC00000) : v; }
+template <class C>
+__device__ __forceinline__ C publishable(C v) { return C{publishable(v.re), publishable(v.im)}; }
+template <class E> __device__ __forceinline__ E one_of();
+template <> __device__ __forceinline__ float one_of<float>() { return 1.f; }
+template <> __device__ __forceinline__ double one_of<double>() { return 1.0; }
+template <> __device__ __forceinline__ cf one_of<cf>() { return cf{1.f, 0.f}; }
+template <> __device__ __forceinline__ cd one_of<cd>() { return cd{1.0, 0.0}; }
+
+template <class E>
+struct PivotRow {
+    int4 d, s, w;
+    uint32_t starts;
+    E diag, v[kPre], u[kPre];  // a_ii, a_ik, a_ki
+};
+
+template <class E>
+__global__ void __launch_bounds__(kSolveThreads, 1)
+k_ilu0_diag(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int4* __restrict__ dsrc,
+            const uint32_t* __restrict__ lmask, const int4* __restrict__ wpos, E* val, E* piv, unsigned* ticket,
+            const int* __restrict__ general, int* err, int* err_row) {
+    if (*general) return;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    TileValues<E>& T = *reinterpret_cast<TileValues<E>*>(smraw);
+    __shared__ int s_tile;
+    if (threadIdx.x == 0) s_tile = int(atomicAdd(ticket, 1u));
+    __syncthreads();
+    const int t = s_tile;
+    if (t >= ntiles) return;
+    const int32_t base = int32_t(t) * kTriTile;
+    const int32_t m = min(kTriTile, n - base);
+    const int nc = (m + 31) >> 5;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    desc += base;
+    dsrc += base;
+    wpos += base;
+    lmask += size_t(t) * kTriChunks;
+
+    auto idx = [&](PivotRow<E>& r, int c) {
+        const int32_t p = 32 * c + lane;
+        r.d = make_int4(-1, 0, 0, -1);
+        r.s = make_int4(-1, -1, -1, -1);
+        r.w = r.s;
+        r.starts = 0u;
+        if (p < m) {
+            r.d = __ldg(desc + p);
+            r.s = __ldg(dsrc + p);
+            r.w = __ldg(wpos + p);
+        }
+        if (c < nc) r.starts = __ldg(lmask + c);
+    };
+    // (the entries read here are written by their own row's lane alone, later)
+    auto values = [&](PivotRow<E>& r) {
+        if (r.d.x < 0) return;
+        r.diag = ldE(val, r.d.w);
+#pragma unroll
+        for (int k = 0; k < kPre; ++k)
+            if (k < r.d.z) {
+                r.v[k] = ldE(val, int64_t(r.d.y) + k);
+                if (at4(r.w, k) >= 0) r.u[k] = ldE(val, at4(r.w, k));
+            }
+    };
+    PivotRow<E> r{}, nx{};
+    idx(r, w);
+    idx(nx, w + kSolveWarps);
+    values(r);
+    for (int c = w; c < nc; c += kSolveWarps) {
+        // in flight meanwhile (complex<double> rows fill the registers as they are: its next values come after the turn)
+        constexpr bool kAhead = sizeof(E) < 16;
+        PivotRow<E> nn{};
+        if (kAhead) values(nx);
+        idx(nn, c + 2 * kSolveWarps);
+        const E* src[kPre];
+        unsigned pend = 0;
+#pragma unroll
+        for (int k = 0; k < kPre; ++k) {
+            const int sk = at4(r.s, k);
+            src[k] = sk >= 0 ? T.xs + sk : &T.ext[w][k][lane];
+            if (sk == -1) T.ext[w][k][lane] = one_of<E>();
+            if (sk <= -2) pend |= 1u << k;
+        }
+        const uint32_t starts = r.starts | 1u;
+        const int steps = __popc(starts);
+        const int mine = r.d.x >= 0 ? __popc(starts & ((2u << lane) - 1u)) : 0;
+        const int most = __reduce_max_sync(0xffffffffu, r.d.z);
+        if (pend != 0u) {
+            Waiter wt;
+            for (;;) {
+                E xe[kPre];
+#pragma unroll
+                for (int k = 0; k < kPre; ++k)
+                    if ((pend >> k) & 1u) xe[k] = Pub<E>::load(piv, -at4(r.s, k) - 2);
+                const bool stop = wt.check(err, 63);
+#pragma unroll
+                for (int k = 0; k < kPre; ++k)
+                    if (((pend >> k) & 1u) && (stop || !Pub<E>::pending(xe[k]))) {
+                        T.ext[w][k][lane] = xe[k];
+                        pend &= ~(1u << k);
+                    }
+                if (pend == 0u) break;
+            }
+        }
+        __syncwarp();
+        if (c > 0) chunk_sync(w == 0 ? kSolveWarps - 1 : w - 1);
+        E piv_i{}, l[kPre];
+#pragma unroll 1
+        for (int s = 1; s <= steps; ++s) {
+            const bool on = mine == s;
+            E acc = r.diag, q[kPre];
+#pragma unroll
+            for (int k = 0; k < kPre; ++k)
+                if (k < most) {  // the same for the whole warp
+                    // lanes that are not at this level divide 1 by 1: no slow path for what they hold
+                    const bool has = on && k < r.d.z;
+                    q[k] = quot(has ? r.v[k] : one_of<E>(), has ? *src[k] : one_of<E>());
+                }
+#pragma unroll
+            for (int k = 0; k < kPre; ++k)
+                if (k < most) {
+                    const E f = fms(acc, q[k], r.u[k]);
+                    acc = (k < r.d.z && at4(r.w, k) >= 0) ? f : acc;
+                }
+            if (on) {
+                T.xs[32 * c + lane] = acc;
+                piv_i = acc;
+#pragma unroll
+                for (int k = 0; k < kPre; ++k) l[k] = q[k];
+            }
+            __syncwarp();
+            if (on) Pub<E>::store(piv, r.d.x, publishable(acc));
+        }
+        __syncwarp();
+        if (c + 1 < nc) chunk_arrive(w);
+        if (r.d.x >= 0) {
+            stE(val, r.d.w, piv_i);
+#pragma unroll
+            for (int k = 0; k < kPre; ++k)
+                if (k < r.d.z) stE(val, int64_t(r.d.y) + k, l[k]);
+            if (zero_of(piv_i)) {
+                atomicOr(err, kErrZeroPivot);
+                atomicMin(err_row, r.d.x);
+            }
+        }
+        if (!kAhead) values(nx);
+        r = nx;
+        nx = nn;
+    }
+}
+
+// ---- ILU(0), general ------------------------------------------------------
 // Row i, for each strictly lower entry k (ascending): l_ik = a_ik / u_kk,
 // then a_ij -= l_ik u_kj for every j > k present in both rows (the IKJ
 // variant of ILU(0), Saad, Iterative Methods for Sparse Linear Systems,
@@ -1102,7 +1307,9 @@ template <class E>
 __global__ void __launch_bounds__(kTriThreads)
 k_ilu0(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int32_t* __restrict__ lvlptr,
        const int32_t* __restrict__ nlev, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
-       const int32_t* __restrict__ dpos, E* val, unsigned* flags, int* err, int* err_row) {
+       const int32_t* __restrict__ dpos, E* val, unsigned* flags, const int* __restrict__ general, int* err,
+       int* err_row) {
+    if (!*general) return;  // k_ilu0_diag has done it
     __shared__ int s_tile;
     __shared__ int s_done;
     if (threadIdx.x == 0) {
@@ -1346,12 +1553,30 @@ cudaError_t launch_trsv_sweeps(const Plan& P, int unit, const E* val, E alpha, c
 template <class E>
 cudaError_t launch_ilu0(const Plan& P, E* val, cudaStream_t s) {
     if (P.n == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(P.flags, 0, (size_t(P.n) + 1) * sizeof(unsigned), s);
-    if (e != cudaSuccess) return e;
-    k_ilu0<E><<<P.ntiles, kTriThreads, 0, s>>>(P.n, P.ntiles, P.desc, P.lvlptr, P.nlev, P.rp, P.ci, P.dpos, val,
-                                               P.flags, P.err, P.err_row);
-    count_launch();
-    return cudaGetLastError();
+    // scratch: the published diagonal, the positions of a_ki, the tile ticket and the kind of matrix
+    const size_t o_piv = (size_t(P.n) * sizeof(int4) + 255) & ~size_t(255);
+    const size_t o_word = (o_piv + size_t(P.n) * sizeof(E) + 255) & ~size_t(255);
+    char* work = static_cast<char*>(fused::analysis_alloc(o_word + 8, s));
+    if (work == nullptr) return cudaErrorMemoryAllocation;
+    int4* wpos = reinterpret_cast<int4*>(work);
+    E* piv = reinterpret_cast<E*>(work + o_piv);
+    unsigned* ticket = reinterpret_cast<unsigned*>(work + o_word);
+    int* general = reinterpret_cast<int*>(work + o_word + 4);
+    cudaError_t e = cudaMemsetAsync(general, 0, sizeof(int), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(P.flags, 0, (size_t(P.n) + 1) * sizeof(unsigned), s);
+    if (e == cudaSuccess) {
+        k_ilu0_pattern<<<(P.n + 255) / 256, 256, 0, s>>>(P.n, P.desc, P.rp, P.ci, P.dpos, wpos, general);
+        k_tri_fill<E><<<int(std::min<int64_t>((int64_t(P.n) + 255) / 256, 148 * 8)), 256, 0, s>>>(P.n, piv, ticket);
+        allow_smem(k_ilu0_diag<E>, sizeof(TileValues<E>));
+        k_ilu0_diag<E><<<P.ntiles, kSolveThreads, sizeof(TileValues<E>), s>>>(
+            P.n, P.ntiles, P.desc, P.dsrc, P.lmask, wpos, val, piv, ticket, general, P.err, P.err_row);
+        k_ilu0<E><<<P.ntiles, kTriThreads, 0, s>>>(P.n, P.ntiles, P.desc, P.lvlptr, P.nlev, P.rp, P.ci, P.dpos, val,
+                                                   P.flags, general, P.err, P.err_row);
+        count_launch(4);
+        e = cudaGetLastError();
+    }
+    fused::analysis_free(work, s);
+    return e;
 }
 
 template cudaError_t launch_trsv<float>(const Plan&, int, const float*, float, const float*, float*, cudaStream_t);
