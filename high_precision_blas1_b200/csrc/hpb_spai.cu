@@ -32,9 +32,11 @@
 // (diffusion); the Frobenius gradient uses Ah^T = Ah.
 //
 // No counterpart in the reference (which has no learned component).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include <cuda_bf16.h>
@@ -46,21 +48,7 @@
 namespace hpb {
 namespace spai {
 
-constexpr int kMaxSlot = 8, kMaxSq = 64;
 constexpr int kThreads = 256;
-
-struct Offsets {
-    int nslot, dslot;
-    int off[kMaxSlot];
-    // A^2 pattern: nsq distinct offsets; sq[p][q] = index of off[p] + off[q]
-    int nsq;
-    int sqoff[kMaxSq];
-    int sq[kMaxSlot][kMaxSlot];
-    // index of off[q] - off[p] in sqoff (-1 if absent)
-    int dq[kMaxSlot][kMaxSlot];
-    // slot of -off[s] (the transposed entry), -1 if absent
-    int rev[kMaxSlot];
-};
 
 __device__ __forceinline__ int slot_of(const Offsets& o, int d) {
     for (int s = 0; s < o.nslot; ++s)
@@ -69,8 +57,6 @@ __device__ __forceinline__ int slot_of(const Offsets& o, int d) {
 }
 
 // ---------------------------------------------------------------- features
-__device__ __forceinline__ float inv_sqrt_dd(float di, float dj) { return 1.f / sqrtf(fabsf(di * dj)); }
-
 __global__ void k_features(int32_t rows, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
                            const float* __restrict__ val, const float* __restrict__ diag,
                            const double* __restrict__ lsum, Offsets o, float* __restrict__ feat) {
@@ -286,6 +272,243 @@ k_forward(int32_t rows, const float* __restrict__ feat, const __nv_bfloat16* __r
     }
 }
 
+// ---------------------------------------------------------------- slot form
+// A system whose rows hold each slot at most once, in slot order, and nothing
+// outside the slots -- every stencil matrix -- is worked on in slot form: entry
+// (i, i + off[s]) at [s * n + i], so consecutive threads read consecutive
+// words at every slot and its neighbours, and no kernel searches a row for a
+// column.  k_slot_load finds out; a system of any other kind takes the CSR
+// kernels (k_features and on).  Sums over all rows are merged per block and
+// then by the last block, nothing of them passes through the host.
+constexpr int kSlotThreads = 128;
+constexpr int kMaxRes = 4;  // residual samples the slot form takes
+
+struct SlotMats {  // training workspace, all slot form: [.. * n + i]
+    int32_t n;
+    const uint8_t* mask;
+    const float *ah, *th;  // Ah, tanh of the outputs
+    float *mh, *y, *z, *rh, *G, *dm;
+    double* lpart;         // block sums of ||G||^2 and ||z_s||^2
+    const double* sums;    // [0] sum of logs, [1 + s] ||rh_s||^2
+    int nres;
+};
+
+// CSR -> slot form; the sum of log|a_ii| and rh_s = r_s / sqrt|a_ii| with
+// ||rh_s||^2 (all Dot2-merged).  *irregular: the system is not of that kind.
+// Rows in a grid-stride loop: with a block for every 128 rows the tickets of
+// the 6912 blocks at 96^3 took longer than the rows (43 against 24 us).
+// A row's entries are matched in one walk over the slots (a search of the
+// slots for each entry took 1000 instructions a row, 38 us at 96^3).
+// NR < 0: the build (no samples; the tables sd, ld instead of diag).
+template <int NR>
+__global__ void __launch_bounds__(kSlotThreads)
+k_slot_load(int32_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const float* __restrict__ val,
+            Offsets o, const float* __restrict__ res, float* __restrict__ raw, uint8_t* __restrict__ mask,
+            float* __restrict__ diag, double* __restrict__ sd, double* __restrict__ ld, float* __restrict__ rh,
+            double* sums, fused::Acc2* partials, unsigned* ticket, int* badflag, int* irregular) {
+    constexpr int ND = NR < 0 ? 1 : 1 + NR;
+    fused::Acc2 acc[ND];
+    bool bad = false;
+    for (int32_t i = blockIdx.x * kSlotThreads + threadIdx.x; i < n; i += gridDim.x * kSlotThreads) {
+        unsigned m = 0;
+        const int32_t e = __ldg(rp + i + 1);
+        int32_t k = __ldg(rp + i);
+        float dv = 0.f;
+#pragma unroll
+        for (int q = 0; q < kMaxSlot; ++q)
+            if (q < o.nslot) {
+                float v = 0.f;
+                if (k < e && __ldg(ci + k) - i == o.off[q]) {
+                    v = __ldg(val + k);
+                    m |= 1u << q;
+                    ++k;
+                }
+                raw[size_t(q) * n + i] = v;
+                if (q == o.dslot) dv = v;
+            }
+        bad |= k != e;  // an entry outside the slots, twice, or out of order
+        mask[i] = uint8_t(m);
+        const double ad = fabs(double(dv)), l = log(ad);
+        if constexpr (NR < 0) {
+            sd[i] = rsqrt(ad);
+            ld[i] = l;
+        } else {
+            diag[i] = dv;
+        }
+        fused::merge2(acc[0].s, acc[0].c, l, 0.0);
+#pragma unroll
+        for (int s = 0; s < NR; ++s) {
+            const float v = __ldg(res + size_t(s) * n + i) / sqrtf(fabsf(dv));
+            rh[size_t(s) * n + i] = v;
+            fused::dot_add(acc[1 + s], double(v), double(v));
+        }
+    }
+    fused::grid_finish_acc<ND>(acc, bad, partials, ticket, badflag, [&](const fused::Acc2* tot, bool anybad) {
+#pragma unroll
+        for (int s = 0; s < ND; ++s) sums[s] = tot[s].s + tot[s].c;
+        *irregular = anybad ? 1 : 0;
+    });
+}
+
+// Row i's Mh by slot, from t = tanh of the outputs.
+__device__ __forceinline__ void slot_mh(int32_t n, int32_t i, unsigned m, const float* __restrict__ th, const Offsets& o,
+                                        float (&mh)[kMaxSlot]) {
+    float sum = 0.f;
+#pragma unroll
+    for (int s = 0; s < kMaxSlot; ++s) {
+        mh[s] = 0.f;
+        if (s >= o.nslot || s == o.dslot || !((m >> s) & 1u)) continue;
+        const int rs = o.rev[s];
+        if (rs < 0) continue;
+        const float S = 0.25f * (__ldg(th + size_t(s) * n + i) + __ldg(th + size_t(rs) * n + (i + o.off[s])));
+        sum += fabsf(S);
+        mh[s] = S;
+    }
+    const float md = 1.f + 0.5f * __ldg(th + size_t(o.dslot) * n + i) + sum;
+#pragma unroll
+    for (int s = 0; s < kMaxSlot; ++s)
+        if (s == o.dslot && ((m >> s) & 1u)) mh[s] = md;
+}
+
+// M = D^{-1/2} Mh D^{-1/2} at A's CSR positions (the build): the row's entries
+// are its slots in order.
+__global__ void __launch_bounds__(kSlotThreads)
+k_slot_assemble(int32_t n, const int32_t* __restrict__ rp, const uint8_t* __restrict__ mask,
+                const double* __restrict__ sd, const float* __restrict__ th, Offsets o,
+                const int* __restrict__ irregular, float* __restrict__ mval) {
+    const int32_t i = blockIdx.x * kSlotThreads + threadIdx.x;
+    if (i >= n || *irregular) return;
+    const unsigned m = __ldg(mask + i);
+    float mh[kMaxSlot];
+    slot_mh(n, i, m, th, o, mh);
+    const double sdi = __ldg(sd + i);
+    int32_t k = __ldg(rp + i);
+#pragma unroll
+    for (int s = 0; s < kMaxSlot; ++s)
+        if (s < o.nslot && ((m >> s) & 1u)) mval[k++] = mh[s] * float(sdi * __ldg(sd + (i + o.off[s])));
+}
+
+// Training, after the forward: Mh, and y_s = Mh rh_s for every sample.
+__global__ void __launch_bounds__(kSlotThreads) k_slot_mh(SlotMats w, Offsets o) {
+    const int32_t n = w.n, i = blockIdx.x * kSlotThreads + threadIdx.x;
+    if (i >= n) return;
+    const unsigned m = __ldg(w.mask + i);
+    float mh[kMaxSlot];
+    slot_mh(n, i, m, w.th, o, mh);
+#pragma unroll
+    for (int s = 0; s < kMaxSlot; ++s)
+        if (s < o.nslot) w.mh[size_t(s) * n + i] = mh[s];
+    for (int r = 0; r < w.nres; ++r) {
+        float y = 0.f;
+#pragma unroll
+        for (int s = 0; s < kMaxSlot; ++s)
+            if (s < o.nslot && ((m >> s) & 1u)) y = fmaf(mh[s], __ldg(w.rh + size_t(r) * n + (i + o.off[s])), y);
+        w.y[size_t(r) * n + i] = y;
+    }
+}
+
+// sum over the block of v (binary64, a fixed tree), valid in thread 0
+__device__ __forceinline__ double slot_block_sum(double v) {
+    __shared__ double sh[kSlotThreads / 32];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = 0.0;
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int q = 0; q < kSlotThreads / 32; ++q) v += sh[q];
+    return v;
+}
+
+// Plane t < nsq: entry t of G = Ah Mh - I, one thread per row (its pairs of
+// slots come from qof: off[p] + off[qof[t][p]] = sqoff[t]); plane nsq + s:
+// z_s = Ah y_s - rh_s.  Block sums of the squares in lpart[plane][block].
+struct PairTable { signed char q[kMaxSq][kMaxSlot]; };
+__global__ void __launch_bounds__(kSlotThreads) k_slot_gz(SlotMats w, Offsets o, PairTable pt) {
+    const int32_t n = w.n, i = blockIdx.x * kSlotThreads + threadIdx.x;
+    const int t = blockIdx.y;
+    float v = 0.f;
+    if (i < n) {
+        const unsigned m = __ldg(w.mask + i);
+        if (t < o.nsq) {
+#pragma unroll
+            for (int p = 0; p < kMaxSlot; ++p) {
+                const int q = pt.q[t][p];
+                if (p >= o.nslot || q < 0 || !((m >> p) & 1u)) continue;
+                const int32_t k = i + o.off[p];
+                if ((__ldg(w.mask + k) >> q) & 1u)
+                    v = fmaf(__ldg(w.ah + size_t(p) * n + i), __ldg(w.mh + size_t(q) * n + k), v);
+            }
+            if (o.sqoff[t] == 0) v -= 1.f;
+            w.G[size_t(t) * n + i] = v;
+        } else {
+            const int s = t - o.nsq;
+#pragma unroll
+            for (int p = 0; p < kMaxSlot; ++p)
+                if (p < o.nslot && ((m >> p) & 1u))
+                    v = fmaf(__ldg(w.ah + size_t(p) * n + i), __ldg(w.y + size_t(s) * n + (i + o.off[p])), v);
+            v -= __ldg(w.rh + size_t(s) * n + i);
+            w.z[size_t(s) * n + i] = v;
+        }
+    }
+    const double l = slot_block_sum(double(v) * double(v));
+    if (threadIdx.x == 0) w.lpart[size_t(t) * gridDim.x + blockIdx.x] = l;
+}
+
+// dm = dL/dMh: slot q = blockIdx.y of row k,
+//   wf 2 sum_p Ah_{k,p} G[k + off_p][off_q - off_p]  +  sum_s wr_s 2 g_s rh_s[j],  g_s = (Ah z_s)_k
+// (Ah symmetric), wr_s = w_resid / (||rh_s||^2 nres); a sample of norm 0 adds nothing.
+__global__ void __launch_bounds__(kSlotThreads) k_slot_dm(SlotMats w, Offsets o, float wf, float w_resid) {
+    const int32_t n = w.n, k = blockIdx.x * kSlotThreads + threadIdx.x;
+    const int q = blockIdx.y;
+    if (k >= n) return;
+    const unsigned m = __ldg(w.mask + k);
+    float dm = 0.f;
+    if ((m >> q) & 1u) {
+        float s = 0.f, a[kMaxSlot];
+#pragma unroll
+        for (int p = 0; p < kMaxSlot; ++p) {
+            a[p] = 0.f;
+            if (p >= o.nslot || !((m >> p) & 1u)) continue;
+            a[p] = __ldg(w.ah + size_t(p) * n + k);
+            const int t = o.dq[p][q];
+            if (t >= 0) s = fmaf(a[p], __ldg(w.G + size_t(t) * n + (k + o.off[p])), s);
+        }
+        dm = wf * 2.f * s;
+        const int32_t j = k + o.off[q];
+        for (int r = 0; r < w.nres; ++r) {
+            const double rr = __ldg(w.sums + 1 + r);
+            if (!(rr > 0.0)) continue;
+            const float wr = float(double(w_resid) / (rr * w.nres));
+            float g = 0.f;
+#pragma unroll
+            for (int p = 0; p < kMaxSlot; ++p)
+                if (p < o.nslot && ((m >> p) & 1u)) g = fmaf(a[p], __ldg(w.z + size_t(r) * n + (k + o.off[p])), g);
+            dm = fmaf(wr * 2.f * g, __ldg(w.rh + size_t(r) * n + j), dm);
+        }
+    }
+    w.dm[size_t(q) * n + k] = dm;
+}
+
+// dL/do_{i,s} (k_dout's formula) from dm and tanh of the outputs in slot form
+__device__ __forceinline__ float slot_dout(const SlotMats& w, const Offsets& o, int32_t i, int s) {
+    const int32_t n = w.n;
+    const unsigned m = __ldg(w.mask + i);
+    if (s >= o.nslot || !((m >> s) & 1u)) return 0.f;
+    auto dm = [&](unsigned mr, int q, int32_t r) { return ((mr >> q) & 1u) ? __ldg(w.dm + size_t(q) * n + r) : 0.f; };
+    const float dmii = dm(m, o.dslot, i), ti = __ldg(w.th + size_t(s) * n + i);
+    if (s == o.dslot) return 0.5f * (1.f - ti * ti) * dmii;
+    const int rs = o.rev[s];
+    if (rs < 0) return 0.f;
+    const int32_t j = i + o.off[s];
+    const unsigned mj = __ldg(w.mask + j);
+    const float S = 0.25f * (ti + __ldg(w.th + size_t(rs) * n + j));
+    const float sg = S > 0.f ? 1.f : (S < 0.f ? -1.f : 0.f);
+    return 0.25f * (1.f - ti * ti) *
+           (__ldg(w.dm + size_t(s) * n + i) + dm(mj, rs, j) + sg * (dmii + dm(mj, o.dslot, j)));
+}
+
 // Backward pass on tensor cores.  A block of kMmaWarps warps takes chunks
 // of 16 * kMmaWarps rows:
 //   phase 1, per warp and its 16 rows, in registers:
@@ -329,10 +552,12 @@ __device__ __forceinline__ void col_pair(const float* a, int stride, int r, int 
     split2(a[r * stride + c], a[(r + 1) * stride + c], hi, lo);
 }
 
+// SLOTS: dL/dout is formed here from the slot-form workspace instead of read.
+template <bool SLOTS>
 __global__ void __launch_bounds__(kMmaWarps * 32, 1)
 k_backward(int32_t rows, const float* __restrict__ feat, const __nv_bfloat16* __restrict__ w,
-           const float* __restrict__ h1g, const float* __restrict__ h2g, const float* __restrict__ dout,
-           float* __restrict__ part) {
+           const float* __restrict__ h1g, const float* __restrict__ h2g, const float* __restrict__ dout, SlotMats sm,
+           Offsets o, float* __restrict__ part) {
     extern __shared__ __align__(16) unsigned char smraw[];
     float* sX = reinterpret_cast<float*>(smraw);   // kBwdRows x kSX
     float* sH1 = sX + kBwdRows * kSX;              // kBwdRows x kSH
@@ -360,11 +585,26 @@ k_backward(int32_t rows, const float* __restrict__ feat, const __nv_bfloat16* __
     const int nchunks = (rows + kBwdRows - 1) / kBwdRows;
     for (int ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
         // ---------------- phase 1: this warp's 16 rows
+        if constexpr (SLOTS) {
+            for (int f = threadIdx.x; f < kBwdRows * kO; f += kMmaWarps * 32) {
+                const int lr = f & (kBwdRows - 1), q = f / kBwdRows;
+                const int32_t row = ch * kBwdRows + lr;
+                sDO[lr * kSO + q] = row < rows ? slot_dout(sm, o, row, q) : 0.f;
+            }
+            __syncthreads();
+        }
         const int la = 16 * warp + g, lb = la + 8;  // rows within the chunk
         const int32_t ra = ch * kBwdRows + la, rb = ch * kBwdRows + lb;
         const bool va = ra < rows, vb = rb < rows;
         auto ld2 = [](const float* p, bool v) { return v ? *reinterpret_cast<const float2*>(p) : make_float2(0.f, 0.f); };
-        const float2 oa = ld2(dout + size_t(ra) * kO + 2 * t, va), ob = ld2(dout + size_t(rb) * kO + 2 * t, vb);
+        float2 oa, ob;
+        if constexpr (SLOTS) {
+            oa = *reinterpret_cast<const float2*>(sDO + la * kSO + 2 * t);
+            ob = *reinterpret_cast<const float2*>(sDO + lb * kSO + 2 * t);
+        } else {
+            oa = ld2(dout + size_t(ra) * kO + 2 * t, va);
+            ob = ld2(dout + size_t(rb) * kO + 2 * t, vb);
+        }
         uint32_t ah[4], al[4];
         split2(oa.x, oa.y, ah[0], al[0]);
         split2(ob.x, ob.y, ah[1], al[1]);
@@ -387,8 +627,10 @@ k_backward(int32_t rows, const float* __restrict__ feat, const __nv_bfloat16* __
             *reinterpret_cast<float2*>(sD2 + la * kSH + 8 * nt + 2 * t) = make_float2(d[nt][0], d[nt][1]);
             *reinterpret_cast<float2*>(sD2 + lb * kSH + 8 * nt + 2 * t) = make_float2(d[nt][2], d[nt][3]);
         }
-        *reinterpret_cast<float2*>(sDO + la * kSO + 2 * t) = oa;
-        *reinterpret_cast<float2*>(sDO + lb * kSO + 2 * t) = ob;
+        if constexpr (!SLOTS) {
+            *reinterpret_cast<float2*>(sDO + la * kSO + 2 * t) = oa;
+            *reinterpret_cast<float2*>(sDO + lb * kSO + 2 * t) = ob;
+        }
         {
             const float2 xa0 = ld2(feat + size_t(ra) * kF + 2 * t, va), xb0 = ld2(feat + size_t(rb) * kF + 2 * t, vb);
             const float2 xa1 = ld2(feat + size_t(ra) * kF + 8 + 2 * t, va);
@@ -503,6 +745,56 @@ __global__ void k_reduce_grad(int nblocks, const float* __restrict__ part, float
     for (int b = 0; b < nblocks; ++b) s += part[size_t(b) * kNumParams + p];
     gsys[p] = float(s);
     gacc[p] += float(s);
+}
+
+// The slot form's closing kernel: the gradient as k_reduce_grad (not taken up
+// if the system turned out irregular), and in the last block the losses
+// (total, Frobenius, residual) and *irregular into out[0..3].
+__global__ void __launch_bounds__(kSlotThreads)
+k_slot_close(int nblocks, const float* __restrict__ part, float* __restrict__ gsys, float* __restrict__ gacc,
+             SlotMats w, int nsq, int nb, float w_frob, float w_resid, const int* __restrict__ irregular,
+             double* __restrict__ out) {
+    if (blockIdx.x + 1 == gridDim.x) {
+        __shared__ double zs[kMaxRes];
+        const int lane = threadIdx.x & 31;
+        for (int r = threadIdx.x >> 5; r < w.nres; r += kSlotThreads / 32) {  // a warp per sample
+            double s = 0.0;
+            for (int b = lane; b < nb; b += 32) s += w.lpart[size_t(nsq + r) * nb + b];
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+            if (lane == 0) zs[r] = s;
+        }
+        double lf = 0.0, lr = 0.0;
+        for (int q = threadIdx.x; q < nsq * nb; q += kSlotThreads) lf += w.lpart[q];
+        __syncthreads();
+        lf = slot_block_sum(lf);
+        for (int r = 0; r < w.nres; ++r) {
+            const double rr = w.sums[1 + r];
+            if (rr > 0.0) lr += zs[r] / rr / w.nres;
+        }
+        if (threadIdx.x == 0) {
+            lf /= w.n;
+            out[0] = w_frob * lf + w_resid * lr;
+            out[1] = lf;
+            out[2] = lr;
+            out[3] = *irregular ? 1.0 : 0.0;
+        }
+        return;
+    }
+    const int p = blockIdx.x * kSlotThreads + threadIdx.x;
+    if (p >= kNumParams || nblocks == 0) return;
+    double s = 0.0;
+    int b = 0;
+    for (; b + 8 <= nblocks; b += 8) {  // eight loads in flight, added in order
+        float v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = __ldg(part + size_t(b + q) * kNumParams + p);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) s += v[q];
+    }
+    for (; b < nblocks; ++b) s += __ldg(part + size_t(b) * kNumParams + p);
+    gsys[p] = float(s);
+    if (!*irregular) gacc[p] += float(s);
 }
 
 // Adam on binary32 master weights, bf16 copy for the kernels
@@ -691,13 +983,22 @@ struct hpb_spai {
     double* lpart = nullptr;
     int part_blocks = 0;
     void* wimg = nullptr;        // the tcgen05 forward's weight image (rebuilt when wb changes)
-    int* tc_err = nullptr;       // mapped pinned word: a tensor-core wait ran out of time
+    int* tc_err = nullptr;       // mapped pinned: [0] a tensor-core wait ran out of time, [1] copy of *irregular
     int* tc_err_dev = nullptr;   // its device address
+    // slot form: the pairs of slots behind each entry of A^2, and the training workspace
+    hpb::spai::PairTable pairs{};
+    size_t slot_rows = 0;
+    char* slot_mem = nullptr;
+    unsigned* slot_sync = nullptr;  // ticket, bad flag, *irregular (each a line apart), behind part
+    double* slot_out = nullptr;     // out[4] of k_slot_close, then this system's gradient, behind that
+    double* slot_host = nullptr;    // pinned copy (from the first training system on)
 };
 
 namespace {
 using hpb::spai::kNumParams;
 constexpr int kGridMlp = 296;
+constexpr size_t kPartBytes = size_t(kGridMlp) * kNumParams * 4;
+constexpr size_t kSlotOutBytes = 4 * sizeof(double) + size_t(kNumParams) * sizeof(float);
 
 int grow(hpb_spai* net, int32_t rows, int64_t nnz) {
     using namespace hpb::spai;
@@ -728,6 +1029,77 @@ int grow(hpb_spai* net, int32_t rows, int64_t nnz) {
     return HPB_SUCCESS;
 }
 
+
+// The slot-form workspace of one system: offsets of its arrays in one block.
+struct SlotArrays {
+    float *raw, *ah, *th, *mh, *y, *z, *rh, *G, *dm, *diag, *feat, *h1, *h2;
+    uint8_t* mask;
+    double *sd, *ld, *sums, *lpart;
+    hpb::fused::Acc2* partials;
+    size_t bytes;
+};
+SlotArrays slot_arrays(char* base, size_t n, const hpb::spai::Offsets& o, bool train) {
+    using namespace hpb::spai;
+    SlotArrays a{};
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        char* p = base + at;
+        at += (bytes + 255) & ~size_t(255);
+        return p;
+    };
+    auto floats = [&](size_t k) { return reinterpret_cast<float*>(take(k * n * sizeof(float))); };
+    const size_t nb = (n + kSlotThreads - 1) / kSlotThreads;
+    a.raw = floats(size_t(o.nslot));
+    a.th = floats(kO);
+    a.mask = reinterpret_cast<uint8_t*>(take(n));
+    a.sums = reinterpret_cast<double*>(take((1 + kMaxRes) * sizeof(double)));
+    a.partials = reinterpret_cast<hpb::fused::Acc2*>(take((1 + kMaxRes) * nb * sizeof(hpb::fused::Acc2)));
+    if (!train) {
+        a.sd = reinterpret_cast<double*>(take(n * sizeof(double)));
+        a.ld = reinterpret_cast<double*>(take(n * sizeof(double)));
+    } else {
+        a.diag = floats(1);
+        a.ah = floats(size_t(o.nslot));
+        a.mh = floats(size_t(o.nslot));
+        a.dm = floats(size_t(o.nslot));
+        a.y = floats(kMaxRes);
+        a.z = floats(kMaxRes);
+        a.rh = floats(kMaxRes);
+        a.G = floats(size_t(o.nsq));
+        a.feat = floats(kF);
+        a.h1 = floats(kH);
+        a.h2 = floats(kH);
+        a.lpart = reinterpret_cast<double*>(take(size_t(o.nsq + kMaxRes) * nb * sizeof(double)));
+    }
+    a.bytes = at;
+    return a;
+}
+
+// k_slot_load for nres samples (-1: the build)
+void launch_slot_load(hpb_spai* net, const hpb_spai_system& sys, int nres, const SlotArrays& a) {
+    using namespace hpb::spai;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int nb = std::min((sys.rows + kSlotThreads - 1) / kSlotThreads, sms * 12);
+    auto go = [&](auto k) {
+        constexpr int NR = decltype(k)::value;
+        k_slot_load<NR><<<nb, kSlotThreads>>>(sys.rows, sys.row_ptr, sys.col_ind, sys.val, net->off, sys.residuals, a.raw,
+                                              a.mask, a.diag, a.sd, a.ld, a.rh, a.sums, a.partials, net->slot_sync,
+                                              reinterpret_cast<int*>(net->slot_sync + 32),
+                                              reinterpret_cast<int*>(net->slot_sync + 64));
+    };
+    switch (nres) {
+        case 1: go(std::integral_constant<int, 1>{}); break;
+        case 2: go(std::integral_constant<int, 2>{}); break;
+        case 3: go(std::integral_constant<int, 3>{}); break;
+        case 4: go(std::integral_constant<int, 4>{}); break;
+        case 0: go(std::integral_constant<int, 0>{}); break;
+        default: go(std::integral_constant<int, -1>{}); break;
+    }
+    hpb::count_launch();
+}
+static_assert(hpb::spai::kMaxRes == 4, "launch_slot_load's cases");
 
 // diag of a binary32 CSR
 // diag(A) (binary32) and log|a_ii| (binary64, for the mean over the rows)
@@ -870,6 +1242,12 @@ int hpb_spai_create(hpb_spai** out, int nslot, int dslot, const int* offsets, ui
                 if (o.sqoff[u] == d) t = u;
             o.dq[p][q] = t;
         }
+    for (int t = 0; t < kMaxSq; ++t)
+        for (int p = 0; p < kMaxSlot; ++p) {
+            net->pairs.q[t][p] = -1;
+            for (int q = 0; t < o.nsq && p < nslot && q < nslot; ++q)
+                if (o.sq[p][q] == t) net->pairs.q[t][p] = static_cast<signed char>(q);
+        }
     for (int p = 0; p < nslot; ++p) {
         o.rev[p] = -1;
         for (int q = 0; q < nslot; ++q)
@@ -892,7 +1270,7 @@ int hpb_spai_create(hpb_spai** out, int nslot, int dslot, const int* offsets, ui
         w[Params::B1 + i] = 0.01f;
         w[Params::B2 + i] = 0.01f;
     }
-    if (cudaHostAlloc(&net->tc_err, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+    if (cudaHostAlloc(&net->tc_err, 2 * sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
         net->tc_err = nullptr;
         hpb_spai_destroy(net);
         return HPB_ERROR_OUT_OF_MEMORY;
@@ -905,13 +1283,17 @@ int hpb_spai_create(hpb_spai** out, int nslot, int dslot, const int* offsets, ui
     if (cudaMalloc(&net->w, kNumParams * 4) || cudaMalloc(&net->wb, kNumParams * 2) ||
         cudaMalloc(&net->m1, kNumParams * 4) || cudaMalloc(&net->m2, kNumParams * 4) ||
         cudaMalloc(&net->grad, kNumParams * 4) || cudaMalloc(&net->gtmp, kNumParams * 4) ||
-        cudaMalloc(&net->part, size_t(kGridMlp) * kNumParams * 4) || cudaMalloc(&net->wimg, kTcImageBytes)) {
+        cudaMalloc(&net->part, kPartBytes + 96 * sizeof(unsigned) + kSlotOutBytes) ||
+        cudaMalloc(&net->wimg, kTcImageBytes)) {
         hpb_spai_destroy(net);
         return HPB_ERROR_OUT_OF_MEMORY;
     }
+    net->slot_sync = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(net->part) + kPartBytes);
+    net->slot_out = reinterpret_cast<double*>(net->slot_sync + 96);
     cudaMemset(net->m1, 0, kNumParams * 4);
     cudaMemset(net->m2, 0, kNumParams * 4);
     cudaMemset(net->grad, 0, kNumParams * 4);
+    cudaMemset(net->slot_sync, 0, 96 * sizeof(unsigned));
     int st = hpb_spai_set_weights(net, w.data());
     if (st) {
         hpb_spai_destroy(net);
@@ -921,7 +1303,8 @@ int hpb_spai_create(hpb_spai** out, int nslot, int dslot, const int* offsets, ui
         hpb_spai_destroy(net);
         return HPB_ERROR_CUDA;
     }
-    cudaFuncSetAttribute(k_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bwd_tc_smem()));
+    cudaFuncSetAttribute(k_backward<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bwd_tc_smem()));
+    cudaFuncSetAttribute(k_backward<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bwd_tc_smem()));
     *out = net;
     return HPB_SUCCESS;
 }
@@ -931,8 +1314,9 @@ int hpb_spai_destroy(hpb_spai* net) {
     cudaDeviceSynchronize();
     void* ptrs[] = {net->w, net->wb, net->m1, net->m2, net->grad, net->gtmp, net->part, net->feat, net->h1, net->h2,
                     net->out, net->dout, net->diag, net->mval, net->dm, net->G, net->y, net->z, net->g, net->lpart,
-                    net->ahat, net->rh, net->wimg};
+                    net->ahat, net->rh, net->wimg, net->slot_mem};
     for (void* p : ptrs) cudaFree(p);
+    if (net->slot_host) cudaFreeHost(net->slot_host);
     if (net->tc_err) cudaFreeHost(net->tc_err);
     if (net->ctx) hpb_destroy(net->ctx);
     delete net;
@@ -968,6 +1352,26 @@ int hpb_spai_assemble(hpb_spai* net, const hpb_spai_system* sys, float* m_val) {
     // the solvers' pool on the legacy stream (no training workspace)
     using hpb::fused::pool_alloc;
     using hpb::fused::pool_free;
+    {
+        const size_t bytes = slot_arrays(nullptr, size_t(n), net->off, false).bytes;
+        char* mem = static_cast<char*>(pool_alloc(bytes, nullptr));
+        if (!mem) return HPB_ERROR_OUT_OF_MEMORY;
+        const SlotArrays a = slot_arrays(mem, size_t(n), net->off, false);
+        launch_slot_load(net, *sys, -1, a);
+        const int* irregular = reinterpret_cast<int*>(net->slot_sync + 64);
+        const cudaError_t fe = forward_slots_tc(SlotSystem{n, a.raw, a.mask, a.diag, a.sd, a.ld, a.sums}, net->off, net->wimg, nullptr,
+                                                nullptr, nullptr, nullptr, a.th, net->tc_err_dev, nullptr);
+        k_slot_assemble<<<(n + kSlotThreads - 1) / kSlotThreads, kSlotThreads>>>(
+            n, sys->row_ptr, a.mask, a.sd, a.th, net->off, irregular, m_val);
+        hpb::count_launch(2);
+        cudaMemcpyAsync(net->tc_err + 1, irregular, sizeof(int), cudaMemcpyDeviceToHost, nullptr);
+        pool_free(mem, nullptr);
+        if (fe != cudaSuccess || cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess)
+            return HPB_ERROR_CUDA;
+        const int tc = take_tc_status(net);
+        if (tc != HPB_SUCCESS) return tc;
+        if (net->tc_err[1] == 0) return HPB_SUCCESS;
+    }
     const size_t R = size_t(n);
     float* diag = static_cast<float*>(pool_alloc(R * 4, nullptr));
     float* feat = static_cast<float*>(pool_alloc(R * kF * 4, nullptr));
@@ -1005,10 +1409,75 @@ int hpb_spai_forward(hpb_spai* net, int32_t rows, const float* feat, float* out,
 }  // extern "C"
 
 namespace {
+// The slot form of loss_impl: eight launches, one copy and one wait for the
+// host (the CSR kernels below: 35 launches, a copy and a wait for every sum).
+// *irregular: nothing was added, the system needs those.
+// Measured on B200 (24^3, three samples): 85 us against 388 us.
+int loss_slots(hpb_spai* net, const hpb_spai_system& sys, float w_frob, float w_resid, double* loss, float* grad_host,
+               bool grad, bool* irregular) {
+    using namespace hpb::spai;
+    const int32_t n = sys.rows;
+    if (net->slot_host == nullptr && cudaMallocHost(&net->slot_host, kSlotOutBytes) != cudaSuccess) {
+        cudaGetLastError();
+        net->slot_host = nullptr;
+        return HPB_ERROR_OUT_OF_MEMORY;
+    }
+    if (size_t(n) > net->slot_rows) {
+        cudaFree(net->slot_mem);
+        net->slot_mem = nullptr;
+        net->slot_rows = 0;
+        if (cudaMalloc(&net->slot_mem, slot_arrays(nullptr, size_t(n), net->off, true).bytes) != cudaSuccess) {
+            cudaGetLastError();
+            net->slot_mem = nullptr;
+            return HPB_ERROR_OUT_OF_MEMORY;
+        }
+        net->slot_rows = size_t(n);
+    }
+    const SlotArrays a = slot_arrays(net->slot_mem, size_t(n), net->off, true);
+    launch_slot_load(net, sys, sys.nres, a);
+    const int* irr = reinterpret_cast<int*>(net->slot_sync + 64);
+    if (forward_slots_tc(SlotSystem{n, a.raw, a.mask, a.diag, a.sd, a.ld, a.sums}, net->off, net->wimg, a.ah, grad ? a.feat : nullptr,
+                         grad ? a.h1 : nullptr, grad ? a.h2 : nullptr, a.th, net->tc_err_dev, nullptr) != cudaSuccess)
+        return HPB_ERROR_CUDA;
+    const SlotMats w{n, a.mask, a.ah, a.th, a.mh, a.y, a.z, a.rh, a.G, a.dm, a.lpart, a.sums, sys.nres};
+    const int nb = (n + kSlotThreads - 1) / kSlotThreads, planes = net->off.nsq + sys.nres;
+    k_slot_mh<<<nb, kSlotThreads>>>(w, net->off);
+    k_slot_gz<<<dim3(unsigned(nb), unsigned(planes)), kSlotThreads>>>(w, net->off, net->pairs);
+    int grid = 0;
+    if (grad) {
+        k_slot_dm<<<dim3(unsigned(nb), unsigned(net->off.nslot)), kSlotThreads>>>(w, net->off, w_frob / float(n), w_resid);
+        const int nchunks = (n + kBwdRows - 1) / kBwdRows;
+        int dev = 0, sms = 148;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        grid = std::max(1, std::min(std::min(kGridMlp, sms), nchunks));
+        k_backward<true><<<grid, kMmaWarps * 32, bwd_tc_smem()>>>(n, a.feat, net->wb, a.h1, a.h2, nullptr, w, net->off,
+                                                                  net->part);
+    }
+    float* gsys = reinterpret_cast<float*>(net->slot_out + 4);
+    const int gblocks = grad ? (kNumParams + kSlotThreads - 1) / kSlotThreads : 0;
+    k_slot_close<<<gblocks + 1, kSlotThreads>>>(grid, net->part, gsys, net->grad, w, net->off.nsq, nb, w_frob, w_resid, irr,
+                                                net->slot_out);
+    hpb::count_launch(grad ? 6 : 4);
+    cudaMemcpyAsync(net->slot_host, net->slot_out, grad && grad_host ? kSlotOutBytes : 4 * sizeof(double),
+                    cudaMemcpyDeviceToHost, nullptr);
+    if (cudaStreamSynchronize(nullptr) != cudaSuccess || cudaGetLastError() != cudaSuccess) return HPB_ERROR_CUDA;
+    *irregular = net->slot_host[3] != 0.0;
+    if (*irregular) return HPB_SUCCESS;
+    if (loss) std::memcpy(loss, net->slot_host, 3 * sizeof(double));
+    if (grad && grad_host) std::memcpy(grad_host, net->slot_host + 4, size_t(kNumParams) * sizeof(float));
+    return take_tc_status(net);
+}
+
 int loss_impl(hpb_spai* net, const hpb_spai_system* sys, float w_frob, float w_resid, double* loss, float* grad_host,
               bool grad) {
     using namespace hpb::spai;
     if (!net || !sys || sys->rows <= 0) return HPB_ERROR_INVALID_VALUE;
+    if (sys->nres >= 0 && sys->nres <= kMaxRes) {
+        bool irregular = false;
+        const int sst = loss_slots(net, *sys, w_frob, w_resid, loss, grad_host, grad, &irregular);
+        if (sst != HPB_SUCCESS || !irregular) return sst;
+    }
     int st = forward_system(net, *sys);
     if (st) return st;
     const int32_t n = sys->rows;
@@ -1056,8 +1525,8 @@ int loss_impl(hpb_spai* net, const hpb_spai_system* sys, float w_frob, float w_r
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const int grid = std::max(1, std::min(std::min(kGridMlp, sms), nchunks));
-        k_backward<<<grid, kMmaWarps * 32, bwd_tc_smem()>>>(n, net->feat, net->wb, net->h1, net->h2, net->dout,
-                                                            net->part);
+        k_backward<false><<<grid, kMmaWarps * 32, bwd_tc_smem()>>>(n, net->feat, net->wb, net->h1, net->h2, net->dout,
+                                                                   SlotMats{}, net->off, net->part);
         k_reduce_grad<<<(kNumParams + 255) / 256, 256>>>(grid, net->part, net->gtmp, net->grad);
         hpb::count_launch(3);
         if (grad_host && cudaMemcpy(grad_host, net->gtmp, kNumParams * 4, cudaMemcpyDeviceToHost) != cudaSuccess)

@@ -18,6 +18,37 @@ struct Params {  // offsets (in elements) of each tensor in the parameter vector
     static constexpr int W1 = 0, B1 = W1 + kF * kH, W2 = B1 + kH, B2 = W2 + kH * kH, W3 = B2 + kH, B3 = W3 + kH * kO;
 };
 
+constexpr int kMaxSlot = 8, kMaxSq = 64;
+
+// Stencil slots: the column offsets col - row a row's entries may have, and
+// the offsets of A^2's pattern.
+struct Offsets {
+    int nslot, dslot;
+    int off[kMaxSlot];
+    // A^2 pattern: nsq distinct offsets; sq[p][q] = index of off[p] + off[q]
+    int nsq;
+    int sqoff[kMaxSq];
+    int sq[kMaxSlot][kMaxSlot];
+    // index of off[q] - off[p] in sqoff (-1 if absent)
+    int dq[kMaxSlot][kMaxSlot];
+    // slot of -off[s] (the transposed entry), -1 if absent
+    int rev[kMaxSlot];
+};
+
+// A system in slot form: entry (i, i + off[s]) at raw[s * n + i] (0 where
+// row i stores none), bit s of mask[i] set where it does.
+struct SlotSystem {
+    int32_t n;
+    const float* raw;
+    const uint8_t* mask;
+    const float* diag;   // a_ii
+    const double* sd;    // 1 / sqrt|a_ii| and log|a_ii|: the build's features come from these,
+    const double* ld;    //   training's (null here) from diag
+    const double* lsum;  // sum of log|a_ii|
+};
+
+__device__ __forceinline__ float inv_sqrt_dd(float di, float dj) { return 1.f / sqrtf(fabsf(di * dj)); }
+
 // Bytes of the tcgen05 forward's weight image (operands in the kernel's
 // shared-memory layout, then the biases).
 constexpr int kTcImageBytes = 2 * (kH * kF + kH * kH + 16 * kH) + (2 * kH + kO) * 4;  // 12832
@@ -35,6 +66,13 @@ cudaError_t weight_image_tc(const __nv_bfloat16* w, void* img, cudaStream_t stre
 // Returns the launch status.
 cudaError_t forward_tc(int32_t rows, const float* feat, const void* img, float* h1, float* h2, float* out, int* err,
                        cudaStream_t stream);
+
+// The forward of a slot-form system with its features formed in the kernel
+// (the features of hpb_spai.cu's comment) and its outputs as
+// th[s * n + i] = tanh(out_{i,s}).  Training (sys.sd null): ah (scaled values
+// Ah, slot form), and feat (row-major, kF per row), h1 and h2 when not null.
+cudaError_t forward_slots_tc(const SlotSystem& sys, const Offsets& o, const void* img, float* ah, float* feat, float* h1,
+                             float* h2, float* th, int* err, cudaStream_t stream);
 
 }  // namespace spai
 }  // namespace hpb

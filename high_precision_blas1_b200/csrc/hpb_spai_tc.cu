@@ -25,6 +25,7 @@
 // the two 8-element K halves of one K = 16 product (LBO) is 16 R bytes.
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "hpb_spai.cuh"
 
@@ -187,6 +188,92 @@ __device__ __forceinline__ void load_feat(const float* __restrict__ feat, int32_
     }
 }
 
+// ---- the features of a slot-form row ------------------------------------
+// NS, DS: the slot count and the diagonal's slot where they are known at
+// compile time (everything stays in registers then), NS = 0 otherwise.
+// TABLES (the build): the neighbours' 1 / sqrt|a_jj| and log|a_jj| come from
+// the binary64 tables of k_slot_load, one multiplication or subtraction and
+// one rounding a feature.  Training keeps the binary32 arithmetic of the CSR
+// path's k_features, operation by operation.
+template <bool TABLES>
+struct SlotRow {
+    float a[kMaxSlot];
+    typename std::conditional<TABLES, double, float>::type sj[kMaxSlot], lj[TABLES ? kMaxSlot : 1];
+    unsigned m;
+};
+struct SlotArgs {
+    SlotSystem sys;
+    int nslot, dslot;
+    int off[kMaxSlot];
+    float *ah, *feat;
+};
+template <bool TABLES, int NS, int DS>
+__device__ __forceinline__ void load_slots(const SlotArgs& g, int32_t row, SlotRow<TABLES>& r) {
+    const int ns = NS ? NS : g.nslot;
+    r.m = 0u;
+    if (row >= g.sys.n) return;
+    r.m = __ldg(g.sys.mask + row);
+#pragma unroll
+    for (int s = 0; s < (NS ? NS : kMaxSlot); ++s)
+        if (s < ns) {
+            r.a[s] = __ldg(g.sys.raw + size_t(s) * g.sys.n + row);
+            if (s == (NS ? DS : g.dslot) || ((r.m >> s) & 1u)) {
+                if constexpr (TABLES) {
+                    r.sj[s] = __ldg(g.sys.sd + (row + g.off[s]));
+                    r.lj[s] = __ldg(g.sys.ld + (row + g.off[s]));
+                } else {
+                    r.sj[s] = __ldg(g.sys.diag + (row + g.off[s]));
+                }
+            }
+        }
+}
+template <bool TABLES, int NS, int DS>
+__device__ __forceinline__ void slot_features(const SlotArgs& g, int32_t row, const SlotRow<TABLES>& r, double mean,
+                                              float (&x)[kF]) {
+    const int ns = NS ? NS : g.nslot, ds = NS ? DS : g.dslot;
+#pragma unroll
+    for (int k = 0; k < kF; ++k) x[k] = 0.f;
+    if (row >= g.sys.n) return;
+    auto si = r.sj[0];
+    auto li = r.lj[0];
+#pragma unroll
+    for (int s = 0; s < (NS ? NS : kMaxSlot); ++s)
+        if (s == ds) {
+            si = r.sj[s];
+            if constexpr (TABLES) li = r.lj[s];
+        }
+#pragma unroll
+    for (int s = 0; s < (NS ? NS : kMaxSlot); ++s) {
+        if (s >= ns) continue;
+        const bool has = (r.m >> s) & 1u;
+        float v = 0.f, l = 0.f;
+        if constexpr (TABLES) {
+            if (has && s != ds) {
+                v = r.a[s] * float(si * r.sj[s]);
+                l = float(r.lj[s] - li);
+            }
+        } else {
+            if (has) v = r.a[s] * inv_sqrt_dd(si, r.sj[s]);
+            if (has && s != ds) l = logf(fabsf(r.sj[s] / si));
+            g.ah[size_t(s) * g.sys.n + row] = v;
+        }
+        if (s == ds) continue;
+        const int f = s - (s > ds ? 1 : 0);
+        x[f] = v;
+        x[f + ns - 1] = l;
+    }
+    if constexpr (TABLES)
+        x[2 * (ns - 1)] = float(li - mean);
+    else
+        x[2 * (ns - 1)] = logf(fabsf(si)) - float(mean);
+    x[2 * (ns - 1) + 1] = 1.f;
+    if (!TABLES && g.feat) {
+        float4* dst = reinterpret_cast<float4*>(g.feat + size_t(row) * kF);
+#pragma unroll
+        for (int k = 0; k < kF / 4; ++k) dst[k] = make_float4(x[4 * k], x[4 * k + 1], x[4 * k + 2], x[4 * k + 3]);
+    }
+}
+
 // The weights as the kernel's shared-memory image: the K-major B operands
 // (W^T: rows n, K contiguous; W3^T padded to 16 rows with zeros) in bytes
 // [0, kOffA1h) and the biases (binary32) after them; built once per weight
@@ -216,9 +303,18 @@ __global__ void k_weight_image(const __nv_bfloat16* __restrict__ w, unsigned cha
     }
 }
 
+// IN_SLOTS, IN_TABLES: the features are formed here from a slot-form system, and the
+// outputs leave as tanh in slot form; otherwise feat and out are row-major.
+// Forming them here, from logarithms and reciprocal roots of the diagonal that
+// k_slot_load took once a row in binary64, saves the pass that wrote 64 bytes
+// a row and the read of them: at 884,736 rows 59 + 61 us for the two kernels,
+// 68 us for this one (B200, seven tanh a row included).
+enum Input { IN_FEATURES, IN_SLOTS, IN_TABLES };
+template <int IN, int NS, int DS>
 __global__ void __launch_bounds__(kTcThreads, 4)
-k_forward_tc(int32_t rows, const float* __restrict__ feat, const unsigned char* __restrict__ img,
+k_forward_tc(int32_t rows, const float* __restrict__ feat, SlotArgs g, const unsigned char* __restrict__ img,
              float* __restrict__ h1g, float* __restrict__ h2g, float* __restrict__ out, int* err) {
+    constexpr bool SLOTS = IN != IN_FEATURES, TABLES = IN == IN_TABLES;
     extern __shared__ __align__(1024) unsigned char sm[];
     const int t = threadIdx.x, warp = t >> 5;
     const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(sm));
@@ -268,10 +364,18 @@ k_forward_tc(int32_t rows, const float* __restrict__ feat, const unsigned char* 
     bool failed = false;
     const int32_t ntiles = (rows + kTile - 1) / kTile;
     float xf[kF];
-    if (int32_t(blockIdx.x) < ntiles) load_feat(feat, int32_t(blockIdx.x) * kTile + t, rows, xf);
+    SlotRow<TABLES> sr;
+    double mean = 0.0;
+    if constexpr (SLOTS) {
+        mean = __ldg(g.sys.lsum) / double(rows > 1 ? rows : 1);
+        load_slots<TABLES, NS, DS>(g, int32_t(blockIdx.x) * kTile + t, sr);
+    } else {
+        if (int32_t(blockIdx.x) < ntiles) load_feat(feat, int32_t(blockIdx.x) * kTile + t, rows, xf);
+    }
     for (int32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int32_t row = tile * kTile + t;
         // ---- layer 1
+        if constexpr (SLOTS) slot_features<TABLES, NS, DS>(g, row, sr, mean, xf);
 #pragma unroll
         for (int kc = 0; kc < kF / 8; ++kc) {
             uint4 hi, lo;
@@ -280,7 +384,12 @@ k_forward_tc(int32_t rows, const float* __restrict__ feat, const unsigned char* 
             *reinterpret_cast<uint4*>(sm + kOffA1l + kmaj(t, kc, kTile)) = lo;
         }
         const int32_t next = tile + gridDim.x;
-        if (next < ntiles) load_feat(feat, next * kTile + t, rows, xf);  // in flight during this tile
+        if (next < ntiles) {  // in flight during this tile
+            if constexpr (SLOTS)
+                load_slots<TABLES, NS, DS>(g, next * kTile + t, sr);
+            else
+                load_feat(feat, next * kTile + t, rows, xf);
+        }
         fence_async_smem();
         fence_before_sync();
         __syncthreads();
@@ -368,10 +477,16 @@ k_forward_tc(int32_t rows, const float* __restrict__ feat, const unsigned char* 
         float o[kN3];
         tmem_ld16(lane_tmem + 0, o);
         if (row < rows) {
-            float4* p = reinterpret_cast<float4*>(out + size_t(row) * kO);
             const float* b3 = sbias + 2 * kH;
-            p[0] = make_float4(o[0] + b3[0], o[1] + b3[1], o[2] + b3[2], o[3] + b3[3]);
-            p[1] = make_float4(o[4] + b3[4], o[5] + b3[5], o[6] + b3[6], o[7] + b3[7]);
+            if constexpr (SLOTS) {
+#pragma unroll
+                for (int q = 0; q < kO; ++q)
+                    if (q < (NS ? NS : g.nslot)) out[size_t(q) * rows + row] = tanhf(o[q] + b3[q]);
+            } else {
+                float4* p = reinterpret_cast<float4*>(out + size_t(row) * kO);
+                p[0] = make_float4(o[0] + b3[0], o[1] + b3[1], o[2] + b3[2], o[3] + b3[3]);
+                p[1] = make_float4(o[4] + b3[4], o[5] + b3[5], o[6] + b3[6], o[7] + b3[7]);
+            }
         }
         fence_before_sync();  // the next tile's products overwrite columns read here
     }
@@ -391,17 +506,20 @@ cudaError_t weight_image_tc(const __nv_bfloat16* w, void* img, cudaStream_t stre
     return cudaGetLastError();
 }
 
-cudaError_t forward_tc(int32_t rows, const float* feat, const void* img, float* h1, float* h2, float* out, int* err,
-                       cudaStream_t stream) {
+namespace {
+template <int IN, int NS, int DS>
+cudaError_t launch_forward(int32_t rows, const float* feat, const SlotArgs& g, const void* img, float* h1, float* h2,
+                           float* out, int* err, cudaStream_t stream) {
     if (rows <= 0) return cudaSuccess;
+    auto kernel = k_forward_tc<IN, NS, DS>;
     int dev = 0, sms = 148, occ = 1;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_forward_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     // the whole unified L1 as shared memory: four blocks per SM (with the
     // default split the occupancy query, and the launch, gave one)
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_forward_tc, cudaFuncAttributePreferredSharedMemoryCarveout,
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  int(cudaSharedmemCarveoutMaxShared));
     if (e != cudaSuccess) return e;
     // four blocks per SM: shared memory bounds residency to four, whose 4 x
@@ -411,9 +529,34 @@ cudaError_t forward_tc(int32_t rows, const float* feat, const void* img, float* 
     occ = 512 / kTmemCols;
     const int32_t ntiles = (rows + kTile - 1) / kTile;
     const int grid = int(std::max<int64_t>(1, std::min<int64_t>(ntiles, int64_t(sms) * occ)));
-    k_forward_tc<<<grid, kTcThreads, kSmemBytes, stream>>>(rows, feat, static_cast<const unsigned char*>(img), h1, h2,
-                                                           out, err);
+    kernel<<<grid, kTcThreads, kSmemBytes, stream>>>(rows, feat, g, static_cast<const unsigned char*>(img), h1, h2, out,
+                                                     err);
     return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t forward_tc(int32_t rows, const float* feat, const void* img, float* h1, float* h2, float* out, int* err,
+                       cudaStream_t stream) {
+    return launch_forward<IN_FEATURES, 0, 0>(rows, feat, SlotArgs{}, img, h1, h2, out, err, stream);
+}
+
+cudaError_t forward_slots_tc(const SlotSystem& sys, const Offsets& o, const void* img, float* ah, float* feat, float* h1,
+                             float* h2, float* th, int* err, cudaStream_t stream) {
+    SlotArgs g{};
+    g.sys = sys;
+    g.nslot = o.nslot;
+    g.dslot = o.dslot;
+    for (int s = 0; s < kMaxSlot; ++s) g.off[s] = o.off[s];
+    g.ah = ah;
+    g.feat = feat;
+    const int shape = o.nslot == 7 && o.dslot == 3 ? 7 : o.nslot == 5 && o.dslot == 2 ? 5 : 0;  // 3-D, 2-D stencil
+    auto go = [&](auto in) {
+        constexpr int IN = decltype(in)::value;
+        if (shape == 7) return launch_forward<IN, 7, 3>(sys.n, nullptr, g, img, h1, h2, th, err, stream);
+        if (shape == 5) return launch_forward<IN, 5, 2>(sys.n, nullptr, g, img, h1, h2, th, err, stream);
+        return launch_forward<IN, 0, 0>(sys.n, nullptr, g, img, h1, h2, th, err, stream);
+    };
+    return sys.sd != nullptr ? go(std::integral_constant<int, IN_TABLES>{}) : go(std::integral_constant<int, IN_SLOTS>{});
 }
 
 }  // namespace spai
