@@ -81,6 +81,55 @@ __device__ __forceinline__ bool finite_e(double v) { return isfinite(v); }
 __device__ __forceinline__ bool finite_e(cf v) { return isfinite(v.re + v.im); }
 __device__ __forceinline__ bool finite_e(cd v) { return isfinite(v.re + v.im); }
 
+// to_s(from_s<E>(v)), v rounded to the storage precision and kept in S,
+// without the two conversions: binary32 <-> binary64 conversions run at 16 a
+// clock and SM on B200, a quarter of the rate of binary64 arithmetic (15.6
+// against 60 measured), and a complex<binary32> product that forms its operand
+// on the way spent more time on them than on memory.  Adding and taking away
+// 1.5 * 2^(e + 29), e the exponent of v (at least -126, binary32's smallest),
+// rounds v to nearest even at binary32's last place.  (A v beyond binary32's
+// range stays finite here; the stored vector it belongs to is infinite.)
+__device__ __forceinline__ double round_f32(double v) {
+    const int e = max(__double2hiint(v) & 0x7ff00000, 0x38100000);
+    const double m = __hiloint2double(e + (29 << 20) + 0x80000, 0);
+    return sub_rn(add_rn(v, m), m);
+}
+template <class E> __device__ __forceinline__ double round_s(double v) {
+    return std::is_same<E, float>::value ? round_f32(v) : v;
+}
+template <class E> __device__ __forceinline__ cd round_s(cd v) {
+    return std::is_same<E, cf>::value ? cd{round_f32(v.re), round_f32(v.im)} : v;
+}
+
+// ------------------------------------------------------------ 16-byte packs
+// VW consecutive elements q*VW .. q*VW + VW - 1 of a vector moved as one
+// 16-byte access (VEC: VW * sizeof(E) == 16 and the vector 16-byte
+// aligned), or one element through ldE / stE (VW == 1).
+template <class E> struct pack_of { static constexpr int value = 16 / int(sizeof(E)); };
+
+template <class E, int VW, bool VEC, bool RO>
+__device__ __forceinline__ void ld_pack(const E* p, int64_t q, E (&o)[VW]) {
+    if constexpr (VEC) {
+        static_assert(VW * sizeof(E) == 16, "one 16-byte pack");
+        const uint4* a = reinterpret_cast<const uint4*>(p) + q;
+        const uint4 t = RO ? __ldg(a) : *a;
+        memcpy(&o[0], &t, 16);
+    } else {
+        static_assert(VW == 1, "one element");
+        o[0] = RO ? ldgE(p, q) : ldE(p, q);
+    }
+}
+template <class E, int VW, bool VEC>
+__device__ __forceinline__ void st_pack(E* p, int64_t q, const E (&v)[VW]) {
+    if constexpr (VEC) {
+        uint4 t;
+        memcpy(&t, &v[0], 16);
+        reinterpret_cast<uint4*>(p)[q] = t;
+    } else {
+        stE(p, q, v[0]);
+    }
+}
+
 // ------------------------------------------------------------ Dot2 pieces
 // (s, c) accumulator of conj(a)*b in binary64 (real) / complex binary64.
 struct Acc2 {

@@ -34,144 +34,11 @@
 #include <new>
 #include <vector>
 
+#include "hpb_bcg.cuh"
 #include "hpb_fused.cuh"
 
 namespace hpb {
 namespace fused {
-
-constexpr int kMaxL = 8;
-constexpr int kThreads = 256;
-
-template <class S>
-struct BcgState {
-    S rho, alpha, omega, beta;
-    S alpha_prev;  // alpha of the previous inner step (its deferred r update)
-    S tau[kMaxL + 1][kMaxL + 1];
-    S sigma[kMaxL + 1], gam[kMaxL + 1], gam1[kMaxL + 1], gam2[kMaxL + 1];
-    S last[2];
-};
-
-struct Report {
-    double rnorm;   // ||r_0|| (compensated)
-    int breakdown;  // rho == 0 met
-    int nonfinite;  // x held a non-finite entry
-};
-
-// The monitor of the device-side cycle loop (default_monitor semantics, one
-// test per cycle): the host sets tol / max_iters / iters once per solve and
-// chunk_left / hl before each launch of the loop graph.
-constexpr int kLoopChunk = 128;  // cycles one launch of the loop graph runs at most
-struct MonState {
-    double tol;
-    double rn;
-    int max_iters;
-    int iters;
-    int chunk_left;
-    int hl;          // history entries written in this launch
-    int finished, conv, valid, breakdown;
-};
-
-template <class E>
-struct Vecs {
-    E* r[kMaxL + 1];
-    E* u[kMaxL + 1];
-};
-
-enum Epi { EPI_NONE = 0, EPI_ALPHA, EPI_BETA, EPI_STEP, EPI_FINAL };
-
-template <class S>
-struct EpiArgs {
-    BcgState<S>* st;
-    Report* rep;
-    int kind, k, j, L;
-    // EPI_FINAL inside the loop graph: the monitor's test and the loop's
-    // condition (monitor_step) after the cycle's report is complete
-    MonState* mon = nullptr;
-    double* hist = nullptr;
-    cudaGraphConditionalHandle cond = 0;
-};
-
-// End of a cycle inside the loop graph: the host loop's test, then the
-// loop's condition.  Every path reaches the one cudaGraphSetConditional
-// call, and the loop stops after chunk_left cycles whatever the test says,
-// so one launch of the graph always ends.
-__device__ inline void monitor_step(MonState* M, const Report* rep, double* hist, int L, cudaGraphConditionalHandle h) {
-    const int it = M->iters + L;
-    M->iters = it;
-    int fin;
-    if (rep->breakdown) {
-        M->breakdown = 1;
-        fin = 1;
-    } else {
-        const double rn = rep->rnorm;
-        const int valid = !rep->nonfinite && isfinite(rn);
-        const int conv = valid && rn <= M->tol;
-        M->rn = rn;
-        M->valid = valid;
-        M->conv = conv;
-        const int k = M->hl;
-        if (k < kLoopChunk) {
-            hist[2 * k] = double(it);
-            hist[2 * k + 1] = rn;
-            M->hl = k + 1;
-        }
-        fin = !valid || conv || it >= M->max_iters;
-    }
-    M->finished = fin;
-    const int left = M->chunk_left - 1;
-    M->chunk_left = left;
-    cudaGraphSetConditional(h, (fin || left <= 0) ? 0u : 1u);
-}
-
-template <class S>
-__device__ void run_epi(const EpiArgs<S>& a, const S* v, bool bad) {
-    BcgState<S>& st = *a.st;
-    switch (a.kind) {
-        case EPI_ALPHA:  // alpha = rho / <rt, u_{j+1}>
-            st.alpha_prev = st.alpha;
-            st.alpha = s_div(st.rho, v[0]);
-            break;
-        case EPI_BETA:  // rho1 = <rt, r_j>; beta = alpha rho1 / rho; rho = rho1
-            if (s_is_zero(st.rho)) a.rep->breakdown = 1;
-            st.beta = s_div(s_mul(st.alpha, v[0]), st.rho);
-            st.rho = v[0];
-            break;
-        case EPI_STEP: {  // sweep k: v = (<r_k, r_k>, <r_k, r_0>, <r_k, r_{k+1}>, ..., <r_k, r_L>)
-            const int k = a.k, L = a.L;
-            st.sigma[k] = v[0];
-            st.gam1[k] = s_div(v[1], v[0]);
-            for (int j = k + 1; j <= L; ++j) st.tau[k][j] = s_div(v[1 + j - k], v[0]);
-            if (k == L) {  // gamma = T^{-1} gamma', gamma'' (the MR part of bicgstabl.h)
-                st.gam[L] = st.gam1[L];
-                st.omega = st.gam[L];
-                for (int jj = L - 1; jj >= 1; --jj) {
-                    S g = st.gam1[jj];
-                    for (int i = jj + 1; i <= L; ++i) g = s_sub(g, s_mul(st.tau[jj][i], st.gam[i]));
-                    st.gam[jj] = g;
-                }
-                for (int jj = 1; jj < L; ++jj) {
-                    S g = st.gam[jj + 1];
-                    for (int i = jj + 1; i < L; ++i) g = s_add(g, s_mul(st.tau[jj][i], st.gam[i + 1]));
-                    st.gam2[jj] = g;
-                }
-            }
-            break;
-        }
-        case EPI_FINAL: {  // v[0] = <rt, r_0>, v[1] = <r_0, r_0>
-            a.rep->rnorm = norm_sqrt(s_real(v[1]));
-            a.rep->nonfinite = bad ? 1 : 0;
-            st.rho = s_neg(s_mul(st.omega, st.rho));  // next cycle: rho = -omega rho
-            if (s_is_zero(st.rho)) a.rep->breakdown = 1;
-            st.beta = s_div(s_mul(st.alpha, v[0]), st.rho);
-            st.rho = v[0];
-            if (a.mon) monitor_step(a.mon, a.rep, a.hist, a.L, a.cond);
-            break;
-        }
-        default:
-            break;
-    }
-    st.last[0] = v[0];
-}
 
 // ------------------------------------------------------------ SpMV (+ Dot2)
 // y = D^{-1} (A x) (diag = D, may be null: no scaling), and <w, y> when DOT.
@@ -382,54 +249,75 @@ void launch_spmv_upd(int j, int L, int lm, int grid, cudaStream_t s, int32_t row
 // The combine is a separate launch (no ticket): the single-launch form with
 // a last-block epilogue stalled on B200 for this pass (every block's thread 0
 // stopped between the block barrier and the ticket atomic) and is not used.
+// Rows move as 16-byte packs (VW elements; the vectors are the workspace's,
+// aligned; the last n % VW rows one by one): with one 8-byte element a load, a
+// resident wave had too few bytes in flight to cover the memory's latency
+// (B200, 2048^2 complex<binary32>, k = L = 2: 35 us instead of 52).
+template <class E, int ND, int VW>
+__device__ __forceinline__ void mgs_rows(int64_t q, int k, bool upd, const Vecs<E>& V,
+                                         const typename scalar_of<E>::type (&ntau)[ND - 1],
+                                         typename scalar_of<E>::type nal, const E* __restrict__ pend_u,
+                                         typename pacc_of<E>::type (&pacc)[ND]) {
+    using S = typename scalar_of<E>::type;
+    constexpr int NV = ND - 1;  // r_k .. r_L
+    constexpr bool VEC = VW * sizeof(E) == 16 && VW > 1;
+    E ve[NV][VW], z[VW], pe[VW], pu[VW];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) ld_pack<E, VW, VEC, false>(V.r[k + i], q, ve[i]);
+    ld_pack<E, VW, VEC, false>(V.r[0], q, z);
+    if (upd) ld_pack<E, VW, VEC, false>(V.r[k - 1], q, pe);
+    if (pend_u) ld_pack<E, VW, VEC, false>(pend_u, q, pu);
+#pragma unroll
+    for (int j = 0; j < VW; ++j) {
+        S pv = upd ? to_s(pe[j]) : s_zero(S{});
+        if (pend_u) {
+            // k = 2, NV = L - 1: the last BiCG step's r_{L-1} -= alpha u_L,
+            // with the FMA of the other r updates (r_{L-1} = r_1 = r_{k-1}
+            // when L = 2)
+            const S uq = to_s(pu[j]);
+            if constexpr (NV >= 2) {
+                ve[NV - 2][j] = from_s<E>(s_fma(nal, uq, to_s(ve[NV - 2][j])));
+            } else {
+                pv = round_s<E>(s_fma(nal, uq, pv));
+                pe[j] = from_s<E>(pv);
+            }
+        }
+        if (upd)
+#pragma unroll
+            for (int i = 0; i < NV; ++i) ve[i][j] = from_s<E>(s_fma(ntau[i], pv, to_s(ve[i][j])));
+    }
+    if (pend_u && NV < 2) st_pack<E, VW, VEC>(V.r[k - 1], q, pe);
+    if (upd)
+#pragma unroll
+        for (int i = 0; i < NV; ++i) st_pack<E, VW, VEC>(V.r[k + i], q, ve[i]);
+#pragma unroll
+    for (int j = 0; j < VW; ++j) {
+        pdot_add(pacc[0], ve[0][j], ve[0][j]);
+        pdot_add(pacc[1], ve[0][j], z[j]);
+#pragma unroll
+        for (int i = 1; i < NV; ++i) pdot_add(pacc[1 + i], ve[0][j], ve[i][j]);
+    }
+}
+
 template <class E, int ND>  // ND = L - k + 2 inner products
 __global__ void __launch_bounds__(kThreads)
 k_mgs_step(int64_t n, int k, Vecs<E> V, const BcgState<typename scalar_of<E>::type>* st,
            typename acc_of<typename scalar_of<E>::type>::type* partials, const E* __restrict__ pend_u) {
     using S = typename scalar_of<E>::type;
     using A = typename acc_of<S>::type;
-    constexpr int NV = ND - 1;  // r_k .. r_L
+    // (binary64 packs cost more in registers, hence blocks, than they gained)
+    constexpr int NV = ND - 1, VW = std::is_same<E, double>::value ? 1 : pack_of<E>::value;
     __shared__ A sh[ND * 32];
     const bool upd = k > 1;
     S ntau[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) ntau[i] = upd ? s_neg(st->tau[k - 1][k + i]) : s_zero(S{});
-    const E* rprev = upd ? V.r[k - 1] : nullptr;
-    const E* r0 = V.r[0];
     const S nal = s_neg(st->alpha);
     typename pacc_of<E>::type pacc[ND];
-    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < n; q += stride) {
-        E ve[NV];
-#pragma unroll
-        for (int i = 0; i < NV; ++i) ve[i] = ldE(V.r[k + i], q);
-        const E z = ldE(r0, q);
-        S pv = upd ? to_s(ldE(rprev, q)) : s_zero(S{});
-        if (pend_u) {
-            // k = 2, NV = L - 1: the last BiCG step's r_{L-1} -= alpha u_L,
-            // with the FMA of the other r updates (r_{L-1} = r_1 = rprev
-            // when L = 2)
-            const S uq = to_s(ldE(pend_u, q));
-            if constexpr (NV >= 2) {
-                ve[NV - 2] = from_s<E>(s_fma(nal, uq, to_s(ve[NV - 2])));
-            } else {
-                const E pe = from_s<E>(s_fma(nal, uq, pv));
-                stE(V.r[k - 1], q, pe);
-                pv = to_s(pe);
-            }
-        }
-        if (upd) {
-#pragma unroll
-            for (int i = 0; i < NV; ++i) {
-                ve[i] = from_s<E>(s_fma(ntau[i], pv, to_s(ve[i])));
-                stE(V.r[k + i], q, ve[i]);
-            }
-        }
-        pdot_add(pacc[0], ve[0], ve[0]);
-        pdot_add(pacc[1], ve[0], z);
-#pragma unroll
-        for (int i = 1; i < NV; ++i) pdot_add(pacc[1 + i], ve[0], ve[i]);
-    }
+    const int64_t first = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, stride = int64_t(gridDim.x) * blockDim.x;
+    const int64_t nq = n / VW;
+    for (int64_t q = first; q < nq; q += stride) mgs_rows<E, ND, VW>(q, k, upd, V, ntau, nal, pend_u, pacc);
+    if (VW > 1 && first < n - nq * VW) mgs_rows<E, ND, 1>(nq * VW + first, k, upd, V, ntau, nal, pend_u, pacc);
     A acc[ND];
 #pragma unroll
     for (int d = 0; d < ND; ++d) acc[d] = widen_acc(pacc[d]);
@@ -717,6 +605,7 @@ struct BcgPlan<E>::Impl {
     int g_ew = 1, g_red = 1, g_sp = 1, g_spd = 1, g_nrm = 1, kernels = 0;
     int64_t nnz = 0;
     int lm = 0;  // load mode of the cycle's products
+    SlotMat<E> slots{};  // the matrix in slot form, when it has one (ns > 0)
     int g_su[kMaxL] = {};  // grids of the update + product kernels
     SolverWorkspace ws;
     Vecs<E> V{};
@@ -781,28 +670,29 @@ int BcgPlan<E>::init(const hpb_solver_params* p, int32_t rows, int64_t nnz, cons
     P.x = x;
     const int64_t n = rows;
     const int64_t need = (n + kThreads - 1) / kThreads;
+    SolverWorkspace& ws = P.ws;
+    int wst = ws.open(sizeof(Report) + 8 * sizeof(double) + sizeof(MonState) + 2 * kLoopChunk * sizeof(double));
+    if (wst != HPB_SUCCESS) return wst;
+    cudaStream_t s = ws.stream;
+    // allocations, the slot form and the diagonal run after the caller's work on the legacy default stream
+    if (cudaEventRecord(ws.ev, 0) != cudaSuccess || cudaStreamWaitEvent(s, ws.ev, 0) != cudaSuccess)
+        return HPB_ERROR_CUDA;
+    if (build_slots<E>(ws, rows, nnz, rp, ci, val, &P.slots) != HPB_SUCCESS) return HPB_ERROR_CUDA;
     P.g_ew = int(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * light_occupancy<E>())));
     P.g_red = int(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * reduction_occupancy<E>(L))));
     P.g_sp = int(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * 8)));  // grid-stride rows, 8 blocks per SM
     P.g_spd = int(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * 6)));
     int g_su_max = 1;
     for (int j = 0; j < L; ++j) {
-        const int cap = std::min(6, spmv_upd_occupancy<E>(j, L));
+        const int cap = P.slots.ns ? spmv_upd_slots_occupancy<E>(P.slots, j, L) : std::min(6, spmv_upd_occupancy<E>(j, L));
         P.g_su[j] = int(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * cap)));
         g_su_max = std::max(g_su_max, P.g_su[j]);
     }
     P.g_nrm = int(std::max<int64_t>(
         1, std::min<int64_t>(need, int64_t(sms) * occupancy_of(reinterpret_cast<const void*>(k_norm<E>)))));
     const int g_ew = P.g_ew, g_red = P.g_red, g_sp = P.g_sp, g_spd = P.g_spd;
-    SolverWorkspace& ws = P.ws;
     Vecs<E>& V = P.V;
     const size_t vb = size_t(n) * sizeof(E);
-    int wst = ws.open(sizeof(Report) + 8 * sizeof(double) + sizeof(MonState) + 2 * kLoopChunk * sizeof(double));
-    if (wst != HPB_SUCCESS) return wst;
-    cudaStream_t s = ws.stream;
-    // allocations and the diagonal run after the caller's work on the legacy default stream
-    if (cudaEventRecord(ws.ev, 0) != cudaSuccess || cudaStreamWaitEvent(s, ws.ev, 0) != cudaSuccess)
-        return HPB_ERROR_CUDA;
     for (int i = 0; i <= L; ++i) {
         V.r[i] = static_cast<E*>(ws.alloc(vb));
         V.u[i] = static_cast<E*>(ws.alloc(vb));
@@ -879,14 +769,24 @@ int BcgPlan<E>::init(const hpb_solver_params* p, int32_t rows, int64_t nnz, cons
     }
     for (int j = 0; j < L; ++j) {
         // u_{j+1} = A (r_j - beta u_j) and alpha = rho / <rt, u_{j+1}>
-        launch_spmv_dot<E, true, true>(lm, g_spd, s, rows, rp, ci, val, diag, V.u[j], V.u[j + 1], rt, partials,
-                                       ticket, badflag, EpiArgs<S>{st, drep, EPI_ALPHA, 0, j, L}, V.r[j]);
+        const EpiArgs<S> alpha{st, drep, EPI_ALPHA, 0, j, L};
+        if (P.slots.ns)
+            launch_spmv_dot_slots<E>(P.slots, true, g_spd, s, rows, diag, V.u[j], V.u[j + 1], rt, partials, ticket,
+                                     badflag, alpha, V.r[j]);
+        else
+            launch_spmv_dot<E, true, true>(lm, g_spd, s, rows, rp, ci, val, diag, V.u[j], V.u[j + 1], rt, partials,
+                                           ticket, badflag, alpha, V.r[j]);
         // the BiCG updates of step j (r_j's deferred) and r_{j+1} = A r_j';
         // before the last step rho = <rt, r_{j+1}> and beta, at it the first
         // MR sweep's inner products
         const bool last = j + 1 == L;
-        launch_spmv_upd<E>(j, L, lm, P.g_su[j], s, rows, rp, ci, val, diag, V, x, rt, st, partials, ticket,
-                           badflag, last ? none : EpiArgs<S>{st, drep, EPI_BETA, 0, j, L});
+        const EpiArgs<S> beta = last ? none : EpiArgs<S>{st, drep, EPI_BETA, 0, j, L};
+        if (P.slots.ns)
+            launch_spmv_upd_slots<E>(P.slots, j, L, P.g_su[j], s, rows, diag, V, x, rt, st, partials, ticket, badflag,
+                                     beta);
+        else
+            launch_spmv_upd<E>(j, L, lm, P.g_su[j], s, rows, rp, ci, val, diag, V, x, rt, st, partials, ticket, badflag,
+                               beta);
         kernels += 2;
     }
     // MR part: the first sweep's combine, then sweeps 2..L; the second

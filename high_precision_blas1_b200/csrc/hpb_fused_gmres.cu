@@ -96,35 +96,6 @@ __device__ __forceinline__ void giv_apply(cd& dx, cd& dy, cd c, cd s) {
 __device__ __forceinline__ double s_abs(double v) { return fabs(v); }
 __device__ __forceinline__ double s_abs(cd v) { return cabs_(v); }
 
-// ------------------------------------------------------------ 16-byte packs
-// VW consecutive elements q*VW .. q*VW + VW - 1 of a vector moved as one
-// 16-byte access (VEC: VW * sizeof(E) == 16 and the vector 16-byte
-// aligned), or one element through ldE / stE (VW == 1).
-template <class E> struct pack_of { static constexpr int value = 16 / int(sizeof(E)); };
-
-template <class E, int VW, bool VEC, bool RO>
-__device__ __forceinline__ void ld_pack(const E* p, int64_t q, E (&o)[VW]) {
-    if constexpr (VEC) {
-        static_assert(VW * sizeof(E) == 16, "one 16-byte pack");
-        const uint4* a = reinterpret_cast<const uint4*>(p) + q;
-        const uint4 t = RO ? __ldg(a) : *a;
-        memcpy(&o[0], &t, 16);
-    } else {
-        static_assert(VW == 1, "one element");
-        o[0] = RO ? ldgE(p, q) : ldE(p, q);
-    }
-}
-template <class E, int VW, bool VEC>
-__device__ __forceinline__ void st_pack(E* p, int64_t q, const E (&v)[VW]) {
-    if constexpr (VEC) {
-        uint4 t;
-        memcpy(&t, &v[0], 16);
-        reinterpret_cast<uint4*>(p)[q] = t;
-    } else {
-        stE(p, q, v[0]);
-    }
-}
-
 // ------------------------------------------------------------ DCGS2 step
 // Arnoldi by classical Gram-Schmidt with a delayed re-orthogonalisation
 // (DCGS2).  At step i the slot V_i holds u: the previous step's vector after
