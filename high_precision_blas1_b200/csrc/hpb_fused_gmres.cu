@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "hpb_fused.cuh"
+#include "hpb_slots.cuh"
 
 namespace hpb {
 namespace fused {
@@ -252,8 +253,8 @@ k_dcgs_dots(int64_t n, int K, int vec, const E* __restrict__ V, const E* __restr
 // the 2T packed accumulators per pass merges the warp.  R is set per launch
 // so the grid is about one resident wave.
 constexpr int kF32T = 4;       // basis vectors per pass
-constexpr int kF32MaxR = 2;    // packs per thread per pass, at most
-constexpr int kF32BlocksPerSm = 3;
+constexpr int kF32MaxR = 7;    // packs per thread per pass, at most
+constexpr int kF32BlocksPerSm = 2;
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const unsigned a = static_cast<unsigned>(__cvta_generic_to_shared(smem));
@@ -785,20 +786,34 @@ k_gm_start(int64_t n, const E* __restrict__ r, E* __restrict__ v0, GmState<typen
     }
 }
 
-// back substitution H(0:k,0:k) y = s(0:k), k = nsteps - 1 (one thread)
+// back substitution H(0:k,0:k) y = s(0:k), k = nsteps: one thread, from the
+// triangle that the block has brought to shared memory (from global memory its
+// k^2 / 2 loads took 114 us at k = 50 on B200, now 9 us; same operations)
 template <class S>
-__global__ void k_gm_solve(GmState<S>* st, int m) {
-    const int ld = m + 1, k = st->nsteps;
-    for (int j = 0; j < m; ++j) {
-        st->y[j] = s_zero(S{});
-        st->neg_y[j] = s_zero(S{});
+__global__ void __launch_bounds__(kGmThreads) k_gm_solve(GmState<S>* st, int m) {
+    extern __shared__ __align__(16) unsigned char solve_raw[];
+    S* const sh = reinterpret_cast<S*>(solve_raw);  // column l's rows 0..l at l (l + 1) / 2, then s, then y
+    const int ld = m + 1, k = st->nsteps, tri = m * (m + 1) / 2;
+    S *const ss = sh + tri, *const sy = ss + m;
+    for (int l = threadIdx.x >> 5; l < k; l += kGmThreads / 32)
+        for (int r = threadIdx.x & 31; r <= l; r += 32) sh[l * (l + 1) / 2 + r] = st->H[size_t(l) * ld + r];
+    for (int j = threadIdx.x; j < m; j += kGmThreads) {
+        if (j < k) ss[j] = st->s[j];
+        sy[j] = s_zero(S{});
     }
-    for (int j = k - 1; j >= 0; --j) {
-        S v = st->s[j];
-        for (int l = j + 1; l < k; ++l) v = s_sub(v, s_mul(st->H[size_t(l) * ld + j], st->y[l]));
-        st->y[j] = s_div(v, st->H[size_t(j) * ld + j]);
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int j = k - 1; j >= 0; --j) {
+            S v = ss[j];
+#pragma unroll 4
+            for (int l = j + 1; l < k; ++l) v = s_sub(v, s_mul(sh[l * (l + 1) / 2 + j], sy[l]));
+            sy[j] = s_div(v, sh[j * (j + 1) / 2 + j]);
+        }
+    __syncthreads();
+    for (int j = threadIdx.x; j < m; j += kGmThreads) {
+        st->y[j] = sy[j];
+        st->neg_y[j] = j < k ? s_neg(sy[j]) : s_zero(S{});
     }
-    for (int j = 0; j < k; ++j) st->neg_y[j] = s_neg(st->y[j]);
 }
 
 // y = x ./ d (Jacobi application as a right preconditioner)
@@ -827,10 +842,32 @@ k_gm_spmv(int32_t rows, const int32_t* __restrict__ rp, const int32_t* __restric
     }
 }
 
-// k_gm_spmv under the load mode of its matrix and x
+// the same product with the matrix in slot form (hpb_slots.cuh); x and y are
+// workspace vectors
+template <class E, int NS>
+__global__ void __launch_bounds__(kGmThreads)
+k_gm_spmv_slots(int32_t rows, SlotMat<E> A, const E* __restrict__ x, E* __restrict__ y) {
+    using S = typename scalar_of<E>::type;
+    const int32_t stride = gridDim.x * kGmThreads;
+    for (int32_t r = blockIdx.x * kGmThreads + threadIdx.x; r < rows; r += stride) {
+        SlotRow<E, NS, SlotX<E>> row;
+        row.load(A, rows, r, [&](int32_t c) { return SlotX<E>{ld_x<LM_ALIGNED>(x, c)}; });
+        stE(y, r, from_s<E>(row.sum(s_zero(S{}))));
+    }
+}
+
+// k_gm_spmv under the load mode of its matrix and x, or the slot form where there is one
 template <class E>
 void launch_gm_spmv(int grid, cudaStream_t s, int32_t rows, int64_t nnz, const int32_t* rp, const int32_t* ci,
-                    const E* val, const E* x, E* y) {
+                    const E* val, const SlotMat<E>& A, const E* x, E* y) {
+    if (A.ns > 5) {
+        k_gm_spmv_slots<E, 7><<<grid, kGmThreads, 0, s>>>(rows, A, x, y);
+        return;
+    }
+    if (A.ns > 0) {
+        k_gm_spmv_slots<E, 5><<<grid, kGmThreads, 0, s>>>(rows, A, x, y);
+        return;
+    }
     dispatch_lm<E>(load_mode<E>(val, x, nnz), [&](auto mode) {
         constexpr int M = decltype(mode)::value;
         k_gm_spmv<E, M><<<grid, kGmThreads, 0, s>>>(rows, rp, ci, val, x, y);
@@ -958,6 +995,7 @@ struct GmPlan<E>::Impl {
     int lm_res = 0;            // load mode of the compensated residual
     SolverWorkspace ws;
     E *V = nullptr, *W = nullptr, *Z = nullptr, *R = nullptr, *diag = nullptr, *T = nullptr;
+    SlotMat<E> slots{}, mslots{};  // A and the CSR preconditioner in slot form (ns > 0: there is one)
     GmState<S>* st = nullptr;
     A* partials = nullptr;
     unsigned int* ticket = nullptr;
@@ -1020,6 +1058,11 @@ int GmPlan<E>::init(const hpb_solver_params* p, int32_t rows, int64_t nnz, const
     cudaStream_t s = ws.stream;
     // allocations and the diagonal run after the caller's work on the legacy default stream
     if (cudaEventRecord(ws.ev, 0) != cudaSuccess || cudaStreamWaitEvent(s, ws.ev, 0) != cudaSuccess)
+        return HPB_ERROR_CUDA;
+    if (build_slots<E>(ws, rows, nnz, rp, ci, val, &P.slots) != HPB_SUCCESS ||
+        (M.kind == 2 && M.rows == rows &&
+         build_slots<E>(ws, M.rows, M.nnz, M.rp, M.ci, M.val, &P.mslots,
+                        M.rp == rp && M.ci == ci && M.nnz == nnz ? &P.slots : nullptr) != HPB_SUCCESS))
         return HPB_ERROR_CUDA;
     E* V = P.V = static_cast<E*>(ws.alloc(vb * size_t(m + 1)));
     E* W = P.W = static_cast<E*>(ws.alloc(vb));
@@ -1094,7 +1137,7 @@ int GmPlan<E>::init(const hpb_solver_params* p, int32_t rows, int64_t nnz, const
             src = Z;
             ++kernels;
         } else if (M.kind == 2) {
-            launch_gm_spmv<E>(g_sp, s, M.rows, M.nnz, M.rp, M.ci, M.val, vi, Z);
+            launch_gm_spmv<E>(g_sp, s, M.rows, M.nnz, M.rp, M.ci, M.val, P.mslots, vi, Z);
             src = Z;
             ++kernels;
         } else if (M.kind == 3 && M.sweeps == 0) {  // z = U^-1 L^-1 v_i (R is free inside the cycle)
@@ -1108,7 +1151,7 @@ int GmPlan<E>::init(const hpb_solver_params* p, int32_t rows, int64_t nnz, const
             src = Z;
             kernels += 2 * (M.sweeps + 1);
         }
-        launch_gm_spmv<E>(g_sp, s, rows, nnz, rp, ci, val, src, W);
+        launch_gm_spmv<E>(g_sp, s, rows, nnz, rp, ci, val, P.slots, src, W);
         int nb = g_md;
         if constexpr (std::is_same<E, float>::value) {
             if (g_f32 > 0) {
@@ -1128,7 +1171,7 @@ int GmPlan<E>::init(const hpb_solver_params* p, int32_t rows, int64_t nnz, const
     k_dcgs_dots<E, false><<<g_md, kGmThreads, 0, s>>>(n, m, vec, V, static_cast<const E*>(nullptr), partials);
     k_dcgs_finish<S><<<m + 1, kGmThreads, 0, s>>>(g_md, m, 1, partials, st, m, ticket);
     kernels += 2;
-    k_gm_solve<S><<<1, 1, 0, s>>>(st, m);
+    k_gm_solve<S><<<1, kGmThreads, size_t(m * (m + 1) / 2 + 2 * m) * sizeof(S), s>>>(st, m);
     ++kernels;
     if (M.kind == 0) {
         k_gs_update<E><<<g_ew, kGmThreads, 0, s>>>(n, m, V, x, x, st->neg_y);
@@ -1140,7 +1183,7 @@ int GmPlan<E>::init(const hpb_solver_params* p, int32_t rows, int64_t nnz, const
         if (M.kind == 1) {
             k_gm_jacobi<E><<<g_ew, kGmThreads, 0, s>>>(n, W, diag, Z);
         } else if (M.kind == 2) {
-            launch_gm_spmv<E>(g_sp, s, M.rows, M.nnz, M.rp, M.ci, M.val, W, Z);
+            launch_gm_spmv<E>(g_sp, s, M.rows, M.nnz, M.rp, M.ci, M.val, P.mslots, W, Z);
         } else if (M.sweeps == 0) {
             tri::launch_trsv<E>(M.lower->plan, 1, M.val, unit_of<E>(), W, R, s);
             tri::launch_trsv<E>(M.upper->plan, 0, M.val, unit_of<E>(), R, Z, s);
