@@ -251,7 +251,10 @@ k_dcgs_dots(int64_t n, int K, int vec, const E* __restrict__ V, const E* __restr
 // (pass, pack) step ahead, across pass boundaries, so the next step's loads
 // are in flight while the current one is computed.  One reduce-scatter of
 // the 2T packed accumulators per pass merges the warp.  R is set per launch
-// so the grid is about one resident wave.
+// so the grid is about one resident wave: up to seven packs at two blocks an
+// SM, so that few merges are made.  A refined GMRES(50) solve on 128^3 rows on
+// B200: 253 ms with at most two packs at three blocks, 259 ms with four at
+// three, 249 ms with five at two, 235 ms with seven at two.
 constexpr int kF32T = 4;       // basis vectors per pass
 constexpr int kF32MaxR = 7;    // packs per thread per pass, at most
 constexpr int kF32BlocksPerSm = 2;
@@ -788,7 +791,8 @@ k_gm_start(int64_t n, const E* __restrict__ r, E* __restrict__ v0, GmState<typen
 
 // back substitution H(0:k,0:k) y = s(0:k), k = nsteps: one thread, from the
 // triangle that the block has brought to shared memory (from global memory its
-// k^2 / 2 loads took 114 us at k = 50 on B200, now 9 us; same operations)
+// k^2 / 2 loads took 114 us at k = 50 on B200, now 30 us; same operations).
+// What is left is the chain of k^2 / 2 dependent multiply-subtracts.
 template <class S>
 __global__ void __launch_bounds__(kGmThreads) k_gm_solve(GmState<S>* st, int m) {
     extern __shared__ __align__(16) unsigned char solve_raw[];

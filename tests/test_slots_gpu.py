@@ -111,3 +111,27 @@ def test_matrices_without_a_slot_form(gpu, kind):
     dense = np.zeros((n, n))
     np.add.at(dense, (np.repeat(np.arange(n), np.diff(A.row_ptr)), A.col_ind), A.val)
     assert np.linalg.norm(dense @ x - b) <= 1e-9 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("t", ["f64", "f32", "c128", "c64"])
+@pytest.mark.parametrize("kind,n,m,jacobi", [("five", 255, 3, False), ("seven", 9000, 10, False), ("one-sided", 5000, 8, True),
+                                             ("tri", 3001, 5, True)])
+def test_gmres_slots(gpu, kind, n, m, jacobi, t):
+    compare(gpu[1], kind, n, t, m, jacobi, 2 * m, gmres=True)
+
+
+@pytest.mark.parametrize("packs", [1, 2, 4, 7, 9])
+def test_gmres_binary32_reduction(gpu, packs):
+    """One cycle of binary32 GMRES against binary64 GMRES with `packs` packs a
+    thread (more than the kernel takes at once for 9), the last pass ragged.
+    Binary32 rounding moves a few steps on a matrix of condition below 2 by
+    some 1e-6; an inner product without its last block moves them by 1e-3."""
+    ctx, torch = gpu
+    wave = 256 * 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    n = 4 * (wave * (packs - 1) + 5)
+    rng = np.random.default_rng(packs)
+    A = csr(n, *matrix("tri", n, rng, False))
+    A.val = A.val.astype(np.float32).astype(np.float64)
+    b = rng.standard_normal(n).astype(np.float32).astype(np.float64)
+    x, y = (solve(torch, A, b, t, 4, False, 4, gmres=True) for t in ("f32", "f64"))
+    assert np.linalg.norm(x - y) <= 1e-4 * np.linalg.norm(y)
