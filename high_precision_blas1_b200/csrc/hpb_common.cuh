@@ -52,6 +52,16 @@ __device__ __forceinline__ void pdl_enter() {
 #endif
 }
 
+// pdl_enter for a kernel that reads through the read-only path (__ldg,
+// const __restrict__): the pointers are made to depend on the wait, so that
+// the compiler cannot move such a load, which it may take to be invariant,
+// ahead of it.
+template <class... T>
+__device__ __forceinline__ void pdl_enter_for(T&... p) {
+    pdl_enter();
+    ([&] { asm volatile("" : "+l"(p)::"memory"); }(), ...);
+}
+
 template <class... KArgs, class... Args>
 inline cudaError_t launch_pdl(cudaStream_t s, int grid, int block, void (*kernel)(KArgs...), Args&&... args) {
     cudaLaunchConfig_t cfg{};
