@@ -265,7 +265,21 @@ constexpr int kCombThreads = 512;   // context entry points
 constexpr int kRedUnroll = 4;
 // TAIL_TICKET: fence + ticket, block-wide final merge (allocation-free entry
 // point); TAIL_WARP: acquire-release ticket, one-warp final merge.
-enum Tail { TAIL_TICKET = 0, TAIL_WARP = 1 };
+// TAIL_ONE: the whole reduction in one block, nothing to merge.
+enum Tail { TAIL_TICKET = 0, TAIL_WARP = 1, TAIL_ONE = 2 };
+constexpr int kOneThreads = 1024;  // TAIL_ONE: at most, kRedUnroll packs each
+
+// Blocks of kCombThreads that have to fit an SM.  The single-input reductions
+// of binary32 storage take few instructions an element and are bound by the
+// loads in flight: with a register bound for three blocks the compiler issues
+// a step's four loads together (nrm2 of 33.5 M c64 on B200: 47.4 -> 43.6 us).
+// Bounding the others cost more than it gave (f64 dot2 of 16 M 40.4 -> 44.7,
+// f64 nrm2 of 16.8 M 25.6 -> 26.9 us), and so did four blocks (44.9) and six or
+// eight packs a step (44.3 and 46.0 us; f64 dot2 40.5 and 71.4).
+template <class E, int OP>
+constexpr int red_min_blocks() {
+    return sizeof(typename real_of<E>::type) == 4 && !op_has_y(OP) ? 3 : 0;  // 0: no bound
+}
 
 __device__ __forceinline__ unsigned atom_add_acq_rel(unsigned int* p, unsigned v) {
     unsigned r;
@@ -300,7 +314,7 @@ __device__ __forceinline__ void write_result(double* o, W S, W C, int op) {
 // sync: the ticket counter.  host_flag (by-value calls): after the result,
 // the last block raises this pinned host word to host_seq.
 template <class E, int OP, bool VEC, int THREADS = kRedThreads, int TAIL = TAIL_TICKET>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, TAIL == TAIL_WARP ? red_min_blocks<E, OP>() : 0)
 reduce_kernel(int64_t n, const E* __restrict__ x, const E* __restrict__ y, void* __restrict__ partials,
               unsigned int* __restrict__ sync, double* __restrict__ out, unsigned int* host_flag = nullptr,
               unsigned host_seq = 0) {
@@ -317,7 +331,36 @@ reduce_kernel(int64_t n, const E* __restrict__ x, const E* __restrict__ y, void*
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     const int64_t nv = n / K;  // full vectors
 
-    if (VEC) {
+    if constexpr (TAIL == TAIL_ONE) {
+        // at most kRedUnroll packs (elements) a thread, all loaded at once
+        const int items = int(VEC ? nv : n), bd = int(blockDim.x), t = int(threadIdx.x);
+        const int64_t i = nv * K + t;
+        const bool ragged = VEC && i < n;
+        E ex{}, ey{};
+        if (ragged) {
+            ex = ldE(x, i);
+            if (op_has_y(OP)) ey = ldE(y, i);
+        }
+        Pack<E> px[kRedUnroll], py[kRedUnroll];
+#pragma unroll
+        for (int u = 0; u < kRedUnroll; ++u)
+            if (t + u * bd < items) {
+                if constexpr (VEC) {
+                    px[u] = ld16<E>(x, t + u * bd);
+                    if (op_has_y(OP)) py[u] = ld16<E>(y, t + u * bd);
+                } else {
+                    px[u].v[0] = ldE(x, t + u * bd);
+                    if (op_has_y(OP)) py[u].v[0] = ldE(y, t + u * bd);
+                }
+            }
+#pragma unroll
+        for (int u = 0; u < kRedUnroll; ++u)
+            if (t + u * bd < items)
+#pragma unroll
+                for (int k = 0; k < K; ++k)
+                    Term<E, OP>::add(s, c, px[u].v[k], op_has_y(OP) ? py[u].v[k] : px[u].v[k]);
+        if (ragged) Term<E, OP>::add(s, c, ex, op_has_y(OP) ? ey : ex);
+    } else if (VEC) {
         int64_t v = gtid;
         for (; v + (kRedUnroll - 1) * stride < nv; v += kRedUnroll * stride) {
             Pack<E> px[kRedUnroll], py[kRedUnroll];
@@ -357,6 +400,16 @@ reduce_kernel(int64_t n, const E* __restrict__ x, const E* __restrict__ y, void*
     __shared__ bool am_last;
     block_combine<COMP>(ws, wc, sh);
 
+    if constexpr (TAIL == TAIL_ONE) {
+        if (threadIdx.x == 0) {
+            write_result<W>(out, ws, wc, OP);
+            if (host_flag != nullptr) {
+                __threadfence_system();
+                *reinterpret_cast<volatile unsigned int*>(host_flag) = host_seq;
+            }
+        }
+        return;
+    }
     W* part = reinterpret_cast<W*>(partials);
     if constexpr (TAIL == TAIL_WARP) {
         if (threadIdx.x == 0) {
@@ -467,6 +520,23 @@ int launch_reduce(hpb_context* ctx, int64_t n, const E* x, const E* y, double* o
     const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(op_has_y(OP) ? y : x)) & 15) == 0;
     const int K = aligned ? VecOf<E>::k : 1;
     const int64_t work = (n / K + kRedUnroll - 1) / kRedUnroll;
+    const int64_t items = n / K;
+    if (items <= kOneThreads * kRedUnroll) {
+        // One block: no partials to write and no ticket to draw.  The line is
+        // where kRedUnroll packs a thread no longer cover the vector.  B200,
+        // against two to eight blocks with a ticket: f64 dot2 of 5000 returned
+        // by value 12.1 -> 11.1 us, of 8000 left on the device 3.9 -> 3.4 us,
+        // f32 nrm2 of 16000 4.0 -> 3.1 us.
+        const int threads = int(std::min<int64_t>(kOneThreads, std::max<int64_t>(32, (items + 31) / 32 * 32)));
+        if (aligned)
+            launch_pdl(ctx->stream, 1, threads, reduce_kernel<E, OP, true, kOneThreads, TAIL_ONE>, n, x, y,
+                       ctx->partials, ctx->red_ticket, out, host_flag, host_seq);
+        else
+            launch_pdl(ctx->stream, 1, threads, reduce_kernel<E, OP, false, kOneThreads, TAIL_ONE>, n, x, y,
+                       ctx->partials, ctx->red_ticket, out, host_flag, host_seq);
+        count_launch();
+        return check_launch(ctx, name);
+    }
     // one resident wave at most (grid capped at the occupancy)
     if (aligned) {
         int grid = grid_for(ctx, work, kCombThreads, 1 << 20);
