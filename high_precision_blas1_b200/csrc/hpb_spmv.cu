@@ -8,9 +8,8 @@
 // the CSR arrays; they are streaming loads (evict-first: each nonzero is
 // read once), while x is gathered through the read-only path, where the
 // 5/7-point stencil neighbours of consecutive rows hit in L1/L2.  On B200 at
-// 1024^2 (f64, 5-point) this measured 5.1 TB/s against 3.7 TB/s for staging
-// each block's nonzero range through shared memory first (the barrier
-// between the two memory phases left HBM idle).  Per-row sums run in index
+// 1024^2 (f64, 5-point, not in L2) this measured 14.1 us against 20.2 us for
+// copying each warp's values and indices to shared memory first.  Per-row sums run in index
 // order with one FMA per nonzero.
 #include "hpb_common.cuh"
 #include "hpb_fused.cuh"
@@ -31,21 +30,66 @@ __device__ __forceinline__ cf mul_s(cf a, cf b) { return cmul(a, b); }
 __device__ __forceinline__ cd mul_s(cd a, cd b) { return cmul(a, b); }
 
 constexpr int kSpmvRows = 256;  // rows (threads) per block
+constexpr int kRowBatch = 5;    // entries whose loads are issued together
+constexpr int kSpmvPerSm = 16;  // blocks an SM, twice what is resident
+
+// A row's entries: with BATCH, kRowBatch of them at a time, all indices and
+// values loaded before the gathers and these before the FMAs, so that a row
+// waits for three loads one after the other (row pointers, indices, x) and not
+// for five, as the compiler's own unrolling by four leaves a five-point row.
+
+template <class E, int LM, bool BATCH>
+__device__ __forceinline__ E row_sum(int32_t b, int32_t e, const int32_t* __restrict__ ci, const E* __restrict__ val,
+                                     const E* __restrict__ x) {
+    constexpr int U = kRowBatch;
+    E acc{};
+    if constexpr (!BATCH) {
+        for (int32_t k = b; k < e; ++k) acc = madd_s(ld_val<LM>(val, k), ld_x<LM>(x, ld_idx<LM>(ci, k)), acc);
+        return acc;
+    }
+    for (int32_t k = b; k < e; k += U) {
+        int32_t c[U];
+        E v[U], xv[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (u < e - k) c[u] = ld_idx<LM>(ci, k + u);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (u < e - k) v[u] = ld_val<LM>(val, k + u);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (u < e - k) xv[u] = ld_x<LM>(x, c[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (u < e - k) acc = madd_s(v[u], xv[u], acc);
+        if (e - k <= U) break;  // (k + U may not fit an int32_t)
+    }
+    return acc;
+}
 
 // LM: the load mode of the matrix and x (ld_val, ld_x)
-template <class E, bool BETA0, int LM>
+//
+// Rows in a grid-stride loop over kSpmvPerSm blocks per SM; each row's sum in
+// index order, so the result does not depend on the launch shape or on BATCH.
+// Bound by HBM once the loads are in flight.  B200, against the loop of one
+// entry at a time over 8 blocks per SM (five-point operators on 1024^2 and
+// 2048^2 rows, seven-point ones on 128^3 and 100^3, alpha A x):
+//   f64  1024^2  14.5 -> 12.1 us      f32  2048^2  35.1 -> 32.9 us
+//   c128 1024^2  28.8 -> 21.7 us      c64  2048^2  56.8 -> 55.8 us
+//   f64  128^3   41.2 -> 33.8 us      f32  128^3   24.7 -> 24.1 us
+//   c64  100^3   20.7 -> 16.8 us      c128 100^3   43.2 -> 32.1 us
+// (among other matrices, so that none of it is in L2: f64 1024^2 17.7 ->
+// 14.1 us).  Batches of 4, 6 and 8 gave 17.3, 17.8 and 15.7 us there (more
+// registers, fewer warps); 8 blocks per SM 15.1, one row a thread 14.4.
+template <class E, bool BETA0, int LM, bool BATCH>
 __global__ void __launch_bounds__(kSpmvRows)
 csr_row_kernel(int32_t rows, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
                const E* __restrict__ val, E alpha, const E* __restrict__ x, E beta, E* __restrict__ y) {
-    // rows in a grid-stride loop over 8 blocks per SM (B200, 1024^2 5-point
-    // operator: 14.7 us against 16.4 us for one row per thread over 4096
-    // blocks); each row's sum in index order, so the result does not depend
-    // on the launch shape
-    const int32_t stride = gridDim.x * kSpmvRows;
-    for (int32_t r = blockIdx.x * kSpmvRows + threadIdx.x; r < rows; r += stride) {
+    pdl_enter_for(rp, ci, val, x, y);
+    const uint32_t stride = gridDim.x * kSpmvRows;
+    for (uint32_t r = blockIdx.x * kSpmvRows + threadIdx.x; r < uint32_t(rows); r += stride) {
         const int32_t b = __ldg(rp + r), e = __ldg(rp + r + 1);
-        E acc{};
-        for (int32_t k = b; k < e; ++k) acc = madd_s(ld_val<LM>(val, k), ld_x<LM>(x, ld_idx<LM>(ci, k)), acc);
+        const E acc = row_sum<E, LM, BATCH>(b, e, ci, val, x);
         E out = BETA0 ? mul_s(alpha, acc) : madd_s(alpha, acc, mul_s(beta, ldE(y, r)));
         stE(y, r, out);
     }
@@ -79,12 +123,12 @@ csr_row_dot_kernel(int32_t rows, const int32_t* __restrict__ rp, const int32_t* 
                    int* badflag, double* out) {
     using S = typename fused::scalar_of<E>::type;
     using A = typename fused::acc_of<S>::type;
+    pdl_enter_for(rp, ci, val, x, y, w, partials, ticket, out);
     A d[1];
     const int32_t stride = gridDim.x * kSpmvRows;
     for (int32_t r = blockIdx.x * kSpmvRows + threadIdx.x; r < rows; r += stride) {
         const int32_t b = __ldg(rp + r), e = __ldg(rp + r + 1);
-        E acc{};
-        for (int32_t k = b; k < e; ++k) acc = madd_s(ld_val<LM>(val, k), ld_x<LM>(x, ld_idx<LM>(ci, k)), acc);
+        const E acc = row_sum<E, LM, false>(b, e, ci, val, x);  // (batches: 21.3 us against 18.5 at 1024^2)
         stE(y, r, acc);
         fused::dot_add(d[0], fused::to_s(ldE(w, r)), fused::to_s(acc));
     }
@@ -109,13 +153,22 @@ int spmv_impl(hpb_context* ctx, int32_t rows, int32_t cols, int64_t nnz, const i
     if ((reinterpret_cast<uintptr_t>(val) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) % kA ||
         (reinterpret_cast<uintptr_t>(rp) | reinterpret_cast<uintptr_t>(ci)) % 4)
         return set_error(ctx, HPB_ERROR_INVALID_VALUE, "%s: pointer not aligned to its element type", name);
-    const int grid = grid_for(ctx, rows, kSpmvRows, 8);
-    dispatch_lm<E>(load_mode<E>(val, x, nnz), [&](auto mode) {
+    const int lm = load_mode<E>(val, x, nnz);
+    // Matrices well above L2 with more than a batch of entries a row keep the
+    // plain loop: it measured 97 us on the seven-point operator of 180^3 rows in
+    // binary64 (B200), the batches 104 us.
+    const bool batch = !(lm & LM_CACHED) || nnz <= int64_t(rows) * kRowBatch;
+    const int grid = grid_for(ctx, rows, kSpmvRows, batch ? kSpmvPerSm : kSpmvPerSm / 2);
+    dispatch_lm<E>(lm, [&](auto mode) {
         constexpr int M = decltype(mode)::value;
-        if (is_zero(beta))
-            csr_row_kernel<E, true, M><<<grid, kSpmvRows, 0, ctx->stream>>>(rows, rp, ci, val, alpha, x, beta, y);
-        else
-            csr_row_kernel<E, false, M><<<grid, kSpmvRows, 0, ctx->stream>>>(rows, rp, ci, val, alpha, x, beta, y);
+        auto go = [&](auto kernel) {
+            launch_pdl(ctx->stream, grid, kSpmvRows, kernel, rows, rp, ci, val, alpha, x, beta, y);
+        };
+        const bool b0 = is_zero(beta);
+        if (batch)
+            b0 ? go(csr_row_kernel<E, true, M, true>) : go(csr_row_kernel<E, false, M, true>);
+        else if constexpr ((M & LM_CACHED) != 0)
+            b0 ? go(csr_row_kernel<E, true, M, false>) : go(csr_row_kernel<E, false, M, false>);
     });
     count_launch();
     return check_launch(ctx, name);
@@ -149,9 +202,8 @@ int spmv_dot2_impl(hpb_context* ctx, int32_t rows, int32_t cols, int64_t nnz, co
     // ticket[1] serves as the (unused) non-finite flag and stays zero.
     dispatch_lm<E>(load_mode<E>(val, x, nnz), [&](auto mode) {
         constexpr int M = decltype(mode)::value;
-        csr_row_dot_kernel<E, M><<<grid, kSpmvRows, 0, ctx->stream>>>(rows, rp, ci, val, x, y, w,
-                                                                      static_cast<A*>(ctx->partials), ctx->ticket,
-                                                                      reinterpret_cast<int*>(ctx->ticket + 1), out);
+        launch_pdl(ctx->stream, grid, kSpmvRows, csr_row_dot_kernel<E, M>, rows, rp, ci, val, x, y, w,
+                   static_cast<A*>(ctx->partials), ctx->ticket, reinterpret_cast<int*>(ctx->ticket + 1), out);
     });
     count_launch();
     return check_launch(ctx, name);
