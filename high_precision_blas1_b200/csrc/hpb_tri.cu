@@ -801,8 +801,8 @@ __global__ void k_tri_fill(int32_t n, E* __restrict__ x, unsigned* ticket) {
 // row's FMAs and a shared store (and, at a non-unit diagonal, a division),
 // whatever the number of rows up to 32; wider levels take several chunks.
 // Measured on B200 (f64, ILU(0) factors of the 1024^2 5-point operator, 2047
-// levels in 128 tiles): lower / upper solve 378-384 / 590-616 us, against
-// 1140 / 1320 us for levels handed round 15 warps one by one (0.22 us a level
+// levels in 128 tiles): lower + upper solve 972 us, against
+// 2460 us for levels handed round 15 warps one by one (0.22 us a level
 // in a single tile, here 0.04: 78 cycles, 180 with the division) with a
 // receiver warp for the other tiles' values; 96^3 7-point 330 / 345 against
 // 846 / 821 us.  What is left is the chain itself and, at each of the 127
@@ -918,14 +918,20 @@ __device__ __forceinline__ void gather_val(RowData<E>& r, const E* __restrict__ 
 }
 
 // The chain of one chunk whose rows have at most ND dependencies: `steps`
-// levels, this lane's row in level `mine` (0: no row).  Every lane computes
+// levels, this lane's row in level `mine` (0: no row).  The turn is taken and
+// handed on in here, with nothing but the levels between: with the choice of
+// ND after the turn was taken, and the last level's values published before it
+// was handed on, a chunk took 100 cycles longer (lower / upper solve of one
+// tile of 1024 x 8 points 103 / 192 us, 82 / 160 as it is).  Every lane computes
 // in every step and only the level's lanes store, so a step has no divergent
 // branch: a lane's term past its own count has a zero value and a source that
 // holds a value already (complex: it is left out, since adding +0 to -0 would
 // change the sign of a zero).
 template <class E, bool UNIT, int ND>
 __device__ __forceinline__ void solve_steps(const RowData<E>& r, const Prep<E>& prep, const E* const (&src)[kPre], E* out,
-                                            int steps, int mine, bool publish, E* xo) {
+                                            int steps, int mine, bool publish, E* xo, int from, int to) {
+    __syncwarp();
+    if (from >= 0) chunk_sync(from);  // the chunks before this one are complete
 #pragma unroll 1
     for (int l = 1; l <= steps; ++l) {
         const bool on = mine == l;
@@ -941,6 +947,7 @@ __device__ __forceinline__ void solve_steps(const RowData<E>& r, const Prep<E>& 
         if (!UNIT) acc = quot_prepared(acc, r.dg, prep, on);
         if (on) *out = acc;
         __syncwarp();
+        if (l == steps && to >= 0) chunk_arrive(to);  // the next chunk goes first
         if (on && publish) Pub<E>::store(xo, 0, acc);
     }
 }
@@ -1017,15 +1024,16 @@ k_trsv(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int4* __r
                 if (pend == 0u) break;
             }
         }
-        __syncwarp();
-        if (c > 0) chunk_sync(w == 0 ? kSolveWarps - 1 : w - 1);  // the chunks before this one are complete
+        const int from = c > 0 ? (w == 0 ? kSolveWarps - 1 : w - 1) : -1, to = c + 1 < nc ? w : -1;
         switch (most) {
-            case 0: solve_steps<E, UNIT, 0>(r, prep, src, out, steps, mine, publish, xo); break;
-            case 1: solve_steps<E, UNIT, 1>(r, prep, src, out, steps, mine, publish, xo); break;
-            case 2: solve_steps<E, UNIT, 2>(r, prep, src, out, steps, mine, publish, xo); break;
-            case 3: solve_steps<E, UNIT, 3>(r, prep, src, out, steps, mine, publish, xo); break;
-            case 4: solve_steps<E, UNIT, 4>(r, prep, src, out, steps, mine, publish, xo); break;
+            case 0: solve_steps<E, UNIT, 0>(r, prep, src, out, steps, mine, publish, xo, from, to); break;
+            case 1: solve_steps<E, UNIT, 1>(r, prep, src, out, steps, mine, publish, xo, from, to); break;
+            case 2: solve_steps<E, UNIT, 2>(r, prep, src, out, steps, mine, publish, xo, from, to); break;
+            case 3: solve_steps<E, UNIT, 3>(r, prep, src, out, steps, mine, publish, xo, from, to); break;
+            case 4: solve_steps<E, UNIT, 4>(r, prep, src, out, steps, mine, publish, xo, from, to); break;
             default:  // rows with more than kPre dependencies among them
+                __syncwarp();
+                if (from >= 0) chunk_sync(from);
                 for (int l = 1; l <= steps; ++l) {
                     if (mine == l) {
                         E acc = r.rhs;
@@ -1044,9 +1052,8 @@ k_trsv(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int4* __r
                     }
                     __syncwarp();
                 }
+                if (to >= 0) chunk_arrive(to);
         }
-        __syncwarp();
-        if (c + 1 < nc) chunk_arrive(w);
         r = nx;
         nx = nn;
     }
