@@ -567,18 +567,25 @@ __device__ __forceinline__ void sort_tile(K* key, int m, F get) {
 // diagonal position) and dsrc, where the first four dependencies are found:
 // >= 0 the tile's own position of that row, <= -2 row -(c + 2) of another
 // tile, -1 none.  pos is the inverse (position of each row in its tile),
-// bit k of lmask[q] says that position 32 q + k starts a new level, and
-// lvlptr / nlev hold the level starts.  Levels are global, so rows of the
+// lvlptr / nlev hold the level starts, and chunks the runs of at most 32
+// positions that a warp of the solve takes at a time: chunks[0].x is their
+// number, chunks[1 + c] the positions in chunk c that start a level (bits) and
+// its first position | length << 16.  Chunks end with a level where that takes
+// at most a sixteenth more of them than runs of 32: a level cut in two
+// costs a step of the chain twice.  Levels are global, so rows of the
 // tile never wait on an other-tile row that is late in its own tile merely
 // because of where the tile boundary falls.
 __global__ void __launch_bounds__(kSortThreads)
 k_tri_sort(int32_t n, const int32_t* __restrict__ ci, const int32_t* __restrict__ beg,
            const int32_t* __restrict__ cnt, const int32_t* __restrict__ dpos, const int32_t* __restrict__ glev,
-           int4* __restrict__ desc, int4* __restrict__ dsrc, uint16_t* __restrict__ pos, uint32_t* __restrict__ lmask,
+           int4* __restrict__ desc, int4* __restrict__ dsrc, uint16_t* __restrict__ pos, uint2* __restrict__ chunks,
            int32_t* __restrict__ lvlptr, int32_t* __restrict__ nlev) {
     extern __shared__ __align__(16) unsigned char shraw[];
     unsigned long long* key = reinterpret_cast<unsigned long long*>(shraw);  // kTriTile
     uint16_t* inv = reinterpret_cast<uint16_t*>(key + kTriTile);             // kTriTile
+    uint16_t* lst = inv + kTriTile;                                          // kTriTile + 1: level starts
+    __shared__ uint16_t cut[kTriChunkCap + 1];  // chunk starts
+    __shared__ int ncut;
     __shared__ int first[kTriChunks + 1];  // level starts before each chunk of 32 positions
     __shared__ int s_lo, s_hi;
     const int t = blockIdx.x;
@@ -640,10 +647,7 @@ k_tri_sort(int32_t n, const int32_t* __restrict__ ci, const int32_t* __restrict_
         const int p = 32 * c + lane;
         const bool st = p < m && (p == 0 || (key[p] >> 13) != (key[p - 1] >> 13));
         const uint32_t w = __ballot_sync(0xffffffffu, st);
-        if (lane == 0) {
-            if (c < nc) lmask[size_t(t) * kTriChunks + c] = w;
-            first[c] = __popc(w);
-        }
+        if (lane == 0) first[c] = __popc(w);
     }
     __syncthreads();
     if (threadIdx.x < 32) {  // exclusive scan of the kTriChunks counts, kTriChunks / 32 per lane
@@ -672,13 +676,18 @@ k_tri_sort(int32_t n, const int32_t* __restrict__ ci, const int32_t* __restrict_
     if (threadIdx.x == 0) {
         nlev[t] = first[kTriChunks];
         lp[first[kTriChunks]] = m;
+        lst[first[kTriChunks]] = uint16_t(m);
     }
     for (int c = threadIdx.x >> 5; c < nc; c += blockDim.x >> 5) {
         const int p = 32 * c + lane;
         const bool st = p < m && (p == 0 || (key[p] >> 13) != (key[p - 1] >> 13));
         const uint32_t w = __ballot_sync(0xffffffffu, st);
         if (p >= m) continue;
-        if (st) lp[first[c] + __popc(w & ((1u << lane) - 1u))] = p;
+        if (st) {
+            const int l = first[c] + __popc(w & ((1u << lane) - 1u));
+            lp[l] = p;
+            lst[l] = uint16_t(p);
+        }
         const int32_t row = base + int32_t(key[p] & 8191ull);
         const int32_t b = __ldg(beg + row), d = __ldg(cnt + row);
         desc[base + p] = make_int4(row, b, d, __ldg(dpos + row));
@@ -693,6 +702,30 @@ k_tri_sort(int32_t n, const int32_t* __restrict__ ci, const int32_t* __restrict_
             }
         }
         dsrc[base + p] = make_int4(sc[0], sc[1], sc[2], sc[3]);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int levels = first[kTriChunks], most = min(nc + nc / 16, kTriChunkCap);
+        int k = 0, from = 0;  // the chunk being filled starts at `from`
+        cut[0] = 0;
+        for (int l = 0; l < levels && k < most; ++l) {
+            const int end = lst[l + 1];
+            if (end - from <= 32) continue;
+            if (lst[l] > from) cut[++k] = uint16_t(from = lst[l]);
+            while (end - from > 32 && k < most) cut[++k] = uint16_t(from += 32);
+        }
+        ncut = k < most ? k + 1 : 0;  // 0: runs of 32
+    }
+    __syncthreads();
+    const int nk = ncut ? ncut : nc;
+    chunks += size_t(t) * (kTriChunkCap + 1);
+    if (threadIdx.x == 0) chunks[0] = make_uint2(unsigned(nk), 0u);
+    for (int c = threadIdx.x >> 5; c < nk; c += blockDim.x >> 5) {
+        const int from = ncut ? cut[c] : 32 * c, to = ncut ? (c + 1 < nk ? int(cut[c + 1]) : m) : min(32 * c + 32, m);
+        const int p = from + lane;
+        const bool st = p < to && (p == 0 || (key[p] >> 13) != (key[p - 1] >> 13));
+        const uint32_t w = __ballot_sync(0xffffffffu, st);
+        if (lane == 0) chunks[1 + c] = make_uint2(w, unsigned(from) | unsigned(to - from) << 16);
     }
 }
 
@@ -789,7 +822,7 @@ __global__ void k_tri_fill(int32_t n, E* __restrict__ x, unsigned* ticket) {
 }
 
 // One tile.  What bounds a solve is the chain of levels, so a tile's rows are
-// taken in level order, 32 positions (a chunk) at a time with one row per
+// taken in level order, up to 32 positions (a chunk) at a time with one row per
 // lane: a warp steps through the levels its chunk spans and passes every
 // value to the next level through shared memory with a __syncwarp.  The
 // block's warps take the chunks round-robin and hand the chain on from chunk
@@ -801,12 +834,14 @@ __global__ void k_tri_fill(int32_t n, E* __restrict__ x, unsigned* ticket) {
 // row's FMAs and a shared store (and, at a non-unit diagonal, a division),
 // whatever the number of rows up to 32; wider levels take several chunks.
 // Measured on B200 (f64, ILU(0) factors of the 1024^2 5-point operator, 2047
-// levels in 128 tiles): lower + upper solve 972 us, against
-// 2460 us for levels handed round 15 warps one by one (0.22 us a level
-// in a single tile, here 0.04: 78 cycles, 180 with the division) with a
-// receiver warp for the other tiles' values; 96^3 7-point 330 / 345 against
-// 846 / 821 us.  What is left is the chain itself and, at each of the 127
-// tile boundaries, about 1.5 us for a value to go out to L2 and be polled.
+// levels in 128 tiles): lower + upper solve 902 us, 972 us with chunks of 32
+// that cut levels in two, and 2460 us for levels handed round 15 warps one by
+// one with a receiver warp for the other tiles' values.  One tile of 1024 x 8
+// points, 1031 levels, takes 73 / 134 us and each further one 2.2 / 3.1 us:
+// the eight levels it starts later, a chunk's worth of waiting and a value's
+// way to L2 and back.  (Polling the other tiles' values in the shared memory of
+// a cluster's blocks instead of L2 took 0.3 us off a tile, 998 against 1011 us
+// in all, and was not worth its code.)
 // (A solver warp fed through a shared-memory ring by the others was slower,
 // 480 / 719 us: about 500 cycles a chunk went into taking over the records.)
 // A division by the diagonal sits on the chain, so the loader prepares it:
@@ -892,20 +927,24 @@ struct RowData {
     int4 d;          // row, first dependency entry, dependency count, diagonal entry
     int4 s;          // dependency sources (dsrc)
     uint32_t starts; // the chunk's level starts
+    int first;       // its first position
     E rhs, dg, v[kPre];
 };
 template <class E>
-__device__ __forceinline__ void gather_idx(RowData<E>& r, int c, int nc, int lane, int32_t m, const int4* __restrict__ desc,
-                                           const int4* __restrict__ dsrc, const uint32_t* __restrict__ lmask) {
-    const int32_t p = 32 * c + lane;
+__device__ __forceinline__ void gather_idx(RowData<E>& r, uint2 chunk, int lane, const int4* __restrict__ desc,
+                                           const int4* __restrict__ dsrc) {
+    r.first = int(chunk.y & 0xffffu);
+    r.starts = chunk.x;
     r.d = make_int4(-1, 0, 0, -1);
     r.s = make_int4(-1, -1, -1, -1);
-    r.starts = 0u;
-    if (p < m) {
-        r.d = __ldg(desc + p);
-        r.s = __ldg(dsrc + p);
+    if (lane < int(chunk.y >> 16)) {
+        r.d = __ldg(desc + r.first + lane);
+        r.s = __ldg(dsrc + r.first + lane);
     }
-    if (c < nc) r.starts = __ldg(lmask + c);
+}
+// Chunk c of the tile's nc; no positions past the last.
+__device__ __forceinline__ uint2 chunk_at(const uint2* __restrict__ chunks, int c, int nc) {
+    return c < nc ? __ldg(chunks + 1 + c) : make_uint2(0u, 0u);
 }
 template <class E, bool UNIT>
 __device__ __forceinline__ void gather_val(RowData<E>& r, const E* __restrict__ val, const E* __restrict__ b) {
@@ -955,7 +994,7 @@ __device__ __forceinline__ void solve_steps(const RowData<E>& r, const Prep<E>& 
 template <class E, bool UPPER, bool UNIT>
 __global__ void __launch_bounds__(kSolveThreads, 1)
 k_trsv(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int4* __restrict__ dsrc,
-       const uint32_t* __restrict__ lmask, const uint16_t* __restrict__ pos, const int32_t* __restrict__ ci,
+       const uint2* __restrict__ chunks, const uint16_t* __restrict__ pos, const int32_t* __restrict__ ci,
        const E* __restrict__ val, E alpha, const E* __restrict__ b, E* x, unsigned* ticket, int* err,
        unsigned long long lim, int32_t withhold) {
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -970,21 +1009,23 @@ k_trsv(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int4* __r
     if (t < 0 || t >= ntiles) return;
     const int32_t base = int32_t(t) * kTriTile;
     const int32_t m = min(kTriTile, n - base);
-    const int nc = (m + 31) >> 5;
+    chunks += size_t(t) * (kTriChunkCap + 1);
+    const int nc = int(__ldg(&chunks->x));
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     desc += base;
     dsrc += base;
-    lmask += size_t(t) * kTriChunks;
 
     RowData<E> r{}, nx{};
-    gather_idx(r, w, nc, lane, m, desc, dsrc, lmask);
-    gather_idx(nx, w + kSolveWarps, nc, lane, m, desc, dsrc, lmask);
+    gather_idx(r, chunk_at(chunks, w, nc), lane, desc, dsrc);
+    gather_idx(nx, chunk_at(chunks, w + kSolveWarps, nc), lane, desc, dsrc);
+    uint2 ahead = chunk_at(chunks, w + 2 * kSolveWarps, nc);
     gather_val<E, UNIT>(r, val, b);
     for (int c = w; c < nc; c += kSolveWarps) {
         // in flight meanwhile: the next chunk's values, the descriptors of the one after it
         RowData<E> nn{};
         gather_val<E, UNIT>(nx, val, b);
-        gather_idx(nn, c + 2 * kSolveWarps, nc, lane, m, desc, dsrc, lmask);
+        gather_idx(nn, ahead, lane, desc, dsrc);
+        ahead = chunk_at(chunks, c + 3 * kSolveWarps, nc);
         // sources in shared memory: the tile's own positions, or (another
         // tile's value; a zero where there is no dependency) the warp's own places
         const E* src[kPre];
@@ -1004,7 +1045,7 @@ k_trsv(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int4* __r
         const int mine = r.d.x >= 0 ? __popc(starts & ((2u << lane) - 1u)) : 0;  // this lane's level within the chunk
         const int most = __reduce_max_sync(0xffffffffu, r.d.z);
         const bool publish = r.d.x != withhold;
-        E* const out = T.xs + 32 * c + lane;
+        E* const out = T.xs + r.first + lane;
         E* const xo = x + (r.d.x >= 0 ? r.d.x : 0);
         // the other tiles' values, last: nothing but the turn comes after their arrival
         if (pend != 0u) {
@@ -1166,13 +1207,14 @@ template <class E>
 struct PivotRow {
     int4 d, s, w;
     uint32_t starts;
+    int first;
     E diag, v[kPre], u[kPre];  // a_ii, a_ik, a_ki
 };
 
 template <class E>
 __global__ void __launch_bounds__(kSolveThreads, 1)
 k_ilu0_diag(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int4* __restrict__ dsrc,
-            const uint32_t* __restrict__ lmask, const int4* __restrict__ wpos, E* val, E* piv, unsigned* ticket,
+            const uint2* __restrict__ chunks, const int4* __restrict__ wpos, E* val, E* piv, unsigned* ticket,
             const int* __restrict__ general, int* err, int* err_row) {
     if (*general) return;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -1183,26 +1225,25 @@ k_ilu0_diag(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int4
     const int t = s_tile;
     if (t >= ntiles) return;
     const int32_t base = int32_t(t) * kTriTile;
-    const int32_t m = min(kTriTile, n - base);
-    const int nc = (m + 31) >> 5;
+    chunks += size_t(t) * (kTriChunkCap + 1);
+    const int nc = int(__ldg(&chunks->x));
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     desc += base;
     dsrc += base;
     wpos += base;
-    lmask += size_t(t) * kTriChunks;
 
-    auto idx = [&](PivotRow<E>& r, int c) {
-        const int32_t p = 32 * c + lane;
+    auto idx = [&](PivotRow<E>& r, uint2 chunk) {
+        const int32_t p = int32_t(chunk.y & 0xffffu) + lane;
+        r.first = p - lane;
         r.d = make_int4(-1, 0, 0, -1);
         r.s = make_int4(-1, -1, -1, -1);
         r.w = r.s;
-        r.starts = 0u;
-        if (p < m) {
+        r.starts = chunk.x;
+        if (lane < int(chunk.y >> 16)) {
             r.d = __ldg(desc + p);
             r.s = __ldg(dsrc + p);
             r.w = __ldg(wpos + p);
         }
-        if (c < nc) r.starts = __ldg(lmask + c);
     };
     // (the entries read here are written by their own row's lane alone, later)
     auto values = [&](PivotRow<E>& r) {
@@ -1216,15 +1257,17 @@ k_ilu0_diag(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int4
             }
     };
     PivotRow<E> r{}, nx{};
-    idx(r, w);
-    idx(nx, w + kSolveWarps);
+    idx(r, chunk_at(chunks, w, nc));
+    idx(nx, chunk_at(chunks, w + kSolveWarps, nc));
+    uint2 ahead = chunk_at(chunks, w + 2 * kSolveWarps, nc);
     values(r);
     for (int c = w; c < nc; c += kSolveWarps) {
         // in flight meanwhile (complex<double> rows fill the registers as they are: its next values come after the turn)
         constexpr bool kAhead = sizeof(E) < 16;
         PivotRow<E> nn{};
         if (kAhead) values(nx);
-        idx(nn, c + 2 * kSolveWarps);
+        idx(nn, ahead);
+        ahead = chunk_at(chunks, c + 3 * kSolveWarps, nc);
         const E* src[kPre];
         unsigned pend = 0;
 #pragma unroll
@@ -1276,7 +1319,7 @@ k_ilu0_diag(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int4
                     acc = (k < r.d.z && at4(r.w, k) >= 0) ? f : acc;
                 }
             if (on) {
-                T.xs[32 * c + lane] = acc;
+                T.xs[r.first + lane] = acc;
                 piv_i = acc;
 #pragma unroll
                 for (int k = 0; k < kPre; ++k) l[k] = q[k];
@@ -1424,7 +1467,7 @@ int analyse(hpb_context* ctx, int upper, int32_t n, int64_t nnz, const int32_t* 
     };
     const size_t nn = size_t(n), nt = size_t(P->ntiles);
     const size_t o_desc = part(keep, nn * sizeof(int4)), o_dsrc = part(keep, nn * sizeof(int4));
-    const size_t o_pos = part(keep, nn * sizeof(uint16_t)), o_lmask = part(keep, nt * kTriChunks * sizeof(uint32_t));
+    const size_t o_pos = part(keep, nn * sizeof(uint16_t)), o_chunks = part(keep, nt * (kTriChunkCap + 1) * sizeof(uint2));
     const size_t o_lvl = part(keep, nt * (kTriTile + 1) * sizeof(int32_t)), o_dpos = part(keep, nn * sizeof(int32_t));
     const size_t o_flags = part(keep, (nn + 1) * sizeof(unsigned));
     const size_t o_err = part(keep, (4 + nt) * sizeof(int));  // err, err_row, rows without a diagonal, -, nlev
@@ -1444,7 +1487,7 @@ int analyse(hpb_context* ctx, int upper, int32_t n, int64_t nnz, const int32_t* 
     P->desc = reinterpret_cast<int4*>(blk + o_desc);
     P->dsrc = reinterpret_cast<int4*>(blk + o_dsrc);
     P->pos = reinterpret_cast<uint16_t*>(blk + o_pos);
-    P->lmask = reinterpret_cast<uint32_t*>(blk + o_lmask);
+    P->chunks = reinterpret_cast<uint2*>(blk + o_chunks);
     P->lvlptr = reinterpret_cast<int32_t*>(blk + o_lvl);
     P->dpos = reinterpret_cast<int32_t*>(blk + o_dpos);
     P->flags = reinterpret_cast<unsigned*>(blk + o_flags);
@@ -1464,10 +1507,10 @@ int analyse(hpb_context* ctx, int upper, int32_t n, int64_t nnz, const int32_t* 
     auto levels = P->upper ? k_tri_levels<true> : k_tri_levels<false>;
     allow_smem(levels, sizeof(LevelTile));
     levels<<<P->ntiles, kGlThreads, sizeof(LevelTile), s>>>(n, P->ntiles, ci, beg, cnt, glev, ticket, P->err);
-    const size_t sort_smem = size_t(kTriTile) * (sizeof(unsigned long long) + sizeof(uint16_t));
+    const size_t sort_smem = size_t(kTriTile) * (sizeof(unsigned long long) + 2 * sizeof(uint16_t)) + 16;
     allow_smem(k_tri_sort, sort_smem);
     k_tri_sort<<<P->ntiles, kSortThreads, sort_smem, s>>>(n, ci, beg, cnt, P->dpos, glev, P->desc, P->dsrc, P->pos,
-                                                          P->lmask, P->lvlptr, P->nlev);
+                                                          P->chunks, P->lvlptr, P->nlev);
     count_launch(3);
     if (cudaGetLastError() != cudaSuccess) return fail(HPB_ERROR_CUDA, "analysis launch failed");
     std::vector<int32_t> got(4 + nt);  // err, err_row, missing, -, nlev
@@ -1500,7 +1543,7 @@ void release(Plan* P) {
     P->block = P->scratch = nullptr;
     P->desc = P->dsrc = nullptr;
     P->pos = nullptr;
-    P->lmask = nullptr;
+    P->chunks = nullptr;
     P->lvlptr = P->nlev = P->dpos = nullptr;
     P->flags = nullptr;
     P->err = P->err_row = nullptr;
@@ -1528,7 +1571,7 @@ cudaError_t launch_trsv(const Plan& P, int unit, const E* val, E alpha, const E*
     }
     auto k = P.upper ? (unit ? k_trsv<E, true, true> : k_trsv<E, true, false>)
                      : (unit ? k_trsv<E, false, true> : k_trsv<E, false, false>);
-    k<<<P.ntiles, kSolveThreads, sm, s>>>(P.n, P.ntiles, P.desc, P.dsrc, P.lmask, P.pos, P.ci, val, alpha, b, x,
+    k<<<P.ntiles, kSolveThreads, sm, s>>>(P.n, P.ntiles, P.desc, P.dsrc, P.chunks, P.pos, P.ci, val, alpha, b, x,
                                         P.flags + P.n, P.err, P.wait_ns ? P.wait_ns : kWaitNs, P.withhold_row);
     count_launch(2);
     return cudaGetLastError();
@@ -1576,7 +1619,7 @@ cudaError_t launch_ilu0(const Plan& P, E* val, cudaStream_t s) {
         k_tri_fill<E><<<int(std::min<int64_t>((int64_t(P.n) + 255) / 256, 148 * 8)), 256, 0, s>>>(P.n, piv, ticket);
         allow_smem(k_ilu0_diag<E>, sizeof(TileValues<E>));
         k_ilu0_diag<E><<<P.ntiles, kSolveThreads, sizeof(TileValues<E>), s>>>(
-            P.n, P.ntiles, P.desc, P.dsrc, P.lmask, wpos, val, piv, ticket, general, P.err, P.err_row);
+            P.n, P.ntiles, P.desc, P.dsrc, P.chunks, wpos, val, piv, ticket, general, P.err, P.err_row);
         k_ilu0<E><<<P.ntiles, kTriThreads, 0, s>>>(P.n, P.ntiles, P.desc, P.lvlptr, P.nlev, P.rp, P.ci, P.dpos, val,
                                                    P.flags, general, P.err, P.err_row);
         count_launch(4);

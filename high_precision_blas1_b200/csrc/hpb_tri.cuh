@@ -27,7 +27,8 @@ namespace tri {
 
 constexpr int kTriTile = 8192;      // rows per tile
 constexpr int kTriThreads = 512;    // threads per factorization block (16 warps)
-constexpr int kTriChunks = kTriTile / 32;  // chunks of 32 positions of a tile
+constexpr int kTriChunks = kTriTile / 32;  // runs of 32 positions of a tile
+constexpr int kTriChunkCap = kTriChunks + kTriChunks / 16;  // chunks of a tile at most
 
 // Error bits of Plan::err (device).
 constexpr int kErrUnsorted = 1;     // column indices of a row not strictly increasing
@@ -50,7 +51,7 @@ struct Plan {
     int4* desc = nullptr;           // n: (row, first dependency, dependency count, diagonal position) in level order
     int4* dsrc = nullptr;           // n: where each of the first four dependencies is found, in level order
     uint16_t* pos = nullptr;        // n: position of each row in its tile's level order
-    uint32_t* lmask = nullptr;      // ntiles * kTriChunks: positions of a chunk that start a level
+    uint2* chunks = nullptr;        // ntiles * (kTriChunkCap + 1): the tile's number of chunks, then the chunks (k_tri_sort)
     int32_t* lvlptr = nullptr;      // ntiles * (kTriTile + 1): level starts within the tile
     int32_t* nlev = nullptr;        // ntiles
     int32_t* dpos = nullptr;        // n: position of the diagonal entry of each row, -1 if absent
