@@ -62,8 +62,19 @@ __device__ __forceinline__ void pdl_enter_for(T&... p) {
     ([&] { asm volatile("" : "+l"(p)::"memory"); }(), ...);
 }
 
+// Is the stream's work being captured into a graph?
+inline bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return st != cudaStreamCaptureStatusNone;
+}
+
+// pdl false: an ordinary launch
 template <class... KArgs, class... Args>
-inline cudaError_t launch_pdl(cudaStream_t s, int grid, int block, void (*kernel)(KArgs...), Args&&... args) {
+inline cudaError_t launch_pdl_if(bool pdl, cudaStream_t s, int grid, int block, void (*kernel)(KArgs...), Args&&... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(unsigned(grid));
     cfg.blockDim = dim3(unsigned(block));
@@ -73,8 +84,12 @@ inline cudaError_t launch_pdl(cudaStream_t s, int grid, int block, void (*kernel
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+template <class... KArgs, class... Args>
+inline cudaError_t launch_pdl(cudaStream_t s, int grid, int block, void (*kernel)(KArgs...), Args&&... args) {
+    return launch_pdl_if(true, s, grid, block, kernel, std::forward<Args>(args)...);
 }
 
 extern std::atomic<uint64_t> g_launches;

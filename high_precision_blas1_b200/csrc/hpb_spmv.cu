@@ -202,7 +202,9 @@ int spmv_dot2_impl(hpb_context* ctx, int32_t rows, int32_t cols, int64_t nnz, co
     // ticket[1] serves as the (unused) non-finite flag and stays zero.
     dispatch_lm<E>(load_mode<E>(val, x, nnz), [&](auto mode) {
         constexpr int M = decltype(mode)::value;
-        launch_pdl(ctx->stream, grid, kSpmvRows, csr_row_dot_kernel<E, M>, rows, rp, ci, val, x, y, w,
+        // (captured: without the programmatic edge, 17.7 against 18.2 us at 1024^2 f64 on B200;
+        // in a row of calls on a stream with it, 18.7 against 19.8 us)
+        launch_pdl_if(!capturing(ctx->stream), ctx->stream, grid, kSpmvRows, csr_row_dot_kernel<E, M>, rows, rp, ci, val, x, y, w,
                    static_cast<A*>(ctx->partials), ctx->ticket, reinterpret_cast<int*>(ctx->ticket + 1), out);
     });
     count_launch();
