@@ -834,8 +834,8 @@ __global__ void k_tri_fill(int32_t n, E* __restrict__ x, unsigned* ticket) {
 // row's FMAs and a shared store (and, at a non-unit diagonal, a division),
 // whatever the number of rows up to 32; wider levels take several chunks.
 // Measured on B200 (f64, ILU(0) factors of the 1024^2 5-point operator, 2047
-// levels in 128 tiles): lower + upper solve 902 us, 972 us with chunks of 32
-// that cut levels in two, and 2460 us for levels handed round 15 warps one by
+// levels in 128 tiles): lower + upper solve 902 us with fifteen warps,
+// 972 us with chunks of 32 that cut levels in two, and 2460 us for levels handed round 15 warps one by
 // one with a receiver warp for the other tiles' values.  One tile of 1024 x 8
 // points, 1031 levels, takes 73 / 134 us and each further one 2.2 / 3.1 us:
 // the eight levels it starts later, a chunk's worth of waiting and a value's
@@ -903,7 +903,13 @@ __device__ __forceinline__ cd quot_prepared(cd a, cd d, const Prep<cd>& p, bool 
     return q;
 }
 
-constexpr int kSolveWarps = 15;  // one named barrier (1..15) behind each warp
+// One named barrier (1..15) behind each warp.  Seven warps are far enough ahead
+// of the chain with their loads and poll L2 half as much as fifteen (lower /
+// upper solve, ILU(0) on B200, fifteen -> seven: f64 1024^2 370 / 545, 1296 ->
+// 334 / 511, 1228 us; f64 96^3 356 / 349, 814 -> 312 / 340, 772; c128 700^2
+// 309 / 560, 2957 -> 275 / 469, 2344; c64 300 x 1000 234 / 408, 1603 -> 254 /
+// 387, 1565); eleven 346 / 538 in the first, and five 338 / 373 in the second.
+constexpr int kSolveWarps = 7;
 constexpr int kSolveThreads = 32 * kSolveWarps;
 
 template <class E>
