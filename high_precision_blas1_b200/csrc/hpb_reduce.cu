@@ -324,16 +324,16 @@ reduce_kernel(int64_t n, const E* __restrict__ x, const E* __restrict__ y, void*
     constexpr bool COMP = op_is_comp(OP);
     constexpr int K = VEC ? VecOf<E>::k : 1;
     unsigned int* const ticket = sync;
-    pdl_enter();  // inputs and the ticket are read only after the previous kernel on the stream completed
 
     Acc s{}, c{};
-    const int64_t gtid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    int64_t gtid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    pdl_enter_for(gtid);
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     const int64_t nv = n / K;  // full vectors
 
     if constexpr (TAIL == TAIL_ONE) {
         // at most kRedUnroll packs (elements) a thread, all loaded at once
-        const int items = int(VEC ? nv : n), bd = int(blockDim.x), t = int(threadIdx.x);
+        const int items = int(VEC ? nv : n), bd = int(blockDim.x), t = int(gtid);
         const int64_t i = nv * K + t;
         const bool ragged = VEC && i < n;
         E ex{}, ey{};
