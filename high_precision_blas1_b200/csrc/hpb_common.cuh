@@ -40,25 +40,42 @@ namespace hpb {
 // Library kernels are launched with programmatic stream serialisation
 // (launch_pdl): a kernel may be scheduled while its predecessor on the
 // stream drains, hiding the launch gap between back-to-back kernels.  Each
-// such kernel calls pdl_enter_for() first: it waits until the predecessor
+// such kernel calls pdl_wait_for() first: it waits until the predecessor
 // grid has completed and its memory is visible
-// (griddepcontrol.wait) -- so nothing is read early -- and then lets its own
-// successor be scheduled (griddepcontrol.launch_dependents).  Launched
-// normally, the wait returns at once.
+// (griddepcontrol.wait) -- so nothing is read early.  pdl_trigger() lets its own
+// successor be scheduled (griddepcontrol.launch_dependents), once every block
+// has called it or ended; pdl_enter_for() does both.  Launched normally, the
+// wait returns at once.
 // The kernels read through the read-only path (__ldg, const __restrict__), and
 // such a load, which the compiler may take to be invariant, could otherwise
 // move ahead of the wait: what every address is formed from -- the thread's
 // index, or the pointers -- is made to depend on it.  (Tied pointers lose their
 // __restrict__, which costs some kernels loads in flight: sum2 of 1 M c128
 // 7.7 us with the index tied, 10.3 with the pointers.)
+template <class T>
+__device__ __forceinline__ void tie(T& v) {
+    static_assert(sizeof(T) == 8 || sizeof(T) == 4, "a pointer or an index");
+    if constexpr (sizeof(T) == 8)
+        asm volatile("" : "+l"(v)::"memory");
+    else
+        asm volatile("" : "+r"(v)::"memory");
+}
 template <class... T>
-__device__ __forceinline__ void pdl_enter_for(T&... a) {
+__device__ __forceinline__ void pdl_wait_for(T&... a) {
 #if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
     cudaGridDependencySynchronize();
+#endif
+    (tie(a), ...);
+}
+__device__ __forceinline__ void pdl_trigger() {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
     cudaTriggerProgrammaticLaunchCompletion();
 #endif
-    static_assert(((sizeof(T) == 8) && ...), "pointers or 64-bit indices");
-    ([&] { asm volatile("" : "+l"(a)::"memory"); }(), ...);
+}
+template <class... T>
+__device__ __forceinline__ void pdl_enter_for(T&... a) {
+    pdl_wait_for(a...);
+    pdl_trigger();
 }
 
 // Is the stream's work being captured into a graph?

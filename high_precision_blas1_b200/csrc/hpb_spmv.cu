@@ -67,32 +67,54 @@ __device__ __forceinline__ E row_sum(int32_t b, int32_t e, const int32_t* __rest
     return acc;
 }
 
+// How a product takes its rows, by the matrix' mean row length.  Each row's sum
+// is in index order whichever it is, so the result does not depend on it.
+//   ROWS_SHORT  up to three entries (and matrices well above L2 of more than
+//               kRowBatch): one entry at a time, as many blocks as are resident
+//   ROWS_BATCH  up to eight: batches, twice the resident blocks
+//   ROWS_LONG   more: batches, the index tied to the wait for the call before
+//               (pdl_wait_for) instead of the pointers, which leaves the
+//               compiler the next batch's loads ahead of this one's sums
+// The call behind is let in when a block has done its rows, so that its blocks
+// do not take L1 and issue slots from rows at work; only batches of complex
+// entries are faster with it let in first.
+// Measured on B200, in rows of calls, against one entry at a time in an
+// ordinary launch, alpha A x (5 pt: 1024^2, 7 pt: 100^3, 9 pt: 700^2, 27 pt:
+// 64^3; rand k: k entries at random columns, 200,000 rows, k < 3: 1 M rows), us:
+//            rand 1        5 pt         7 pt         9 pt         27 pt        rand 20
+//   f64    9.1 ->  7.3  14.6 -> 12.0  20.8 -> 18.0  14.5 -> 11.1  37.1 -> 25.9  39.1 -> 31.2
+//   f32    8.4 ->  6.9  10.6 ->  6.9  14.6 -> 10.6  10.4 ->  6.2  26.9 -> 17.6  30.9 -> 25.4
+//   c64   10.3 ->  7.8  14.6 -> 12.1  21.2 -> 17.1  15.1 -> 10.5  38.1 -> 26.0  37.1 -> 33.1
+//   c128  11.8 -> 10.2  27.6 -> 21.8  43.1 -> 32.5  30.2 -> 24.0  57.6 -> 41.9  45.4 -> 37.2
+// Batches with tied pointers took 38 us (f32) and 54 us (c128) for rand 20 and
+// 61 us for 27 pt in c64 with beta; one entry at a time takes 35 us for 27 pt in
+// f64; batches take 8.2 us for rand 1 in f64, and 20.5 us instead of 16.2 for a
+// tridiagonal c64 matrix with beta.  (Among other matrices, so that none of it is in L2:
+// 5 pt f64 17.7 -> 14.1 us.)  Batches of 4, 6 and 8 gave 17.3, 17.8 and 15.7 us
+// there (more registers, fewer warps); 8 blocks per SM 15.1, one row a thread 14.4.
+enum Rows { ROWS_SHORT = 0, ROWS_BATCH, ROWS_LONG };
+
 // LM: the load mode of the matrix and x (ld_val, ld_x)
-//
-// Rows in a grid-stride loop over kSpmvPerSm blocks per SM; each row's sum in
-// index order, so the result does not depend on the launch shape or on BATCH.
-// Bound by HBM once the loads are in flight.  B200, against the loop of one
-// entry at a time over 8 blocks per SM (five-point operators on 1024^2 and
-// 2048^2 rows, seven-point ones on 128^3 and 100^3, alpha A x):
-//   f64  1024^2  14.5 -> 12.1 us      f32  2048^2  35.1 -> 32.9 us
-//   c128 1024^2  28.8 -> 21.7 us      c64  2048^2  56.8 -> 55.8 us
-//   f64  128^3   41.2 -> 33.8 us      f32  128^3   24.7 -> 24.1 us
-//   c64  100^3   20.7 -> 16.8 us      c128 100^3   43.2 -> 32.1 us
-// (among other matrices, so that none of it is in L2: f64 1024^2 17.7 ->
-// 14.1 us).  Batches of 4, 6 and 8 gave 17.3, 17.8 and 15.7 us there (more
-// registers, fewer warps); 8 blocks per SM 15.1, one row a thread 14.4.
-template <class E, bool BETA0, int LM, bool BATCH>
+template <class E, bool BETA0, int LM, int FORM>
 __global__ void __launch_bounds__(kSpmvRows)
 csr_row_kernel(int32_t rows, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
                const E* __restrict__ val, E alpha, const E* __restrict__ x, E beta, E* __restrict__ y) {
-    pdl_enter_for(rp, ci, val, x, y);
+    constexpr bool kEarly = FORM == ROWS_BATCH && is_cplx<E>::value;
+    constexpr bool kTieIndex = FORM == ROWS_LONG || (FORM == ROWS_BATCH && std::is_same<E, cf>::value && !BETA0);
     const uint32_t stride = gridDim.x * kSpmvRows;
-    for (uint32_t r = blockIdx.x * kSpmvRows + threadIdx.x; r < uint32_t(rows); r += stride) {
+    uint32_t r = blockIdx.x * kSpmvRows + threadIdx.x;
+    if constexpr (kTieIndex)
+        pdl_wait_for(r);
+    else
+        pdl_wait_for(rp, ci, val, x, y);
+    if (kEarly) pdl_trigger();
+    for (; r < uint32_t(rows); r += stride) {
         const int32_t b = __ldg(rp + r), e = __ldg(rp + r + 1);
-        const E acc = row_sum<E, LM, BATCH>(b, e, ci, val, x);
+        const E acc = row_sum<E, LM, FORM != ROWS_SHORT>(b, e, ci, val, x);
         E out = BETA0 ? mul_s(alpha, acc) : madd_s(alpha, acc, mul_s(beta, ldE(y, r)));
         stE(y, r, out);
     }
+    if (!kEarly) pdl_trigger();
 }
 
 __device__ __forceinline__ void write_hi_lo(const fused::Acc2& a, double* out) {
@@ -154,21 +176,26 @@ int spmv_impl(hpb_context* ctx, int32_t rows, int32_t cols, int64_t nnz, const i
         (reinterpret_cast<uintptr_t>(rp) | reinterpret_cast<uintptr_t>(ci)) % 4)
         return set_error(ctx, HPB_ERROR_INVALID_VALUE, "%s: pointer not aligned to its element type", name);
     const int lm = load_mode<E>(val, x, nnz);
-    // Matrices well above L2 with more than a batch of entries a row keep the
-    // plain loop: it measured 97 us on the seven-point operator of 180^3 rows in
-    // binary64 (B200), the batches 104 us.
-    const bool batch = !(lm & LM_CACHED) || nnz <= int64_t(rows) * kRowBatch;
-    const int grid = grid_for(ctx, rows, kSpmvRows, batch ? kSpmvPerSm : kSpmvPerSm / 2);
+    // the form (enum Rows).  Matrices well above L2 with more than a batch of
+    // entries a row: one entry at a time measured 97 us on the seven-point
+    // operator of 180^3 rows in binary64 (B200), the batches 104 us.
+    const int64_t n = rows;
+    const int form = nnz <= 3 * n || ((lm & LM_CACHED) && nnz > n * kRowBatch) ? ROWS_SHORT
+                     : nnz <= 8 * n                                           ? ROWS_BATCH
+                                                                              : ROWS_LONG;
+    const int grid = grid_for(ctx, rows, kSpmvRows, form == ROWS_SHORT ? kSpmvPerSm / 2 : kSpmvPerSm);
     dispatch_lm<E>(lm, [&](auto mode) {
         constexpr int M = decltype(mode)::value;
         auto go = [&](auto kernel) {
             launch_pdl(ctx->stream, grid, kSpmvRows, kernel, rows, rp, ci, val, alpha, x, beta, y);
         };
         const bool b0 = is_zero(beta);
-        if (batch)
-            b0 ? go(csr_row_kernel<E, true, M, true>) : go(csr_row_kernel<E, false, M, true>);
-        else if constexpr ((M & LM_CACHED) != 0)
-            b0 ? go(csr_row_kernel<E, true, M, false>) : go(csr_row_kernel<E, false, M, false>);
+        if (form == ROWS_SHORT)
+            b0 ? go(csr_row_kernel<E, true, M, ROWS_SHORT>) : go(csr_row_kernel<E, false, M, ROWS_SHORT>);
+        else if (form == ROWS_BATCH)
+            b0 ? go(csr_row_kernel<E, true, M, ROWS_BATCH>) : go(csr_row_kernel<E, false, M, ROWS_BATCH>);
+        else if constexpr ((M & LM_CACHED) == 0)
+            b0 ? go(csr_row_kernel<E, true, M, ROWS_LONG>) : go(csr_row_kernel<E, false, M, ROWS_LONG>);
     });
     count_launch();
     return check_launch(ctx, name);
