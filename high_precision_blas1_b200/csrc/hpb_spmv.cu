@@ -145,15 +145,20 @@ csr_row_dot_kernel(int32_t rows, const int32_t* __restrict__ rp, const int32_t* 
                    int* badflag, double* out) {
     using S = typename fused::scalar_of<E>::type;
     using A = typename fused::acc_of<S>::type;
-    pdl_enter_for(rp, ci, val, x, y, w, partials, ticket, out);
+    uint32_t r = blockIdx.x * kSpmvRows + threadIdx.x;
+    pdl_wait_for(r);
     A d[1];
-    const int32_t stride = gridDim.x * kSpmvRows;
-    for (int32_t r = blockIdx.x * kSpmvRows + threadIdx.x; r < rows; r += stride) {
+    const uint32_t stride = gridDim.x * kSpmvRows;
+    for (; r < uint32_t(rows); r += stride) {
         const int32_t b = __ldg(rp + r), e = __ldg(rp + r + 1);
+        E we;
+        if (!is_cplx<E>::value) we = ldE(w, r);  // in flight with the row's entries
         const E acc = row_sum<E, LM, false>(b, e, ci, val, x);  // (batches: 21.3 us against 18.5 at 1024^2)
+        if (is_cplx<E>::value) we = ldE(w, r);
         stE(y, r, acc);
-        fused::dot_add(d[0], fused::to_s(ldE(w, r)), fused::to_s(acc));
+        fused::dot_add(d[0], fused::to_s(we), fused::to_s(acc));
     }
+    pdl_trigger();
     fused::grid_finish_acc<1>(d, false, partials, ticket, badflag, [&](const A* tot, bool) { write_hi_lo(tot[0], out); });
 }
 
@@ -225,14 +230,18 @@ int spmv_dot2_impl(hpb_context* ctx, int32_t rows, int32_t cols, int64_t nnz, co
     if (grid > ctx->num_sms * 6) grid = ctx->num_sms * 6;
     if (grid > ctx->max_blocks) grid = ctx->max_blocks;
     if (grid < 1) grid = 1;
+    // The call behind is let in when a block has done its rows.  Not where the
+    // call is captured (17.5 us without a programmatic edge, 18.2 with it, 1024^2
+    // f64 on B200), and not for rows so long that a few blocks are still at work
+    // while it takes the idle SMs unevenly (40 entries a row, 100,000 rows, f64:
+    // 46.9 us let in late, 43.2 in an ordinary launch).
+    const bool early = !capturing(ctx->stream) && nnz <= 32 * int64_t(rows);
     // ticket[0]: the reductions' counter (same stream, so never concurrent);
     // ticket[1] serves as the (unused) non-finite flag and stays zero.
     dispatch_lm<E>(load_mode<E>(val, x, nnz), [&](auto mode) {
         constexpr int M = decltype(mode)::value;
-        // (captured: without the programmatic edge, 17.7 against 18.2 us at 1024^2 f64 on B200;
-        // in a row of calls on a stream with it, 18.7 against 19.8 us)
-        launch_pdl_if(!capturing(ctx->stream), ctx->stream, grid, kSpmvRows, csr_row_dot_kernel<E, M>, rows, rp, ci, val, x, y, w,
-                   static_cast<A*>(ctx->partials), ctx->ticket, reinterpret_cast<int*>(ctx->ticket + 1), out);
+        launch_pdl_if(early, ctx->stream, grid, kSpmvRows, csr_row_dot_kernel<E, M>, rows, rp, ci, val, x, y, w,
+                      static_cast<A*>(ctx->partials), ctx->ticket, reinterpret_cast<int*>(ctx->ticket + 1), out);
     });
     count_launch();
     return check_launch(ctx, name);
