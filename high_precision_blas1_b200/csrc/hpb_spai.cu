@@ -983,13 +983,13 @@ struct hpb_spai {
     double* lpart = nullptr;
     int part_blocks = 0;
     void* wimg = nullptr;        // the tcgen05 forward's weight image (rebuilt when wb changes)
-    int* tc_err = nullptr;       // mapped pinned: [0] a tensor-core wait ran out of time, [1] copy of *irregular
+    int* tc_err = nullptr;       // mapped pinned word: a tensor-core wait ran out of time
     int* tc_err_dev = nullptr;   // its device address
     // slot form: the pairs of slots behind each entry of A^2, and the training workspace
     hpb::spai::PairTable pairs{};
     size_t slot_rows = 0;
     char* slot_mem = nullptr;
-    unsigned* slot_sync = nullptr;  // ticket, bad flag, *irregular (each a line apart), behind part
+    unsigned* slot_sync = nullptr;  // k_slot_load's ticket and bad flag (a line apart), behind part
     double* slot_out = nullptr;     // out[4] of k_slot_close, then this system's gradient, behind that
     double* slot_host = nullptr;    // pinned copy (from the first training system on)
 };
@@ -1036,6 +1036,7 @@ struct SlotArrays {
     uint8_t* mask;
     double *sd, *ld, *sums, *lpart;
     hpb::fused::Acc2* partials;
+    int* irregular;  // the call's own: threads may build with one network at the same time
     size_t bytes;
 };
 SlotArrays slot_arrays(char* base, size_t n, const hpb::spai::Offsets& o, bool train) {
@@ -1053,6 +1054,7 @@ SlotArrays slot_arrays(char* base, size_t n, const hpb::spai::Offsets& o, bool t
     a.th = floats(kO);
     a.mask = reinterpret_cast<uint8_t*>(take(n));
     a.sums = reinterpret_cast<double*>(take((1 + kMaxRes) * sizeof(double)));
+    a.irregular = reinterpret_cast<int*>(take(sizeof(int)));
     a.partials = reinterpret_cast<hpb::fused::Acc2*>(take((1 + kMaxRes) * nb * sizeof(hpb::fused::Acc2)));
     if (!train) {
         a.sd = reinterpret_cast<double*>(take(n * sizeof(double)));
@@ -1086,8 +1088,7 @@ void launch_slot_load(hpb_spai* net, const hpb_spai_system& sys, int nres, const
         constexpr int NR = decltype(k)::value;
         k_slot_load<NR><<<nb, kSlotThreads>>>(sys.rows, sys.row_ptr, sys.col_ind, sys.val, net->off, sys.residuals, a.raw,
                                               a.mask, a.diag, a.sd, a.ld, a.rh, a.sums, a.partials, net->slot_sync,
-                                              reinterpret_cast<int*>(net->slot_sync + 32),
-                                              reinterpret_cast<int*>(net->slot_sync + 64));
+                                              reinterpret_cast<int*>(net->slot_sync + 32), a.irregular);
     };
     switch (nres) {
         case 1: go(std::integral_constant<int, 1>{}); break;
@@ -1270,7 +1271,7 @@ int hpb_spai_create(hpb_spai** out, int nslot, int dslot, const int* offsets, ui
         w[Params::B1 + i] = 0.01f;
         w[Params::B2 + i] = 0.01f;
     }
-    if (cudaHostAlloc(&net->tc_err, 2 * sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+    if (cudaHostAlloc(&net->tc_err, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
         net->tc_err = nullptr;
         hpb_spai_destroy(net);
         return HPB_ERROR_OUT_OF_MEMORY;
@@ -1283,17 +1284,17 @@ int hpb_spai_create(hpb_spai** out, int nslot, int dslot, const int* offsets, ui
     if (cudaMalloc(&net->w, kNumParams * 4) || cudaMalloc(&net->wb, kNumParams * 2) ||
         cudaMalloc(&net->m1, kNumParams * 4) || cudaMalloc(&net->m2, kNumParams * 4) ||
         cudaMalloc(&net->grad, kNumParams * 4) || cudaMalloc(&net->gtmp, kNumParams * 4) ||
-        cudaMalloc(&net->part, kPartBytes + 96 * sizeof(unsigned) + kSlotOutBytes) ||
+        cudaMalloc(&net->part, kPartBytes + 64 * sizeof(unsigned) + kSlotOutBytes) ||
         cudaMalloc(&net->wimg, kTcImageBytes)) {
         hpb_spai_destroy(net);
         return HPB_ERROR_OUT_OF_MEMORY;
     }
     net->slot_sync = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(net->part) + kPartBytes);
-    net->slot_out = reinterpret_cast<double*>(net->slot_sync + 96);
+    net->slot_out = reinterpret_cast<double*>(net->slot_sync + 64);
     cudaMemset(net->m1, 0, kNumParams * 4);
     cudaMemset(net->m2, 0, kNumParams * 4);
     cudaMemset(net->grad, 0, kNumParams * 4);
-    cudaMemset(net->slot_sync, 0, 96 * sizeof(unsigned));
+    cudaMemset(net->slot_sync, 0, 64 * sizeof(unsigned));
     int st = hpb_spai_set_weights(net, w.data());
     if (st) {
         hpb_spai_destroy(net);
@@ -1358,19 +1359,19 @@ int hpb_spai_assemble(hpb_spai* net, const hpb_spai_system* sys, float* m_val) {
         if (!mem) return HPB_ERROR_OUT_OF_MEMORY;
         const SlotArrays a = slot_arrays(mem, size_t(n), net->off, false);
         launch_slot_load(net, *sys, -1, a);
-        const int* irregular = reinterpret_cast<int*>(net->slot_sync + 64);
         const cudaError_t fe = forward_slots_tc(SlotSystem{n, a.raw, a.mask, a.diag, a.sd, a.ld, a.sums}, net->off, net->wimg, nullptr,
                                                 nullptr, nullptr, nullptr, a.th, net->tc_err_dev, nullptr);
         k_slot_assemble<<<(n + kSlotThreads - 1) / kSlotThreads, kSlotThreads>>>(
-            n, sys->row_ptr, a.mask, a.sd, a.th, net->off, irregular, m_val);
+            n, sys->row_ptr, a.mask, a.sd, a.th, net->off, a.irregular, m_val);
         hpb::count_launch(2);
-        cudaMemcpyAsync(net->tc_err + 1, irregular, sizeof(int), cudaMemcpyDeviceToHost, nullptr);
+        const cudaError_t le = cudaGetLastError();
+        int irregular = 0;
+        const cudaError_t ce = cudaMemcpy(&irregular, a.irregular, sizeof(int), cudaMemcpyDeviceToHost);
         pool_free(mem, nullptr);
-        if (fe != cudaSuccess || cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess)
-            return HPB_ERROR_CUDA;
+        if (fe != cudaSuccess || le != cudaSuccess || ce != cudaSuccess) return HPB_ERROR_CUDA;
         const int tc = take_tc_status(net);
         if (tc != HPB_SUCCESS) return tc;
-        if (net->tc_err[1] == 0) return HPB_SUCCESS;
+        if (irregular == 0) return HPB_SUCCESS;
     }
     const size_t R = size_t(n);
     float* diag = static_cast<float*>(pool_alloc(R * 4, nullptr));
@@ -1435,7 +1436,6 @@ int loss_slots(hpb_spai* net, const hpb_spai_system& sys, float w_frob, float w_
     }
     const SlotArrays a = slot_arrays(net->slot_mem, size_t(n), net->off, true);
     launch_slot_load(net, sys, sys.nres, a);
-    const int* irr = reinterpret_cast<int*>(net->slot_sync + 64);
     if (forward_slots_tc(SlotSystem{n, a.raw, a.mask, a.diag, a.sd, a.ld, a.sums}, net->off, net->wimg, a.ah, grad ? a.feat : nullptr,
                          grad ? a.h1 : nullptr, grad ? a.h2 : nullptr, a.th, net->tc_err_dev, nullptr) != cudaSuccess)
         return HPB_ERROR_CUDA;
@@ -1456,7 +1456,7 @@ int loss_slots(hpb_spai* net, const hpb_spai_system& sys, float w_frob, float w_
     }
     float* gsys = reinterpret_cast<float*>(net->slot_out + 4);
     const int gblocks = grad ? (kNumParams + kSlotThreads - 1) / kSlotThreads : 0;
-    k_slot_close<<<gblocks + 1, kSlotThreads>>>(grid, net->part, gsys, net->grad, w, net->off.nsq, nb, w_frob, w_resid, irr,
+    k_slot_close<<<gblocks + 1, kSlotThreads>>>(grid, net->part, gsys, net->grad, w, net->off.nsq, nb, w_frob, w_resid, a.irregular,
                                                 net->slot_out);
     hpb::count_launch(grad ? 6 : 4);
     cudaMemcpyAsync(net->slot_host, net->slot_out, grad && grad_host ? kSlotOutBytes : 4 * sizeof(double),
