@@ -254,27 +254,39 @@ __device__ __forceinline__ bool is_dep(int32_t n, int32_t i, int32_t j) {
 }
 
 // Row d has met a dependency of level lv - 1; its last one puts it on the
-// queue.  The count is taken down only after the maximum has returned (the
-// decrement's operand depends on it), so whoever takes the row off the queue
-// finds its final level.
+// queue.  The maximum is released with the count and acquired by whoever takes
+// the count to zero, the row released with its place in the queue, so whoever
+// takes it off (next_row) finds its final level.
 __device__ __forceinline__ void meet(LevelTile& T, int d, int lv) {
-    int old, left;
-    asm volatile("atom.shared::cta.max.s32 %0, [%1], %2;"
-                 : "=r"(old)
-                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&T.lev[d]))), "r"(lv)
+    asm volatile("red.relaxed.cta.shared::cta.max.s32 [%0], %1;" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(&T.lev[d]))),
+                 "r"(lv)
                  : "memory");
-    asm volatile("atom.shared::cta.add.s32 %0, [%1], %2;"
+    int left;
+    asm volatile("atom.acq_rel.cta.shared::cta.add.s32 %0, [%1], -1;"
                  : "=r"(left)
-                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&T.left[d]))), "r"((old >> 31) - 1)
+                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&T.left[d])))
                  : "memory");
     if (left == 1) {
         int at;
-        asm volatile("atom.shared::cta.add.s32 %0, [%1], 1;"
+        asm volatile("atom.relaxed.cta.shared::cta.add.s32 %0, [%1], 1;"
                      : "=r"(at)
                      : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&T.tail)))
                      : "memory");
-        *reinterpret_cast<volatile uint16_t*>(&T.queue[at]) = uint16_t(d);
+        asm volatile("st.release.cta.shared::cta.u16 [%0], %1;" ::"r"(
+                         static_cast<uint32_t>(__cvta_generic_to_shared(&T.queue[at]))),
+                     "h"(uint16_t(d))
+                     : "memory");
     }
+}
+// The queue's entry at `at` (kNoRow: not there yet).
+__device__ __forceinline__ int next_row(const LevelTile& T, int at) {
+    uint16_t v;
+    asm volatile("ld.acquire.cta.shared::cta.u16 %0, [%1];"
+                 : "=h"(v)
+                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(&T.queue[at])))
+                 : "memory");
+    return int(v);
 }
 
 template <bool UPPER>
@@ -423,14 +435,12 @@ k_tri_levels(int32_t n, int32_t ntiles, const int32_t* __restrict__ ci, const in
         // of them: a lane each, its dependents one after another.  This chain
         // of shared loads and atomics is what a level costs, so it is kept
         // short (one warp issues it; every instruction counts).
-        const volatile uint16_t* queue = T.queue;
         int head = 0, spins = 0;
         const int grp = lane >> 2, sub = lane & 3;
         unsigned long long t0 = 0;
         while (head < m) {
-            // (the second read, by the whole warp after the first, finds all that the first found)
-            const int wide = head + lane < m ? int(queue[head + lane]) : int(kNoRow);
-            int row = head + grp < m ? int(queue[head + grp]) : int(kNoRow);
+            const int wide = head + lane < m ? next_row(T, head + lane) : int(kNoRow);
+            int row = __shfl_sync(0xffffffffu, wide, grp);
             const unsigned none = __ballot_sync(0xffffffffu, wide == int(kNoRow));
             const int k = none ? __ffs(int(none)) - 1 : 32;  // rows ready without a gap
             if (k == 0) {
