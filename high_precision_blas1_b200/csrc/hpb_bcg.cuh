@@ -156,9 +156,9 @@ void launch_spmv_upd_slots(const SlotMat<E>& A, int j, int L, int grid, cudaStre
                            const Vecs<E>& V, E* x, const E* w, BcgState<typename scalar_of<E>::type>* st,
                            typename acc_of<typename scalar_of<E>::type>::type* partials, unsigned int* ticket,
                            int* badflag, EpiArgs<typename scalar_of<E>::type> ea);
-// resident blocks per SM of the second for step j of l
+// resident blocks per SM of the second for step j of l, with ns slots
 template <class E>
-int spmv_upd_slots_occupancy(const SlotMat<E>& A, int j, int L);
+int spmv_upd_slots_occupancy(int ns, int j, int L);
 
 }  // namespace fused
 }  // namespace hpb

@@ -180,9 +180,9 @@ void launch_spmv_upd_slots(const SlotMat<E>& A, int j, int L, int grid, cudaStre
 }
 
 template <class E>
-int spmv_upd_slots_occupancy(const SlotMat<E>& A, int j, int L) {
+int spmv_upd_slots_occupancy(int ns, int j, int L) {
     int occ = 1;
-    with_slots(A.ns, [&](auto nsc) {
+    with_slots(ns, [&](auto nsc) {
         with_step(j, [&](auto jc) {
             constexpr int NS = decltype(nsc)::value, J = decltype(jc)::value;
             const void* f = J + 1 == L ? reinterpret_cast<const void*>(k_spmv_upd_slots<E, J, true, NS>)
@@ -202,7 +202,7 @@ int spmv_upd_slots_occupancy(const SlotMat<E>& A, int j, int L) {
                                            const Vecs<E>&, E*, const E*, BcgState<scalar_of<E>::type>*,                 \
                                            acc_of<scalar_of<E>::type>::type*, unsigned int*, int*,                      \
                                            EpiArgs<scalar_of<E>::type>);                                                \
-    template int spmv_upd_slots_occupancy<E>(const SlotMat<E>&, int, int);
+    template int spmv_upd_slots_occupancy<E>(int, int, int);
 HPB_BCG_SLOTS(float)
 HPB_BCG_SLOTS(double)
 HPB_BCG_SLOTS(cf)

@@ -521,6 +521,7 @@ struct SolverWorkspace {
     cudaGraphExec_t exec = nullptr;
     int open(size_t pinned_bytes);
     void* alloc(size_t bytes);
+    void free_last();  // gives the last alloc()'s memory back
     ~SolverWorkspace();
 };
 

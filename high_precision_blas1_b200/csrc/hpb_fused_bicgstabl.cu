@@ -672,22 +672,31 @@ int BcgPlan<E>::init(const hpb_solver_params* p, int32_t rows, int64_t nnz, cons
     const int64_t n = rows;
     const int64_t need = (n + kThreads - 1) / kThreads;
     SolverWorkspace& ws = P.ws;
-    int wst = ws.open(sizeof(Report) + 8 * sizeof(double) + sizeof(MonState) + 2 * kLoopChunk * sizeof(double));
+    int wst = ws.open(sizeof(Report) + 8 * sizeof(double) + sizeof(MonState) + 2 * kLoopChunk * sizeof(double) +
+                      sizeof(OffsetTable));
     if (wst != HPB_SUCCESS) return wst;
     cudaStream_t s = ws.stream;
-    // allocations, the slot form and the diagonal run after the caller's work on the legacy default stream
+    // allocations, the matrix' offsets and the diagonal run after the caller's work on the legacy default stream
     if (cudaEventRecord(ws.ev, 0) != cudaSuccess || cudaStreamWaitEvent(s, ws.ev, 0) != cudaSuccess)
         return HPB_ERROR_CUDA;
-    if (build_slots<E>(ws, rows, nnz, rp, ci, val, &P.slots) != HPB_SUCCESS) return HPB_ERROR_CUDA;
+    P.hrep = static_cast<Report*>(ws.pinned);
+    P.hnorm = reinterpret_cast<double*>(static_cast<char*>(ws.pinned) + sizeof(Report));
+    P.hmon = reinterpret_cast<MonState*>(P.hnorm + 8);
+    P.hhist = reinterpret_cast<double*>(P.hmon + 1);
+    OffsetTable* const offs = reinterpret_cast<OffsetTable*>(P.hhist + 2 * kLoopChunk);
+    if (find_slots(ws, rows, nnz, rp, ci, offs) != HPB_SUCCESS) return HPB_ERROR_CUDA;
     P.g_ew = int(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * light_occupancy<E>())));
     P.g_red = int(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * reduction_occupancy<E>(L))));
     P.g_sp = int(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * 8)));  // grid-stride rows, 8 blocks per SM
     P.g_spd = int(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * 6)));
+    // the update + product's grids on the CSR and on the slots, of which one is
+    // taken when it is known whether there are slots
+    auto su_grid = [&](int cap) { return int(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * cap))); };
     int g_su_max = 1;
     for (int j = 0; j < L; ++j) {
-        const int cap = P.slots.ns ? spmv_upd_slots_occupancy<E>(P.slots, j, L) : std::min(6, spmv_upd_occupancy<E>(j, L));
-        P.g_su[j] = int(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * cap)));
+        P.g_su[j] = su_grid(std::min(6, spmv_upd_occupancy<E>(j, L)));
         g_su_max = std::max(g_su_max, P.g_su[j]);
+        for (int ns : {5, kMaxSlots}) g_su_max = std::max(g_su_max, su_grid(spmv_upd_slots_occupancy<E>(ns, j, L)));
     }
     P.g_nrm = int(std::max<int64_t>(
         1, std::min<int64_t>(need, int64_t(sms) * occupancy_of(reinterpret_cast<const void*>(k_norm<E>)))));
@@ -717,10 +726,6 @@ int BcgPlan<E>::init(const hpb_solver_params* p, int32_t rows, int64_t nnz, cons
     P.dnorm = static_cast<double*>(ws.alloc(4 * sizeof(double)));
     if (!P.rt || !P.tmp || (jac && !P.diag) || !P.st || !P.drep || !P.partials || !P.ticket || !P.badflag || !P.dnorm)
         return HPB_ERROR_OUT_OF_MEMORY;
-    P.hrep = static_cast<Report*>(ws.pinned);
-    P.hnorm = reinterpret_cast<double*>(static_cast<char*>(ws.pinned) + sizeof(Report));
-    P.hmon = reinterpret_cast<MonState*>(P.hnorm + 8);
-    P.hhist = reinterpret_cast<double*>(P.hmon + 1);
     P.mon = static_cast<MonState*>(ws.alloc(sizeof(MonState)));
     P.dhist = static_cast<double*>(ws.alloc(2 * kLoopChunk * sizeof(double)));
     if (!P.mon || !P.dhist) return HPB_ERROR_OUT_OF_MEMORY;
@@ -730,7 +735,10 @@ int BcgPlan<E>::init(const hpb_solver_params* p, int32_t rows, int64_t nnz, cons
         k_diag<E><<<(rows + 255) / 256, 256, 0, s>>>(rows, rp, ci, val, P.diag);
         count_launch();
     }
-    if (cudaStreamSynchronize(s) != cudaSuccess) return HPB_ERROR_CUDA;
+    if (cudaStreamSynchronize(s) != cudaSuccess || make_slots<E>(ws, rows, nnz, rp, ci, val, offs, &P.slots) != HPB_SUCCESS)
+        return HPB_ERROR_CUDA;
+    if (P.slots.ns > 0)
+        for (int j = 0; j < L; ++j) P.g_su[j] = su_grid(spmv_upd_slots_occupancy<E>(P.slots.ns, j, L));
 
     // ---- one cycle as a CUDA graph
     BcgState<S>* st = P.st;

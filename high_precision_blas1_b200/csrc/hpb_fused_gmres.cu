@@ -1057,16 +1057,18 @@ int GmPlan<E>::init(const hpb_solver_params* p, int32_t rows, int64_t nnz, const
     const int g_rc = P.g_rc = int(std::max<int64_t>(1, (int64_t(rows) + kGmThreads - 1) / kGmThreads));
     SolverWorkspace& ws = P.ws;
     const size_t vb = size_t(n) * sizeof(E);
-    int wst = ws.open(sizeof(GmHostView));
+    int wst = ws.open(sizeof(GmHostView) + 2 * sizeof(OffsetTable));
     if (wst != HPB_SUCCESS) return wst;
     cudaStream_t s = ws.stream;
     // allocations and the diagonal run after the caller's work on the legacy default stream
     if (cudaEventRecord(ws.ev, 0) != cudaSuccess || cudaStreamWaitEvent(s, ws.ev, 0) != cudaSuccess)
         return HPB_ERROR_CUDA;
-    if (build_slots<E>(ws, rows, nnz, rp, ci, val, &P.slots) != HPB_SUCCESS ||
-        (M.kind == 2 && M.rows == rows &&
-         build_slots<E>(ws, M.rows, M.nnz, M.rp, M.ci, M.val, &P.mslots,
-                        M.rp == rp && M.ci == ci && M.nnz == nnz ? &P.slots : nullptr) != HPB_SUCCESS))
+    // the offsets of A and of a CSR preconditioner; the slots once all else is allocated
+    OffsetTable* const offs = reinterpret_cast<OffsetTable*>(static_cast<GmHostView*>(ws.pinned) + 1);
+    const bool m_slots = M.kind == 2 && M.rows == rows;
+    const bool m_like = m_slots && M.rp == rp && M.ci == ci && M.nnz == nnz;
+    if (find_slots(ws, rows, nnz, rp, ci, offs) != HPB_SUCCESS ||
+        (m_slots && !m_like && find_slots(ws, M.rows, M.nnz, M.rp, M.ci, offs + 1) != HPB_SUCCESS))
         return HPB_ERROR_CUDA;
     E* V = P.V = static_cast<E*>(ws.alloc(vb * size_t(m + 1)));
     E* W = P.W = static_cast<E*>(ws.alloc(vb));
@@ -1124,7 +1126,11 @@ int GmPlan<E>::init(const hpb_solver_params* p, int32_t rows, int64_t nnz, const
         k_gm_diag<E><<<(rows + 255) / 256, 256, 0, s>>>(rows, rp, ci, val, diag);
         count_launch();
     }
-    if (cudaStreamSynchronize(s) != cudaSuccess) return HPB_ERROR_CUDA;
+    if (cudaStreamSynchronize(s) != cudaSuccess ||
+        make_slots<E>(ws, rows, nnz, rp, ci, val, offs, &P.slots) != HPB_SUCCESS ||
+        (m_slots && make_slots<E>(ws, M.rows, M.nnz, M.rp, M.ci, M.val, offs + 1, &P.mslots,
+                                  m_like ? &P.slots : nullptr) != HPB_SUCCESS))
+        return HPB_ERROR_CUDA;
 
     const int lm_res = P.lm_res = load_mode<E>(val, x, nnz);
     // ---- one restart cycle as a CUDA graph

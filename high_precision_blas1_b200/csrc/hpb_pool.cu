@@ -111,6 +111,11 @@ void* SolverWorkspace::alloc(size_t bytes) {
     return p;
 }
 
+void SolverWorkspace::free_last() {
+    pool_free(dev.back(), stream);
+    dev.pop_back();
+}
+
 SolverWorkspace::~SolverWorkspace() {
     if (stream) cudaStreamSynchronize(stream);
     if (exec) cudaGraphExecDestroy(exec);

@@ -11,13 +11,8 @@ namespace {
 constexpr int kFindThreads = 256;
 constexpr int kNoOffset = INT_MIN;
 
-// Distinct offsets col - row of the whole matrix into table (kMaxSlots words,
-// kNoOffset where free); *bad: more than that, or a row whose columns do not
-// increase within [0, rows).  Each block collects its own in shared memory.
-struct OffsetTable {
-    int off[kMaxSlots];
-    int bad;
-};
+// Distinct offsets col - row of the whole matrix.  Each block collects its own in
+// shared memory.
 __global__ void k_slots_init(OffsetTable* t) {
     if (threadIdx.x < kMaxSlots) t->off[threadIdx.x] = kNoOffset;
     if (threadIdx.x == kMaxSlots) t->bad = 0;
@@ -93,42 +88,46 @@ k_slots_fill(int32_t rows, const int32_t* __restrict__ rp, const int32_t* __rest
 
 }  // namespace
 
-template <class E>
-int build_slots(SolverWorkspace& ws, int32_t rows, int64_t nnz, const int32_t* rp, const int32_t* ci, const E* val,
-                SlotMat<E>* out, const SlotMat<E>* like) {
-    *out = SlotMat<E>{};
-    if (rows <= 0 || nnz <= 0) return HPB_SUCCESS;
+int find_slots(SolverWorkspace& ws, int32_t rows, int64_t nnz, const int32_t* rp, const int32_t* ci, OffsetTable* host) {
+    host->bad = 1;
+    // at least nnz / rows offsets: a matrix with longer rows has no slot form
+    if (rows <= 0 || nnz <= 0 || nnz > int64_t(rows) * kMaxSlots) return HPB_SUCCESS;
     cudaStream_t s = ws.stream;
+    OffsetTable* t = static_cast<OffsetTable*>(ws.alloc(sizeof(OffsetTable)));
+    if (t == nullptr) return HPB_SUCCESS;
+    k_slots_init<<<1, 32, 0, s>>>(t);
+    k_slots_find<<<int(std::min<int64_t>((int64_t(rows) + kFindThreads - 1) / kFindThreads, 148 * 8)), kFindThreads, 0, s>>>(
+        rows, nnz, rp, ci, t);
+    count_launch(2);
+    return cudaMemcpyAsync(host, t, sizeof(*t), cudaMemcpyDeviceToHost, s) == cudaSuccess ? HPB_SUCCESS : HPB_ERROR_CUDA;
+}
+
+template <class E>
+int make_slots(SolverWorkspace& ws, int32_t rows, int64_t nnz, const int32_t* rp, const int32_t* ci, const E* val,
+               const OffsetTable* host, SlotMat<E>* out, const SlotMat<E>* like) {
+    *out = SlotMat<E>{};
     SlotMat<E> A;
     if (like != nullptr) {
         if (like->ns == 0) return HPB_SUCCESS;
         A = *like;
     } else {
-        // at least nnz / rows offsets: a matrix with longer rows has no slot form
-        if (nnz > int64_t(rows) * kMaxSlots) return HPB_SUCCESS;
-        OffsetTable* t = static_cast<OffsetTable*>(ws.alloc(sizeof(OffsetTable)));
-        if (t == nullptr) return HPB_SUCCESS;
-        k_slots_init<<<1, 32, 0, s>>>(t);
-        k_slots_find<<<int(std::min<int64_t>((int64_t(rows) + kFindThreads - 1) / kFindThreads, 148 * 8)), kFindThreads, 0,
-                       s>>>(rows, nnz, rp, ci, t);
-        count_launch(2);
-        OffsetTable h;
-        if (cudaMemcpyAsync(&h, t, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess)
-            return HPB_ERROR_CUDA;
-        if (h.bad) return HPB_SUCCESS;
+        if (host->bad) return HPB_SUCCESS;
         for (int q = 0; q < kMaxSlots; ++q)
-            if (h.off[q] != kNoOffset) A.off[A.ns++] = h.off[q];
+            if (host->off[q] != kNoOffset) A.off[A.ns++] = host->off[q];
         std::sort(A.off, A.off + A.ns);
         if (A.ns == 0 || int64_t(std::max(A.ns, 5)) * rows > nnz + nnz / 3) return HPB_SUCCESS;
     }
     const int held = std::max(A.ns, 5);  // kernels read at least five slots
     E* v = static_cast<E*>(ws.alloc(size_t(held) * size_t(rows) * sizeof(E)));
-    uint8_t* mask = v ? static_cast<uint8_t*>(ws.alloc(size_t(rows))) : nullptr;
-    if (mask == nullptr) return HPB_SUCCESS;
+    if (v == nullptr) return HPB_SUCCESS;
+    uint8_t* mask = static_cast<uint8_t*>(ws.alloc(size_t(rows)));
+    if (mask == nullptr) {
+        ws.free_last();
+        return HPB_SUCCESS;
+    }
     SlotTarget<E> t{v, mask, A.ns, held, {}};
     for (int q = 0; q < kMaxSlots; ++q) t.off[q] = A.off[q];
-    k_slots_fill<E><<<int((int64_t(rows) + kFindThreads - 1) / kFindThreads), kFindThreads, 0, s>>>(rows, rp, ci, val, t);
+    k_slots_fill<E><<<int((int64_t(rows) + kFindThreads - 1) / kFindThreads), kFindThreads, 0, ws.stream>>>(rows, rp, ci, val, t);
     count_launch();
     if (cudaGetLastError() != cudaSuccess) return HPB_ERROR_CUDA;
     A.val = v;
@@ -138,8 +137,8 @@ int build_slots(SolverWorkspace& ws, int32_t rows, int64_t nnz, const int32_t* r
 }
 
 #define HPB_SLOTS_INST(E)                                                                                       \
-    template int build_slots<E>(SolverWorkspace&, int32_t, int64_t, const int32_t*, const int32_t*, const E*, \
-                                SlotMat<E>*, const SlotMat<E>*);
+    template int make_slots<E>(SolverWorkspace&, int32_t, int64_t, const int32_t*, const int32_t*, const E*, \
+                               const OffsetTable*, SlotMat<E>*, const SlotMat<E>*);
 HPB_SLOTS_INST(float)
 HPB_SLOTS_INST(double)
 HPB_SLOTS_INST(cf)

@@ -25,16 +25,28 @@ struct SlotMat {
     int off[kMaxSlots] = {};  // (with fewer than five slots val holds five: the others empty)
 };
 
-// The slot form of a CSR matrix if it has one (ns > 0 on return), in
-// workspace memory on the workspace's stream; waits for that stream once.
+// Distinct offsets col - row of a whole matrix (kNoOffset where free); bad: more
+// than kMaxSlots, or a row whose columns do not increase within [0, rows).
+struct OffsetTable {
+    int off[kMaxSlots];
+    int bad;
+};
+
+// The slot form of a CSR matrix if it has one, in two steps that both leave
+// their work on the workspace's stream: find_slots fills *host (pinned), which
+// may be read once the stream has been waited for; make_slots then fills the
+// slots in workspace memory (ns > 0 on return).  A plan makes its slots after
+// all it cannot do without is allocated: without memory for them the matrix
+// stays CSR.
 // Rule: at most kMaxSlots distinct offsets, columns increasing in every row
 // and within [0, rows), and no more than a quarter of the slots empty (a
 // matrix that fills its slots less would move more bytes than its CSR).
-// Without memory for it the matrix stays CSR.  `like`: a slot form of a matrix
-// with the same row pointers and column indices, whose offsets are taken over.
+// `like`: a slot form of a matrix with the same row pointers and column
+// indices, whose offsets are taken over (no find_slots then, host unused).
+int find_slots(SolverWorkspace& ws, int32_t rows, int64_t nnz, const int32_t* rp, const int32_t* ci, OffsetTable* host);
 template <class E>
-int build_slots(SolverWorkspace& ws, int32_t rows, int64_t nnz, const int32_t* rp, const int32_t* ci, const E* val,
-                SlotMat<E>* out, const SlotMat<E>* like = nullptr);
+int make_slots(SolverWorkspace& ws, int32_t rows, int64_t nnz, const int32_t* rp, const int32_t* ci, const E* val,
+               const OffsetTable* host, SlotMat<E>* out, const SlotMat<E>* like = nullptr);
 
 // y_i = sum_s a_{i,s} x(i + off[s]) over the slots row i stores, in slot order;
 // X: (column) -> operand.  Every load is issued whether the row stores the slot
