@@ -1375,7 +1375,7 @@ k_ilu0(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int32_t* 
        const int32_t* __restrict__ nlev, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
        const int32_t* __restrict__ dpos, E* val, unsigned* flags, const int* __restrict__ general, int* err,
        int* err_row) {
-    if (!*general) return;  // k_ilu0_diag has done it
+    if (general != nullptr && !*general) return;  // k_ilu0_diag has done it
     __shared__ int s_tile;
     __shared__ int s_done;
     if (threadIdx.x == 0) {
@@ -1619,26 +1619,31 @@ cudaError_t launch_trsv_sweeps(const Plan& P, int unit, const E* val, E alpha, c
 template <class E>
 cudaError_t launch_ilu0(const Plan& P, E* val, cudaStream_t s) {
     if (P.n == 0) return cudaSuccess;
-    // scratch: the published diagonal, the positions of a_ki, the tile ticket and the kind of matrix
+    // scratch: the published diagonal, the positions of a_ki, the tile ticket and the
+    // kind of matrix.  Without memory for it the general kernel, which needs none.
     const size_t o_piv = (size_t(P.n) * sizeof(int4) + 255) & ~size_t(255);
     const size_t o_word = (o_piv + size_t(P.n) * sizeof(E) + 255) & ~size_t(255);
     char* work = static_cast<char*>(fused::analysis_alloc(o_word + 8, s));
-    if (work == nullptr) return cudaErrorMemoryAllocation;
-    int4* wpos = reinterpret_cast<int4*>(work);
-    E* piv = reinterpret_cast<E*>(work + o_piv);
-    unsigned* ticket = reinterpret_cast<unsigned*>(work + o_word);
-    int* general = reinterpret_cast<int*>(work + o_word + 4);
-    cudaError_t e = cudaMemsetAsync(general, 0, sizeof(int), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(P.flags, 0, (size_t(P.n) + 1) * sizeof(unsigned), s);
+    int* general = work ? reinterpret_cast<int*>(work + o_word + 4) : nullptr;
+    cudaError_t e = cudaMemsetAsync(P.flags, 0, (size_t(P.n) + 1) * sizeof(unsigned), s);
+    if (e == cudaSuccess && work != nullptr) {
+        int4* wpos = reinterpret_cast<int4*>(work);
+        E* piv = reinterpret_cast<E*>(work + o_piv);
+        unsigned* ticket = reinterpret_cast<unsigned*>(work + o_word);
+        e = cudaMemsetAsync(general, 0, sizeof(int), s);
+        if (e == cudaSuccess) {
+            k_ilu0_pattern<<<(P.n + 255) / 256, 256, 0, s>>>(P.n, P.desc, P.rp, P.ci, P.dpos, wpos, general);
+            k_tri_fill<E><<<int(std::min<int64_t>((int64_t(P.n) + 255) / 256, 148 * 8)), 256, 0, s>>>(P.n, piv, ticket);
+            allow_smem(k_ilu0_diag<E>, sizeof(TileValues<E>));
+            k_ilu0_diag<E><<<P.ntiles, kSolveThreads, sizeof(TileValues<E>), s>>>(
+                P.n, P.ntiles, P.desc, P.dsrc, P.chunks, wpos, val, piv, ticket, general, P.err, P.err_row);
+            count_launch(3);
+        }
+    }
     if (e == cudaSuccess) {
-        k_ilu0_pattern<<<(P.n + 255) / 256, 256, 0, s>>>(P.n, P.desc, P.rp, P.ci, P.dpos, wpos, general);
-        k_tri_fill<E><<<int(std::min<int64_t>((int64_t(P.n) + 255) / 256, 148 * 8)), 256, 0, s>>>(P.n, piv, ticket);
-        allow_smem(k_ilu0_diag<E>, sizeof(TileValues<E>));
-        k_ilu0_diag<E><<<P.ntiles, kSolveThreads, sizeof(TileValues<E>), s>>>(
-            P.n, P.ntiles, P.desc, P.dsrc, P.chunks, wpos, val, piv, ticket, general, P.err, P.err_row);
         k_ilu0<E><<<P.ntiles, kTriThreads, 0, s>>>(P.n, P.ntiles, P.desc, P.lvlptr, P.nlev, P.rp, P.ci, P.dpos, val,
                                                    P.flags, general, P.err, P.err_row);
-        count_launch(4);
+        count_launch();
         e = cudaGetLastError();
     }
     fused::analysis_free(work, s);

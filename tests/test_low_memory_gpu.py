@@ -80,6 +80,20 @@ def analysis(ctx, A, upper):
     return h
 
 
+def test_ilu0_without_scratch(gpu):
+    """24 bytes a row (100 MB) of scratch for the recurrence, 60 MB left: the general factorisation's bits are the same."""
+    ctx, torch = gpu
+    A = five_point(torch)
+    h = analysis(ctx, A, 0)
+    want, got = A[2].clone(), A[2].clone()
+    ctx.check(L.hpb_csr_ilu0_f64(ctx.h, h, want.data_ptr()), "ilu0")
+    with Scarce(torch, 60 * MB):
+        st = L.hpb_csr_ilu0_f64(ctx.h, h, got.data_ptr())
+    L.hpb_csr_tri_destroy(h)
+    assert st == 0
+    assert torch.equal(got.view(torch.int64), want.view(torch.int64))
+
+
 def test_analysis_after_a_solve(gpu):
     """What a solve's workspace keeps in its pool is there for an analysis when nothing else is."""
     ctx, torch = gpu
