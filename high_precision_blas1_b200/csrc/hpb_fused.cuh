@@ -506,11 +506,14 @@ __device__ __forceinline__ void grid_finish(A (&acc)[ND], bool bad, A* partials,
 // are cached per host thread.  open() first, then alloc().
 void* pool_alloc(size_t bytes, cudaStream_t stream);
 void pool_free(void* p, cudaStream_t stream);
-// The same for the arrays of triangular analyses, which callers create and
+// The same as pool_alloc for the arrays of triangular analyses, which callers create and
 // release in turn with each new matrix: a pool of their own that keeps freed
 // memory up to a bound (hpb_pool.cu).
 void* analysis_alloc(size_t bytes, cudaStream_t stream);
 void analysis_free(void* p, cudaStream_t stream);
+// Pinned host memory of at most 4 KB from a list each thread keeps.
+void* pinned_acquire(size_t bytes);
+void pinned_release(void* p);
 
 struct SolverWorkspace {
     std::vector<void*> dev;

@@ -1003,26 +1003,33 @@ constexpr size_t kSlotOutBytes = 4 * sizeof(double) + size_t(kNumParams) * sizeo
 int grow(hpb_spai* net, int32_t rows, int64_t nnz) {
     using namespace hpb::spai;
     if (size_t(rows) <= net->cap_rows && size_t(nnz) <= net->cap_nnz) return HPB_SUCCESS;
-    float** fr[] = {&net->feat, &net->h1, &net->h2, &net->out, &net->dout, &net->diag,
-                    &net->y,    &net->z,  &net->g,  &net->G,   &net->rh,   &net->ahat};
-    for (auto f : fr) {
-        cudaFree(*f);
-        *f = nullptr;
-    }
-    cudaFree(net->mval);
-    cudaFree(net->dm);
-    cudaFree(net->lpart);
-    net->mval = net->dm = nullptr;
-    net->lpart = nullptr;
+    float** fr[] = {&net->feat, &net->h1, &net->h2, &net->out, &net->dout, &net->diag, &net->y,
+                    &net->z,    &net->g,  &net->G,  &net->rh,  &net->ahat, &net->mval, &net->dm};
     const size_t R = size_t(rows), Z = size_t(nnz ? nnz : 1);
-    if (cudaMalloc(&net->feat, R * kF * 4) || cudaMalloc(&net->h1, R * kH * 4) || cudaMalloc(&net->h2, R * kH * 4) ||
-        cudaMalloc(&net->out, R * kO * 4) || cudaMalloc(&net->dout, R * kO * 4) || cudaMalloc(&net->diag, R * 4) ||
-        cudaMalloc(&net->y, R * 4) || cudaMalloc(&net->z, R * 4) || cudaMalloc(&net->g, R * 4) ||
-        cudaMalloc(&net->G, R * kMaxSq * 4) || cudaMalloc(&net->mval, Z * 4) || cudaMalloc(&net->dm, Z * 4) ||
-        cudaMalloc(&net->rh, R * 4) || cudaMalloc(&net->ahat, Z * 4) ||
-        cudaMalloc(&net->lpart, ((R + kThreads - 1) / kThreads + 1) * 8)) {
+    const size_t len[] = {R * kF, R * kH, R * kH, R * kO, R * kO, R, R, R, R, R * kMaxSq, R, Z, Z, Z};
+    static_assert(sizeof(fr) / sizeof(fr[0]) == sizeof(len) / sizeof(len[0]), "a length for each array");
+    auto attempt = [&] {
+        for (auto f : fr) {
+            cudaFree(*f);
+            *f = nullptr;
+        }
+        cudaFree(net->lpart);
+        net->lpart = nullptr;
         net->cap_rows = net->cap_nnz = 0;
-        return HPB_ERROR_OUT_OF_MEMORY;
+        bool ok = true;
+        for (size_t k = 0; ok && k < sizeof(len) / sizeof(len[0]); ++k)
+            ok = cudaMalloc(fr[k], len[k] * sizeof(float)) == cudaSuccess;
+        return ok && cudaMalloc(&net->lpart, ((R + kThreads - 1) / kThreads + 1) * sizeof(double)) == cudaSuccess;
+    };
+    if (!attempt()) {  // once more without the slot form's workspace, which the system does not take
+        cudaGetLastError();
+        cudaFree(net->slot_mem);
+        net->slot_mem = nullptr;
+        net->slot_rows = 0;
+        if (!attempt()) {
+            cudaGetLastError();
+            return HPB_ERROR_OUT_OF_MEMORY;
+        }
     }
     net->cap_rows = R;
     net->cap_nnz = Z;
@@ -1353,10 +1360,7 @@ int hpb_spai_assemble(hpb_spai* net, const hpb_spai_system* sys, float* m_val) {
     // the solvers' pool on the legacy stream (no training workspace)
     using hpb::fused::pool_alloc;
     using hpb::fused::pool_free;
-    {
-        const size_t bytes = slot_arrays(nullptr, size_t(n), net->off, false).bytes;
-        char* mem = static_cast<char*>(pool_alloc(bytes, nullptr));
-        if (!mem) return HPB_ERROR_OUT_OF_MEMORY;
+    if (char* mem = static_cast<char*>(pool_alloc(slot_arrays(nullptr, size_t(n), net->off, false).bytes, nullptr))) {
         const SlotArrays a = slot_arrays(mem, size_t(n), net->off, false);
         launch_slot_load(net, *sys, -1, a);
         const cudaError_t fe = forward_slots_tc(SlotSystem{n, a.raw, a.mask, a.diag, a.sd, a.ld, a.sums}, net->off, net->wimg, nullptr,
@@ -1365,13 +1369,17 @@ int hpb_spai_assemble(hpb_spai* net, const hpb_spai_system* sys, float* m_val) {
             n, sys->row_ptr, a.mask, a.sd, a.th, net->off, a.irregular, m_val);
         hpb::count_launch(2);
         const cudaError_t le = cudaGetLastError();
-        int irregular = 0;
-        const cudaError_t ce = cudaMemcpy(&irregular, a.irregular, sizeof(int), cudaMemcpyDeviceToHost);
+        int* const word = static_cast<int*>(hpb::fused::pinned_acquire(sizeof(int)));  // the calling thread's
+        int pageable = 0, *const got = word ? word : &pageable;
+        cudaError_t ce = cudaMemcpyAsync(got, a.irregular, sizeof(int), cudaMemcpyDeviceToHost, nullptr);
         pool_free(mem, nullptr);
+        if (ce == cudaSuccess) ce = cudaStreamSynchronize(nullptr);
+        const bool irregular = *got != 0;
+        hpb::fused::pinned_release(word);
         if (fe != cudaSuccess || le != cudaSuccess || ce != cudaSuccess) return HPB_ERROR_CUDA;
         const int tc = take_tc_status(net);
         if (tc != HPB_SUCCESS) return tc;
-        if (irregular == 0) return HPB_SUCCESS;
+        if (!irregular) return HPB_SUCCESS;
     }
     const size_t R = size_t(n);
     float* diag = static_cast<float*>(pool_alloc(R * 4, nullptr));
@@ -1412,16 +1420,18 @@ int hpb_spai_forward(hpb_spai* net, int32_t rows, const float* feat, float* out,
 namespace {
 // The slot form of loss_impl: eight launches, one copy and one wait for the
 // host (the CSR kernels below: 35 launches, a copy and a wait for every sum).
-// *irregular: nothing was added, the system needs those.
+// *irregular: nothing was added, the system needs those (or there is no memory
+// for the slot form).
 // Measured on B200 (24^3, three samples): 85 us against 388 us.
 int loss_slots(hpb_spai* net, const hpb_spai_system& sys, float w_frob, float w_resid, double* loss, float* grad_host,
                bool grad, bool* irregular) {
     using namespace hpb::spai;
     const int32_t n = sys.rows;
+    *irregular = true;
     if (net->slot_host == nullptr && cudaMallocHost(&net->slot_host, kSlotOutBytes) != cudaSuccess) {
         cudaGetLastError();
         net->slot_host = nullptr;
-        return HPB_ERROR_OUT_OF_MEMORY;
+        return HPB_SUCCESS;
     }
     if (size_t(n) > net->slot_rows) {
         cudaFree(net->slot_mem);
@@ -1430,7 +1440,7 @@ int loss_slots(hpb_spai* net, const hpb_spai_system& sys, float w_frob, float w_
         if (cudaMalloc(&net->slot_mem, slot_arrays(nullptr, size_t(n), net->off, true).bytes) != cudaSuccess) {
             cudaGetLastError();
             net->slot_mem = nullptr;
-            return HPB_ERROR_OUT_OF_MEMORY;
+            return HPB_SUCCESS;
         }
         net->slot_rows = size_t(n);
     }

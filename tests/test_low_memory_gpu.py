@@ -1,11 +1,14 @@
-"""Calls that use memory where there is some, when there is not: they run as
-they would without it.  The rest of the device's memory is held by one
-allocation meanwhile."""
+"""Calls that use memory where there is some -- slot forms of a solver's
+matrices, the diagonal recurrence of ILU(0), the slot form of a training system
+-- when there is not: they run as they would without it.  The rest of the
+device's memory is held by one allocation meanwhile."""
 import ctypes as C
 
+import numpy as np
 import pytest
 
-from high_precision_blas1_b200 import _lib
+from gpu_utils import host
+from high_precision_blas1_b200 import _lib, problems, spai
 
 pytestmark = pytest.mark.gpu
 L = _lib.lib
@@ -103,3 +106,25 @@ def test_analysis_after_a_solve(gpu):
         h = [analysis(ctx, A, k) for k in (0, 1)]  # 58 bytes a row each: 480 MB, and 50 MB for a while
     for k in h:
         L.hpb_csr_tri_destroy(k)
+
+
+def test_training_system_outside_the_slot_form(gpu):
+    """It needs the general workspace; the slot form's, tried before, does not stand in its way."""
+    torch = gpu[1]
+    n = 64
+    A = problems.diffusion3d_lognormal(n, seed=1, sigma=1.0, corr=2.0)
+    rows = np.repeat(np.arange(A.n), np.diff(A.row_ptr))
+    r, c, v = np.append(rows, [10, 13]), np.append(A.col_ind, [13, 10]), np.append(A.val, [0.0, 0.0])
+    order = np.lexsort((c, r))
+    rp = np.zeros(A.n + 1, np.int32)
+    rp[1:] = np.cumsum(np.bincount(r, minlength=A.n))
+    D = spai.DeviceCSR(torch, problems.CSR(A.n, rp, c[order].astype(np.int32), v[order]))
+    offs, dslot = spai.stencil7(n)
+    want = spai.SpaiNet(offs, dslot, seed=1)
+    loss, g = want.loss_grad(D, want_grad=True)
+    want.close()
+    net = spai.SpaiNet(offs, dslot, seed=1)
+    with Scarce(torch, int(1.5 * 900 * A.n)):  # each workspace takes 800 to 900 bytes a row
+        got, h = net.loss_grad(D, want_grad=True)
+    net.close()
+    assert np.array_equal(got, loss) and np.array_equal(h, g)
