@@ -24,6 +24,7 @@ namespace {
 
 constexpr int kSortThreads = 1024;
 constexpr int kPre = 4;                          // dependencies per row prefetched into registers
+constexpr int kMore = 10;                        // solve: those of rows with more than kPre, at most
 constexpr int kMerge = 8;                        // ILU(0): update pairs per batch of loads
 // Every wait ends after kWaitNs of GPU time (%globaltimer) at the latest.
 // A legitimate wait lasts at most as long as the launch itself (a tile waits
@@ -1088,7 +1089,30 @@ k_trsv(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int4* __r
             case 2: solve_steps<E, UNIT, 2>(r, prep, src, out, steps, mine, publish, xo, from, to); break;
             case 3: solve_steps<E, UNIT, 3>(r, prep, src, out, steps, mine, publish, xo, from, to); break;
             case 4: solve_steps<E, UNIT, 4>(r, prep, src, out, steps, mine, publish, xo, from, to); break;
-            default:  // rows with more than kPre dependencies among them
+            default: {  // rows with more than kPre dependencies among them
+                // The next kMore: sources and values, and other tiles' values, before the
+                // turn.  (Looked up during it -- column, position, value one after another,
+                // other tiles' rows one by one from L2 -- they were most of a solve: lower /
+                // upper, ILU(0) on B200, f64 27-point 64^3 4964 / 5347 -> 708 / 803 us, 13-point
+                // 500^2 2022 / 2785 -> 801 / 913, f32 27-point 64^3 3500 / 4103 -> 628 / 748.)
+                int ms[kMore];
+                E mv[kMore], mx[kMore];
+#pragma unroll
+                for (int k = 0; k < kMore; ++k) {
+                    ms[k] = -1;
+                    if (kPre + k < r.d.z) {
+                        const int32_t e = r.d.y + kPre + k, j = __ldg(ci + e), jl = j - base;
+                        mv[k] = ldE(val, e);
+                        if (jl >= 0 && jl < m)
+                            ms[k] = __ldg(pos + j);
+                        else
+                            mx[k] = Pub<E>::load(x, j);
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < kMore; ++k)
+                    if (kPre + k < r.d.z && ms[k] < 0 && Pub<E>::pending(mx[k]))
+                        mx[k] = await_value(x, __ldg(ci + (r.d.y + kPre + k)), mx[k], err, lim);
                 __syncwarp();
                 if (from >= 0) chunk_sync(from);
                 for (int l = 1; l <= steps; ++l) {
@@ -1097,19 +1121,23 @@ k_trsv(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int4* __r
 #pragma unroll
                         for (int k = 0; k < kPre; ++k)
                             if (k < r.d.z) acc = fms(acc, r.v[k], *src[k]);
-                        for (int32_t e = r.d.y + kPre; e < r.d.y + r.d.z; ++e) {
+#pragma unroll
+                        for (int k = 0; k < kMore; ++k)
+                            if (kPre + k < r.d.z) acc = fms(acc, mv[k], ms[k] >= 0 ? T.xs[ms[k]] : mx[k]);
+                        for (int32_t e = r.d.y + kPre + kMore; e < r.d.y + r.d.z; ++e) {
                             const int32_t j = __ldg(ci + e), jl = j - base;
                             const E xv = (jl >= 0 && jl < m) ? T.xs[__ldg(pos + j)]
                                                              : await_value(x, j, Pub<E>::load(x, j), err, lim);
                             acc = fms(acc, ldE(val, e), xv);
                         }
-                        if (!UNIT) acc = quot(acc, r.dg);
+                        if (!UNIT) acc = quot_prepared(acc, r.dg, prep, true);
                         *out = acc;
                         if (publish) Pub<E>::store(xo, 0, acc);
                     }
                     __syncwarp();
                 }
                 if (to >= 0) chunk_arrive(to);
+            }
         }
         r = nx;
         nx = nn;
