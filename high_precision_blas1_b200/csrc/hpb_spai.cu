@@ -291,7 +291,14 @@ struct SlotMats {  // training workspace, all slot form: [.. * n + i]
     double* lpart;         // block sums of ||G||^2 and ||z_s||^2
     const double* sums;    // [0] sum of logs, [1 + s] ||rh_s||^2
     int nres;
+    const int* irregular;  // not 0: no slot form
 };
+// Row i's mask, empty in a system without a slot form, so that the kernels that
+// would take longest end soon (both loads are in flight together).
+__device__ __forceinline__ unsigned slot_mask(const SlotMats& w, int32_t i) {
+    const unsigned m = __ldg(w.mask + i);
+    return __ldg(w.irregular) ? 0u : m;
+}
 
 // CSR -> slot form; the sum of log|a_ii| and rh_s = r_s / sqrt|a_ii| with
 // ||rh_s||^2 (all Dot2-merged).  *irregular: the system is not of that kind.
@@ -430,7 +437,7 @@ __global__ void __launch_bounds__(kSlotThreads) k_slot_gz(SlotMats w, Offsets o,
     const int t = blockIdx.y;
     float v = 0.f;
     if (i < n) {
-        const unsigned m = __ldg(w.mask + i);
+        const unsigned m = slot_mask(w, i);
         if (t < o.nsq) {
 #pragma unroll
             for (int p = 0; p < kMaxSlot; ++p) {
@@ -463,7 +470,7 @@ __global__ void __launch_bounds__(kSlotThreads) k_slot_dm(SlotMats w, Offsets o,
     const int32_t n = w.n, k = blockIdx.x * kSlotThreads + threadIdx.x;
     const int q = blockIdx.y;
     if (k >= n) return;
-    const unsigned m = __ldg(w.mask + k);
+    const unsigned m = slot_mask(w, k);
     float dm = 0.f;
     if ((m >> q) & 1u) {
         float s = 0.f, a[kMaxSlot];
@@ -559,6 +566,8 @@ k_backward(int32_t rows, const float* __restrict__ feat, const __nv_bfloat16* __
            const float* __restrict__ h1g, const float* __restrict__ h2g, const float* __restrict__ dout, SlotMats sm,
            Offsets o, float* __restrict__ part) {
     extern __shared__ __align__(16) unsigned char smraw[];
+    int irregular = 0;
+    if constexpr (SLOTS) irregular = __ldg(sm.irregular);
     float* sX = reinterpret_cast<float*>(smraw);   // kBwdRows x kSX
     float* sH1 = sX + kBwdRows * kSX;              // kBwdRows x kSH
     float* sH2 = sH1 + kBwdRows * kSH;
@@ -582,7 +591,7 @@ k_backward(int32_t rows, const float* __restrict__ feat, const __nv_bfloat16* __
     for (int i = 0; i < kBwdTilesPerWarp; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
     float bsum = 0.f;  // bias gradient of parameter column threadIdx.x (< 2 kH + kO)
     __syncthreads();
-    const int nchunks = (rows + kBwdRows - 1) / kBwdRows;
+    const int nchunks = irregular ? 0 : (rows + kBwdRows - 1) / kBwdRows;
     for (int ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
         // ---------------- phase 1: this warp's 16 rows
         if constexpr (SLOTS) {
@@ -1363,7 +1372,7 @@ int hpb_spai_assemble(hpb_spai* net, const hpb_spai_system* sys, float* m_val) {
     if (char* mem = static_cast<char*>(pool_alloc(slot_arrays(nullptr, size_t(n), net->off, false).bytes, nullptr))) {
         const SlotArrays a = slot_arrays(mem, size_t(n), net->off, false);
         launch_slot_load(net, *sys, -1, a);
-        const cudaError_t fe = forward_slots_tc(SlotSystem{n, a.raw, a.mask, a.diag, a.sd, a.ld, a.sums}, net->off, net->wimg, nullptr,
+        const cudaError_t fe = forward_slots_tc(SlotSystem{n, a.raw, a.mask, a.diag, a.sd, a.ld, a.sums, a.irregular}, net->off, net->wimg, nullptr,
                                                 nullptr, nullptr, nullptr, a.th, net->tc_err_dev, nullptr);
         k_slot_assemble<<<(n + kSlotThreads - 1) / kSlotThreads, kSlotThreads>>>(
             n, sys->row_ptr, a.mask, a.sd, a.th, net->off, a.irregular, m_val);
@@ -1421,7 +1430,8 @@ namespace {
 // The slot form of loss_impl: eight launches, one copy and one wait for the
 // host (the CSR kernels below: 35 launches, a copy and a wait for every sum).
 // *irregular: nothing was added, the system needs those (or there is no memory
-// for the slot form).
+// for the slot form).  It is known on the device once k_slot_load has run; the
+// kernels behind it that would take longest then end at once.
 // Measured on B200 (24^3, three samples): 85 us against 388 us.
 int loss_slots(hpb_spai* net, const hpb_spai_system& sys, float w_frob, float w_resid, double* loss, float* grad_host,
                bool grad, bool* irregular) {
@@ -1446,10 +1456,10 @@ int loss_slots(hpb_spai* net, const hpb_spai_system& sys, float w_frob, float w_
     }
     const SlotArrays a = slot_arrays(net->slot_mem, size_t(n), net->off, true);
     launch_slot_load(net, sys, sys.nres, a);
-    if (forward_slots_tc(SlotSystem{n, a.raw, a.mask, a.diag, a.sd, a.ld, a.sums}, net->off, net->wimg, a.ah, grad ? a.feat : nullptr,
+    if (forward_slots_tc(SlotSystem{n, a.raw, a.mask, a.diag, a.sd, a.ld, a.sums, a.irregular}, net->off, net->wimg, a.ah, grad ? a.feat : nullptr,
                          grad ? a.h1 : nullptr, grad ? a.h2 : nullptr, a.th, net->tc_err_dev, nullptr) != cudaSuccess)
         return HPB_ERROR_CUDA;
-    const SlotMats w{n, a.mask, a.ah, a.th, a.mh, a.y, a.z, a.rh, a.G, a.dm, a.lpart, a.sums, sys.nres};
+    const SlotMats w{n, a.mask, a.ah, a.th, a.mh, a.y, a.z, a.rh, a.G, a.dm, a.lpart, a.sums, sys.nres, a.irregular};
     const int nb = (n + kSlotThreads - 1) / kSlotThreads, planes = net->off.nsq + sys.nres;
     k_slot_mh<<<nb, kSlotThreads>>>(w, net->off);
     k_slot_gz<<<dim3(unsigned(nb), unsigned(planes)), kSlotThreads>>>(w, net->off, net->pairs);

@@ -45,6 +45,7 @@ struct SlotSystem {
     const double* sd;    // 1 / sqrt|a_ii| and log|a_ii|: the build's features come from these,
     const double* ld;    //   training's (null here) from diag
     const double* lsum;  // sum of log|a_ii|
+    const int* irregular;  // not 0: the system has no slot form, nothing is done
 };
 
 __device__ __forceinline__ float inv_sqrt_dd(float di, float dj) { return 1.f / sqrtf(fabsf(di * dj)); }

@@ -326,11 +326,14 @@ k_forward_tc(int32_t rows, const float* __restrict__ feat, SlotArgs g, const uns
         constexpr int NW = kImgW / 16, NB = kImgBias / 16, PER = (NW + NB + kTcThreads - 1) / kTcThreads;
         const uint4* src = reinterpret_cast<const uint4*>(img);
         uint4 v[PER];
+        int irregular = 0;
+        if constexpr (SLOTS) irregular = __ldg(g.sys.irregular);
 #pragma unroll
         for (int r = 0; r < PER; ++r) {
             const int q = t + r * kTcThreads;
             if (q < NW + NB) v[r] = __ldg(src + q);
         }
+        if (irregular != 0) return;
 #pragma unroll
         for (int r = 0; r < PER; ++r) {
             const int q = t + r * kTcThreads;
