@@ -146,11 +146,11 @@ __device__ void run_epi(const EpiArgs<S>& a, const S* v, bool bad) {
 
 // The slot-form products (hpb_bcg_slots.cu): k_spmv_dot and k_spmv_upd of
 // hpb_fused_bicgstabl.cu with the matrix as slots, element by element the same
-// operations.  xr null: the operand is x itself, else x - beta u as there.
+// operations.  The first: y = A (r - beta u) and <w, y>, then the epilogue.
 template <class E>
-void launch_spmv_dot_slots(const SlotMat<E>& A, bool dot, int grid, cudaStream_t s, int32_t rows, const E* diag,
-                           const E* x, E* y, const E* w, typename acc_of<typename scalar_of<E>::type>::type* partials,
-                           unsigned int* ticket, int* badflag, EpiArgs<typename scalar_of<E>::type> ea, const E* xr);
+void launch_spmv_dot_slots(const SlotMat<E>& A, int grid, cudaStream_t s, int32_t rows, const E* diag, const E* u, E* y,
+                           const E* w, typename acc_of<typename scalar_of<E>::type>::type* partials,
+                           unsigned int* ticket, int* badflag, EpiArgs<typename scalar_of<E>::type> ea, const E* r);
 template <class E>
 void launch_spmv_upd_slots(const SlotMat<E>& A, int j, int L, int grid, cudaStream_t s, int32_t rows, const E* diag,
                            const Vecs<E>& V, E* x, const E* w, BcgState<typename scalar_of<E>::type>* st,

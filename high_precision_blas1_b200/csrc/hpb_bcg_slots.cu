@@ -21,36 +21,29 @@ namespace hpb {
 namespace fused {
 namespace {
 
-template <class E, bool DOT, bool UPD, int NS>
+template <class E, int NS>
 __global__ void __launch_bounds__(kThreads)
-k_spmv_dot_slots(int32_t rows, SlotMat<E> A, const E* __restrict__ diag, const E* __restrict__ x, E* __restrict__ y,
+k_spmv_dot_slots(int32_t rows, SlotMat<E> A, const E* __restrict__ diag, const E* __restrict__ u, E* __restrict__ y,
                  const E* __restrict__ w, typename acc_of<typename scalar_of<E>::type>::type* partials,
-                 unsigned int* ticket, int* badflag, EpiArgs<typename scalar_of<E>::type> ea, const E* __restrict__ xr) {
+                 unsigned int* ticket, int* badflag, EpiArgs<typename scalar_of<E>::type> ea, const E* __restrict__ rr) {
     using S = typename scalar_of<E>::type;
     using AC = typename acc_of<S>::type;
     typename pacc_of<E>::type pacc;
-    S nb = s_zero(S{});
-    if (UPD) nb = s_neg(ea.st->beta);
+    const S nb = s_neg(ea.st->beta);
     constexpr int XL = LM_ALIGNED;
     const int32_t stride = gridDim.x * kThreads;
     for (int32_t r = blockIdx.x * kThreads + threadIdx.x; r < rows; r += stride) {
-        SlotRow<E, NS, typename std::conditional<UPD, SlotFma<E>, SlotX<E>>::type> row;
-        E we{};
-        if (DOT) we = ldE(w, r);
-        if constexpr (UPD)
-            row.load(A, rows, r, [&](int32_t c) { return SlotFma<E>{ld_x<XL>(x, c), ld_x<XL>(xr, c), nb}; });
-        else
-            row.load(A, rows, r, [&](int32_t c) { return SlotX<E>{ldgE(x, c)}; });
+        SlotRow<E, NS, SlotFma<E>> row;
+        const E we = ldE(w, r);
+        row.load(A, rows, r, [&](int32_t c) { return SlotFma<E>{ld_x<XL>(u, c), ld_x<XL>(rr, c), nb}; });
         S acc = row.sum(s_zero(S{}));
         if (diag) acc = s_div(acc, to_s(ldE(diag, r)));
         const E out = from_s<E>(acc);
         stE(y, r, out);
-        if (DOT) pdot_add(pacc, we, out);
+        pdot_add(pacc, we, out);
     }
-    if (DOT) {
-        AC dacc[1] = {widen_acc(pacc)};
-        grid_finish<1>(dacc, false, partials, ticket, badflag, [&](const S* v, bool bad) { run_epi(ea, v, bad); });
-    }
+    AC dacc[1] = {widen_acc(pacc)};
+    grid_finish<1>(dacc, false, partials, ticket, badflag, [&](const S* v, bool bad) { run_epi(ea, v, bad); });
 }
 
 template <class E, int J, bool MR, int NS>
@@ -147,17 +140,12 @@ void with_step(int j, F f) {
 }  // namespace
 
 template <class E>
-void launch_spmv_dot_slots(const SlotMat<E>& A, bool dot, int grid, cudaStream_t s, int32_t rows, const E* diag,
-                           const E* x, E* y, const E* w, typename acc_of<typename scalar_of<E>::type>::type* partials,
-                           unsigned int* ticket, int* badflag, EpiArgs<typename scalar_of<E>::type> ea, const E* xr) {
+void launch_spmv_dot_slots(const SlotMat<E>& A, int grid, cudaStream_t s, int32_t rows, const E* diag, const E* u, E* y,
+                           const E* w, typename acc_of<typename scalar_of<E>::type>::type* partials,
+                           unsigned int* ticket, int* badflag, EpiArgs<typename scalar_of<E>::type> ea, const E* r) {
     with_slots(A.ns, [&](auto nsc) {
         constexpr int NS = decltype(nsc)::value;
-        if (dot && xr)
-            k_spmv_dot_slots<E, true, true, NS><<<grid, kThreads, 0, s>>>(rows, A, diag, x, y, w, partials, ticket, badflag,
-                                                                          ea, xr);
-        else
-            k_spmv_dot_slots<E, false, false, NS><<<grid, kThreads, 0, s>>>(rows, A, diag, x, y, w, partials, ticket,
-                                                                            badflag, ea, xr);
+        k_spmv_dot_slots<E, NS><<<grid, kThreads, 0, s>>>(rows, A, diag, u, y, w, partials, ticket, badflag, ea, r);
     });
 }
 
@@ -195,7 +183,7 @@ int spmv_upd_slots_occupancy(int ns, int j, int L) {
 }
 
 #define HPB_BCG_SLOTS(E)                                                                                                 \
-    template void launch_spmv_dot_slots<E>(const SlotMat<E>&, bool, int, cudaStream_t, int32_t, const E*, const E*, E*, \
+    template void launch_spmv_dot_slots<E>(const SlotMat<E>&, int, cudaStream_t, int32_t, const E*, const E*, E*,       \
                                            const E*, acc_of<scalar_of<E>::type>::type*, unsigned int*, int*,            \
                                            EpiArgs<scalar_of<E>::type>, const E*);                                      \
     template void launch_spmv_upd_slots<E>(const SlotMat<E>&, int, int, int, cudaStream_t, int32_t, const E*,           \

@@ -780,8 +780,8 @@ int BcgPlan<E>::init(const hpb_solver_params* p, int32_t rows, int64_t nnz, cons
         // u_{j+1} = A (r_j - beta u_j) and alpha = rho / <rt, u_{j+1}>
         const EpiArgs<S> alpha{st, drep, EPI_ALPHA, 0, j, L};
         if (P.slots.ns)
-            launch_spmv_dot_slots<E>(P.slots, true, g_spd, s, rows, diag, V.u[j], V.u[j + 1], rt, partials, ticket,
-                                     badflag, alpha, V.r[j]);
+            launch_spmv_dot_slots<E>(P.slots, g_spd, s, rows, diag, V.u[j], V.u[j + 1], rt, partials, ticket, badflag,
+                                     alpha, V.r[j]);
         else
             launch_spmv_dot<E, true, true>(lm, g_spd, s, rows, rp, ci, val, diag, V.u[j], V.u[j + 1], rt, partials,
                                            ticket, badflag, alpha, V.r[j]);

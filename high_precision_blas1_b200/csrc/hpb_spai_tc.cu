@@ -196,7 +196,7 @@ __device__ __forceinline__ void load_feat(const float* __restrict__ feat, int32_
 // one rounding a feature.  Training keeps the binary32 arithmetic of the CSR
 // path's k_features, operation by operation.
 template <bool TABLES>
-struct SlotRow {
+struct FeatureRow {
     float a[kMaxSlot];
     typename std::conditional<TABLES, double, float>::type sj[kMaxSlot], lj[TABLES ? kMaxSlot : 1];
     unsigned m;
@@ -208,7 +208,7 @@ struct SlotArgs {
     float *ah, *feat;
 };
 template <bool TABLES, int NS, int DS>
-__device__ __forceinline__ void load_slots(const SlotArgs& g, int32_t row, SlotRow<TABLES>& r) {
+__device__ __forceinline__ void load_slots(const SlotArgs& g, int32_t row, FeatureRow<TABLES>& r) {
     const int ns = NS ? NS : g.nslot;
     r.m = 0u;
     if (row >= g.sys.n) return;
@@ -228,7 +228,7 @@ __device__ __forceinline__ void load_slots(const SlotArgs& g, int32_t row, SlotR
         }
 }
 template <bool TABLES, int NS, int DS>
-__device__ __forceinline__ void slot_features(const SlotArgs& g, int32_t row, const SlotRow<TABLES>& r, double mean,
+__device__ __forceinline__ void slot_features(const SlotArgs& g, int32_t row, const FeatureRow<TABLES>& r, double mean,
                                               float (&x)[kF]) {
     const int ns = NS ? NS : g.nslot, ds = NS ? DS : g.dslot;
 #pragma unroll
@@ -367,7 +367,7 @@ k_forward_tc(int32_t rows, const float* __restrict__ feat, SlotArgs g, const uns
     bool failed = false;
     const int32_t ntiles = (rows + kTile - 1) / kTile;
     float xf[kF];
-    SlotRow<TABLES> sr;
+    FeatureRow<TABLES> sr;
     double mean = 0.0;
     if constexpr (SLOTS) {
         mean = __ldg(g.sys.lsum) / double(rows > 1 ? rows : 1);

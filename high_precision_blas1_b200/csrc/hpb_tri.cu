@@ -340,95 +340,95 @@ k_tri_levels(int32_t n, int32_t ntiles, const int32_t* __restrict__ ci, const in
     }
     more = __syncthreads_or(more);
     if (more) {  // ---- rows with more dependents: a list by offsets
-    // exclusive scan of off: kTriTile / kGlThreads entries per thread
-    {
-        constexpr int P = kTriTile / kGlThreads;
-        int v[P], s = 0;
+        // exclusive scan of off: kTriTile / kGlThreads entries per thread
+        {
+            constexpr int P = kTriTile / kGlThreads;
+            int v[P], s = 0;
 #pragma unroll
-        for (int k = 0; k < P; ++k) {
-            v[k] = T.off[tid * P + k];
-            s += v[k];
-        }
-        int x = s;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, d);
-            if (lane >= d) x += y;
-        }
-        if (lane == 31) T.scan[warp] = x;
-        __syncthreads();
-        if (warp == 0) {
-            const int ws = T.scan[lane];
-            int y = ws;
+            for (int k = 0; k < P; ++k) {
+                v[k] = T.off[tid * P + k];
+                s += v[k];
+            }
+            int x = s;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
-                const int z = __shfl_up_sync(0xffffffffu, y, d);
-                if (lane >= d) y += z;
+                const int y = __shfl_up_sync(0xffffffffu, x, d);
+                if (lane >= d) x += y;
             }
-            T.scan[lane] = y - ws;
-            if (lane == 31) T.edges = y;
+            if (lane == 31) T.scan[warp] = x;
+            __syncthreads();
+            if (warp == 0) {
+                const int ws = T.scan[lane];
+                int y = ws;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int z = __shfl_up_sync(0xffffffffu, y, d);
+                    if (lane >= d) y += z;
+                }
+                T.scan[lane] = y - ws;
+                if (lane == 31) T.edges = y;
+            }
+            __syncthreads();
+            int acc = T.scan[warp] + x - s;
+#pragma unroll
+            for (int k = 0; k < P; ++k) {
+                T.off[tid * P + k] = acc;
+                acc += v[k];
+            }
         }
         __syncthreads();
-        int acc = T.scan[warp] + x - s;
-#pragma unroll
-        for (int k = 0; k < P; ++k) {
-            T.off[tid * P + k] = acc;
-            acc += v[k];
+        if (T.edges > kMaxEdges) {  // ---- relaxation sweeps
+            volatile int* lev = T.lev;
+            int* ext = T.left;
+            for (int r = tid; r < m; r += kGlThreads) {  // 1 + the largest level from outside the tile
+                const int32_t i = base + r, b = __ldg(beg + i), c = __ldg(cnt + i);
+                int e = 0;
+                for (int32_t k = b; k < b + c; ++k) {
+                    const int32_t j = __ldg(ci + k), jl = j - base;
+                    if (!is_dep<UPPER>(n, i, j) || (jl >= 0 && jl < m)) continue;
+                    Waiter w;
+                    int v;
+                    while ((v = int(ld_relaxed32(glev + j))) < 0)
+                        if (w.check(err, 63)) break;
+                    e = max(e, v + 1);
+                }
+                ext[r] = e;
+                lev[r] = e;
+            }
+            __syncthreads();
+            // contiguous segments walked in dependency order until a sweep
+            // changes nothing (a sweep that changes something brings one more row
+            // of the longest in-tile chain to its final value)
+            const int seg = (m + kGlThreads - 1) / kGlThreads;
+            const int s0 = min(m, tid * seg), s1 = min(m, s0 + seg);
+            int changed, sweeps = 0;
+            do {
+                changed = 0;
+                for (int k = 0; k < s1 - s0; ++k) {
+                    const int r = UPPER ? s1 - 1 - k : s0 + k;
+                    const int32_t i = base + r, b = __ldg(beg + i), c = __ldg(cnt + i);
+                    int lv = ext[r];
+                    for (int32_t e = b; e < b + c; ++e) {
+                        const int32_t j = __ldg(ci + e), jl = j - base;
+                        if (is_dep<UPPER>(n, i, j) && jl >= 0 && jl < m) lv = max(lv, lev[jl] + 1);
+                    }
+                    if (lv > lev[r]) {
+                        lev[r] = lv;
+                        changed = 1;
+                    }
+                }
+            } while (__syncthreads_or(changed) && ++sweeps <= m);
+            for (int r = tid; r < m; r += kGlThreads) st_relaxed32(glev + base + r, unsigned(lev[r]));
+            return;
         }
-    }
-    __syncthreads();
-    if (T.edges > kMaxEdges) {  // ---- relaxation sweeps
-        volatile int* lev = T.lev;
-        int* ext = T.left;
-        for (int r = tid; r < m; r += kGlThreads) {  // 1 + the largest level from outside the tile
+        for (int r = tid; r < m; r += kGlThreads) {
             const int32_t i = base + r, b = __ldg(beg + i), c = __ldg(cnt + i);
-            int e = 0;
             for (int32_t k = b; k < b + c; ++k) {
                 const int32_t j = __ldg(ci + k), jl = j - base;
-                if (!is_dep<UPPER>(n, i, j) || (jl >= 0 && jl < m)) continue;
-                Waiter w;
-                int v;
-                while ((v = int(ld_relaxed32(glev + j))) < 0)
-                    if (w.check(err, 63)) break;
-                e = max(e, v + 1);
+                if (is_dep<UPPER>(n, i, j) && jl >= 0 && jl < m) T.to[atomicAdd(&T.off[jl], 1)] = uint16_t(r);
             }
-            ext[r] = e;
-            lev[r] = e;
         }
-        __syncthreads();
-        // contiguous segments walked in dependency order until a sweep
-        // changes nothing (a sweep that changes something brings one more row
-        // of the longest in-tile chain to its final value)
-        const int seg = (m + kGlThreads - 1) / kGlThreads;
-        const int s0 = min(m, tid * seg), s1 = min(m, s0 + seg);
-        int changed, sweeps = 0;
-        do {
-            changed = 0;
-            for (int k = 0; k < s1 - s0; ++k) {
-                const int r = UPPER ? s1 - 1 - k : s0 + k;
-                const int32_t i = base + r, b = __ldg(beg + i), c = __ldg(cnt + i);
-                int lv = ext[r];
-                for (int32_t e = b; e < b + c; ++e) {
-                    const int32_t j = __ldg(ci + e), jl = j - base;
-                    if (is_dep<UPPER>(n, i, j) && jl >= 0 && jl < m) lv = max(lv, lev[jl] + 1);
-                }
-                if (lv > lev[r]) {
-                    lev[r] = lv;
-                    changed = 1;
-                }
-            }
-        } while (__syncthreads_or(changed) && ++sweeps <= m);
-        for (int r = tid; r < m; r += kGlThreads) st_relaxed32(glev + base + r, unsigned(lev[r]));
-        return;
-    }
-    for (int r = tid; r < m; r += kGlThreads) {
-        const int32_t i = base + r, b = __ldg(beg + i), c = __ldg(cnt + i);
-        for (int32_t k = b; k < b + c; ++k) {
-            const int32_t j = __ldg(ci + k), jl = j - base;
-            if (is_dep<UPPER>(n, i, j) && jl >= 0 && jl < m) T.to[atomicAdd(&T.off[jl], 1)] = uint16_t(r);
-        }
-    }
-    __syncthreads();  // off[r] is now the end of row r's part, its start the end of row r - 1's
+        __syncthreads();  // off[r] is now the end of row r's part, its start the end of row r - 1's
     }
 
     if (warp == 0) {  // ---- the queue
