@@ -500,7 +500,7 @@ def gmres_cycle_bytes(n, nnz, m, elem=4, idx=4):
     return total
 
 
-def bicgstabl_cycle_bytes(n, nnz, L, elem=8):
+def bicgstabl_cycle_bytes(n, nnz, L, elem=8, slots=0):
     """Algorithmic HBM bytes of one fused BiCGStab(L) cycle: 2L SpMVs (2L-1
     with the Dot2 against rt; the L products of r_j - beta u_j gather both
     vectors, and so do the L products of r_j - alpha u_{j+1}), the BiCG
@@ -509,8 +509,9 @@ def bicgstabl_cycle_bytes(n, nnz, L, elem=8):
     modified Gram-Schmidt sweeps and the closing update, each vector read or
     written once per kernel.  The first MGS sweep's inner products are formed
     by the last step's kernel from the values it holds (no pass of their
-    own)."""
-    mat = (elem + 4.0) * nnz + 4.0 * (n + 1)
+    own).  slots: the matrix in slot form with that many slots (at least five
+    are held), a value in each and a byte of mask per row, instead of CSR."""
+    mat = (elem * max(slots, 5) + 1.0) * n if slots else (elem + 4.0) * nnz + 4.0 * (n + 1)
     spmv = mat + 2.0 * elem * n
     vec = elem * float(n)
     passes = L                                             # r_j gathered beside u_j by A (r_j - beta u_j)
@@ -628,16 +629,17 @@ def bench_solver(args, ws, rank, local, torch, dist):
 
 
 def solver_roofline(A, iters, t_step, plain):
-    """Whole-solve HBM roofline of the fused BiCGStab(L): algorithmic bytes
-    per cycle x cycles / solve time (the plain path moves more: its
-    reductions and updates are separate kernels)."""
+    """Whole-solve HBM roofline of the fused BiCGStab(L), which holds the
+    five-point matrix in slot form: algorithmic bytes per cycle x cycles /
+    solve time (the plain path moves more: its reductions and updates are
+    separate kernels, its matrix is CSR)."""
     cycles = iters[-1] // SOLVER_L
-    per_cycle = bicgstabl_cycle_bytes(A.n, A.nnz, SOLVER_L)
+    per_cycle = bicgstabl_cycle_bytes(A.n, A.nnz, SOLVER_L, slots=0 if plain else 5)
     hbm, src = peaks()
     ach = per_cycle * cycles / t_step / 1e9
     return {"bytes_per_cycle": per_cycle, "cycles": cycles, "achieved": ach, "peak": hbm, "peak_source": src,
             "unit": "GB/s", "frac": ach / hbm, "bound_s": per_cycle * cycles / (hbm * 1e9),
-            "note": "fused-path byte model" + (" (timed path is the plain one)" if plain else "")}
+            "note": "fused-path byte model" + (" (CSR; timed path is the plain one)" if plain else ", matrix in slot form")}
 
 
 # ------------------------------------------------ precision / complex / learned forms
@@ -1099,15 +1101,18 @@ def dot2_same_box(torch, L, ctx, calls=200):
 def dot2_floors(torch, L, ctx, xs, ys, n, calls=200):
     """What bounds one launch at 16.8 MB: back-to-back launches of a library
     kernel with no work (hpb_fill_f64 of one element, an ordinary launch),
-    the Dot2 kernel itself with n = 0 (a programmatic launch and the
-    combine, nothing to read), the plain FMA dot over the same pair
-    (hpb_dot_f64: the same single-pass combine without the error-free
-    transformations), beside Dot2."""
+    Dot2 with n = 0 (one block, nothing to read or merge), Dot2 of the
+    shortest vector that takes several blocks (the programmatic launch, the
+    ticket and the last block's combine, as at n, with 115 KB to read), the
+    plain FMA dot over the same pair (hpb_dot_f64: the same single-pass
+    combine without the error-free transformations), beside Dot2."""
     R = len(xs)
     one = torch.zeros(1, dtype=torch.float64, device="cuda")
     od = torch.zeros(4, dtype=torch.float64, device="cuda")
     t_launch = _events_us(torch, lambda i: L.hpb_fill_f64(ctx.h, 1, 0.0, one.data_ptr()), calls)
-    # the same Dot2 kernel with nothing to read: launch (programmatic, as every Dot2) + one block's combine
+    few = 2 * 4096 + 2  # binary64 elements: one 16-byte pack more than one block takes
+    t_few = _events_us(torch, lambda i: L.hpb_dot2_f64(ctx.h, few, xs[0].data_ptr(), ys[0].data_ptr(),
+                                                       od.data_ptr()), calls)
     t_empty = _events_us(torch, lambda i: L.hpb_dot2_f64(ctx.h, 0, xs[0].data_ptr(), ys[0].data_ptr(),
                                                          od.data_ptr()), calls)
     t_plain = _events_us(torch, lambda i: L.hpb_dot_f64(ctx.h, n, xs[i % R].data_ptr(), ys[i % R].data_ptr(),
@@ -1115,7 +1120,7 @@ def dot2_floors(torch, L, ctx, xs, ys, n, calls=200):
     t_dot2 = _events_us(torch, lambda i: L.hpb_dot2_f64(ctx.h, n, xs[i % R].data_ptr(), ys[i % R].data_ptr(),
                                                         od.data_ptr()), calls)
     hbm, _ = peaks()
-    return {"launch_floor_us": t_launch, "dot2_n0_us": t_empty, "plain_dot_us": t_plain, "dot2_us": t_dot2,
+    return {"launch_floor_us": t_launch, "dot2_n0_us": t_empty, "dot2_few_blocks_us": t_few, "plain_dot_us": t_plain, "dot2_us": t_dot2,
             "transfer_at_peak_us": 16.0 * n / (hbm * 1e9) * 1e6,
             "note": "one launch at 16.8 MB: launch floor + HBM transfer at the measured peak bound a single-pass "
                     "reduction from below; the plain dot shows what the compensation itself costs"}
