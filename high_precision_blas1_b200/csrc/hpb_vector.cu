@@ -111,11 +111,14 @@ constexpr int kMapThreads = 256;
 // four packs a thread gave 102 and 104 us of the 101; one block for every 256
 // packs 103 us, 512 threads 102 us, 128 threads 104 us.  The programmatic
 // launch overlaps the start of a call with the end of the one before: f64
-// axpy on 1 M 6.2 -> 4.0 us a call in a row of calls.
+// axpy on 1 M 6.2 -> 3.8 us a call in a row of calls.  The call behind is let in
+// when a block is done: with it let in first, calls in a captured graph on
+// vectors of a few hundred thousand entries took up to 1.2 times as long as
+// ordinary launches there (c64 lincomb4 on 300,000 3.0 -> 3.6 us; now 2.8).
 template <class E, class F, int NIN, bool VEC>
 __global__ void __launch_bounds__(kMapThreads)
 map_kernel(int64_t n, F f, const E* a0, const E* a1, const E* a2, const E* a3, E* z) {
-    pdl_enter_for(a0, a1, a2, a3, z);
+    pdl_wait_for(a0, a1, a2, a3, z);
     const int64_t gtid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     if (VEC) {
@@ -152,6 +155,7 @@ map_kernel(int64_t n, F f, const E* a0, const E* a1, const E* a2, const E* a3, E
             stE(z, i, f(e0, e1, e2, e3));
         }
     }
+    pdl_trigger();
 }
 
 inline bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -175,8 +179,14 @@ int launch_map(hpb_context* ctx, int64_t n, F f, const E* a0, const E* a1, const
     if (bits % kElemAlign != 0)
         return set_error(ctx, HPB_ERROR_INVALID_VALUE, "%s: pointer not aligned to its element type", name);
     const int K = aligned ? VK<E>::k : 1;
-    // more blocks than are resident (the kernel's comment has both sides)
-    int grid = grid_for(ctx, (n + K - 1) / K, kMapThreads, 32);
+    // More blocks than are resident (the kernel's comment has both sides), in
+    // whole waves: where a block for every 256 packs makes fewer than two or four
+    // waves, one or two of them (in a captured graph on B200, one, two and four
+    // waves: f64 axpy on 1 M 3.70, 3.94, 3.94 us, on 2 M 6.20, 5.77, 6.49; c128 axpy
+    // on 1 M 4.85, 4.54, 5.13; c64 axpy on 3 M 13.4, 11.4, 11.0).
+    const int64_t blocks = ((n + K - 1) / K + kMapThreads - 1) / kMapThreads;
+    const int waves = blocks <= int64_t(16) * ctx->num_sms ? 1 : blocks <= int64_t(32) * ctx->num_sms ? 2 : 4;
+    int grid = grid_for(ctx, (n + K - 1) / K, kMapThreads, 8 * waves);
     if (aligned)
         launch_pdl(ctx->stream, grid, kMapThreads, map_kernel<E, F, NIN, true>, n, f, a0, a1, a2, a3, z);
     else
