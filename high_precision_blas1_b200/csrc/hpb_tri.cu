@@ -1008,6 +1008,72 @@ __device__ __forceinline__ void solve_steps(const RowData<E>& r, const Prep<E>& 
     }
 }
 
+// The chain of one chunk in which rows have more than kPre dependencies: the
+// sources and values of the next kMore, and other tiles' values, are taken in
+// before the turn.  (Looked up during it -- column, position, value one after
+// another, other tiles' rows one by one from L2 -- they were most of a solve:
+// lower / upper, ILU(0) on B200, f64 27-point 64^3 4964 / 5347 -> 932 / 1067 us,
+// 13-point 500^2 2022 / 2785 -> 1085 / 1231, f32 27-point 64^3 3500 / 4103 ->
+// 705 / 905.)
+// A function of its own: inside the kernel it cost the rows of at most kPre
+// dependencies 3 % of the lower solve (321 -> 330 us at 1024^2).
+template <class E, bool UNIT>
+__device__ __noinline__ void long_rows(RowData<E> r, Prep<E> prep, int w, int lane, int steps, int mine, bool publish,
+                                       int from, int to, int32_t base, int32_t m, const int32_t* __restrict__ ci,
+                                       const uint16_t* __restrict__ pos, const E* __restrict__ val, E* x, int* err,
+                                       unsigned long long lim) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    TileValues<E>& T = *reinterpret_cast<TileValues<E>*>(smraw);
+    const E* src[kPre];
+#pragma unroll
+    for (int k = 0; k < kPre; ++k) {
+        const int sk = at4(r.s, k);
+        src[k] = sk >= 0 ? T.xs + sk : &T.ext[w][k][lane];
+    }
+    int ms[kMore];
+    E mv[kMore], mx[kMore];
+#pragma unroll
+    for (int k = 0; k < kMore; ++k) {
+        ms[k] = -1;
+        if (kPre + k < r.d.z) {
+            const int32_t e = r.d.y + kPre + k, j = __ldg(ci + e), jl = j - base;
+            mv[k] = ldE(val, e);
+            if (jl >= 0 && jl < m)
+                ms[k] = __ldg(pos + j);
+            else
+                mx[k] = Pub<E>::load(x, j);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kMore; ++k)
+        if (kPre + k < r.d.z && ms[k] < 0 && Pub<E>::pending(mx[k]))
+            mx[k] = await_value(x, __ldg(ci + (r.d.y + kPre + k)), mx[k], err, lim);
+    __syncwarp();
+    if (from >= 0) chunk_sync(from);
+    for (int l = 1; l <= steps; ++l) {
+        if (mine == l) {
+            E acc = r.rhs;
+#pragma unroll
+            for (int k = 0; k < kPre; ++k)
+                if (k < r.d.z) acc = fms(acc, r.v[k], *src[k]);
+#pragma unroll
+            for (int k = 0; k < kMore; ++k)
+                if (kPre + k < r.d.z) acc = fms(acc, mv[k], ms[k] >= 0 ? T.xs[ms[k]] : mx[k]);
+            for (int32_t e = r.d.y + kPre + kMore; e < r.d.y + r.d.z; ++e) {
+                const int32_t j = __ldg(ci + e), jl = j - base;
+                const E xv = (jl >= 0 && jl < m) ? T.xs[__ldg(pos + j)]
+                                                 : await_value(x, j, Pub<E>::load(x, j), err, lim);
+                acc = fms(acc, ldE(val, e), xv);
+            }
+            if (!UNIT) acc = quot_prepared(acc, r.dg, prep, true);
+            T.xs[r.first + lane] = acc;
+            if (publish) Pub<E>::store(x, r.d.x, acc);
+        }
+        __syncwarp();
+    }
+    if (to >= 0) chunk_arrive(to);
+}
+
 template <class E, bool UPPER, bool UNIT>
 __global__ void __launch_bounds__(kSolveThreads, 1)
 k_trsv(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int4* __restrict__ dsrc,
@@ -1089,55 +1155,8 @@ k_trsv(int32_t n, int32_t ntiles, const int4* __restrict__ desc, const int4* __r
             case 2: solve_steps<E, UNIT, 2>(r, prep, src, out, steps, mine, publish, xo, from, to); break;
             case 3: solve_steps<E, UNIT, 3>(r, prep, src, out, steps, mine, publish, xo, from, to); break;
             case 4: solve_steps<E, UNIT, 4>(r, prep, src, out, steps, mine, publish, xo, from, to); break;
-            default: {  // rows with more than kPre dependencies among them
-                // The next kMore: sources and values, and other tiles' values, before the
-                // turn.  (Looked up during it -- column, position, value one after another,
-                // other tiles' rows one by one from L2 -- they were most of a solve: lower /
-                // upper, ILU(0) on B200, f64 27-point 64^3 4964 / 5347 -> 708 / 803 us, 13-point
-                // 500^2 2022 / 2785 -> 801 / 913, f32 27-point 64^3 3500 / 4103 -> 628 / 748.)
-                int ms[kMore];
-                E mv[kMore], mx[kMore];
-#pragma unroll
-                for (int k = 0; k < kMore; ++k) {
-                    ms[k] = -1;
-                    if (kPre + k < r.d.z) {
-                        const int32_t e = r.d.y + kPre + k, j = __ldg(ci + e), jl = j - base;
-                        mv[k] = ldE(val, e);
-                        if (jl >= 0 && jl < m)
-                            ms[k] = __ldg(pos + j);
-                        else
-                            mx[k] = Pub<E>::load(x, j);
-                    }
-                }
-#pragma unroll
-                for (int k = 0; k < kMore; ++k)
-                    if (kPre + k < r.d.z && ms[k] < 0 && Pub<E>::pending(mx[k]))
-                        mx[k] = await_value(x, __ldg(ci + (r.d.y + kPre + k)), mx[k], err, lim);
-                __syncwarp();
-                if (from >= 0) chunk_sync(from);
-                for (int l = 1; l <= steps; ++l) {
-                    if (mine == l) {
-                        E acc = r.rhs;
-#pragma unroll
-                        for (int k = 0; k < kPre; ++k)
-                            if (k < r.d.z) acc = fms(acc, r.v[k], *src[k]);
-#pragma unroll
-                        for (int k = 0; k < kMore; ++k)
-                            if (kPre + k < r.d.z) acc = fms(acc, mv[k], ms[k] >= 0 ? T.xs[ms[k]] : mx[k]);
-                        for (int32_t e = r.d.y + kPre + kMore; e < r.d.y + r.d.z; ++e) {
-                            const int32_t j = __ldg(ci + e), jl = j - base;
-                            const E xv = (jl >= 0 && jl < m) ? T.xs[__ldg(pos + j)]
-                                                             : await_value(x, j, Pub<E>::load(x, j), err, lim);
-                            acc = fms(acc, ldE(val, e), xv);
-                        }
-                        if (!UNIT) acc = quot_prepared(acc, r.dg, prep, true);
-                        *out = acc;
-                        if (publish) Pub<E>::store(xo, 0, acc);
-                    }
-                    __syncwarp();
-                }
-                if (to >= 0) chunk_arrive(to);
-            }
+            default:  // rows with more than kPre dependencies among them
+                long_rows<E, UNIT>(r, prep, w, lane, steps, mine, publish, from, to, base, m, ci, pos, val, x, err, lim);
         }
         r = nx;
         nx = nn;
