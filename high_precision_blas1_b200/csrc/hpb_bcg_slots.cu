@@ -81,9 +81,8 @@ k_spmv_upd_slots(int32_t rows, SlotMat<E> A, const E* __restrict__ diag, Vecs<E>
         if (J >= 1) r[J - 1] = round_s<E>(s_fma(nalp, u[J], r[J - 1]));
 #pragma unroll
         for (int i = 0; i <= J; ++i) {
-            const S t = s_fma(nb, u[i], r[i]);
-            u[i] = round_s<E>(t);
-            stE(V.u[i], q, from_s<E>(t));
+            u[i] = round_s<E>(s_fma(nb, u[i], r[i]));
+            stE(V.u[i], q, from_s<E>(u[i]));
         }
 #pragma unroll
         for (int i = 0; i < J; ++i) {

@@ -278,9 +278,8 @@ __device__ __forceinline__ void mgs_rows(int64_t q, int k, bool upd, const Vecs<
             if constexpr (NV >= 2) {
                 ve[NV - 2][j] = from_s<E>(s_fma(nal, uq, to_s(ve[NV - 2][j])));
             } else {
-                const S t = s_fma(nal, uq, pv);
-                pv = round_s<E>(t);
-                pe[j] = from_s<E>(t);
+                pv = round_s<E>(s_fma(nal, uq, pv));
+                pe[j] = from_s<E>(pv);
             }
         }
         if (upd)
