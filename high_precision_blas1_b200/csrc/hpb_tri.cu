@@ -845,14 +845,14 @@ __global__ void k_tri_fill(int32_t n, E* __restrict__ x, unsigned* ticket) {
 // row's FMAs and a shared store (and, at a non-unit diagonal, a division),
 // whatever the number of rows up to 32; wider levels take several chunks.
 // Measured on B200 (f64, ILU(0) factors of the 1024^2 5-point operator, 2047
-// levels in 128 tiles): lower + upper solve 902 us with fifteen warps,
-// 972 us with chunks of 32 that cut levels in two, and 2460 us for levels handed round 15 warps one by
-// one with a receiver warp for the other tiles' values.  One tile of 1024 x 8
-// points, 1031 levels, takes 73 / 134 us and each further one 2.2 / 3.1 us:
-// the eight levels it starts later, a chunk's worth of waiting and a value's
-// way to L2 and back.  (Polling the other tiles' values in the shared memory of
-// a cluster's blocks instead of L2 took 0.3 us off a tile, 998 against 1011 us
-// in all, and was not worth its code.)
+// levels in 128 tiles): lower + upper solve 826 us; with fifteen warps instead
+// of seven 902 us, and with these 972 us with chunks of 32 that cut levels in
+// two and 2460 us for levels handed round the warps one by one with a receiver
+// warp for the other tiles' values.  One tile of 1024 x 8 points, 1031 levels,
+// takes 66 / 129 us and each further one 2.0 / 3.0 us: the eight levels it
+// starts later, a chunk's worth of waiting and a value's way to L2 and back.
+// (Polling the other tiles' values in the shared memory of a cluster's blocks
+// instead of L2 took 0.3 us off a tile and was not worth its code.)
 // (A solver warp fed through a shared-memory ring by the others was slower,
 // 480 / 719 us: about 500 cycles a chunk went into taking over the records.)
 // A division by the diagonal sits on the chain, so the loader prepares it:
@@ -1211,7 +1211,7 @@ k_tri_sweep(int32_t n, const int32_t* __restrict__ rp, const int32_t* __restrict
 // chunks of the level order, d by position in shared memory and published
 // once to a sentinel-filled array for the other tiles.  The operations are
 // those of the general kernel (k_ilu0) in the same order, so the same bits.
-// Measured on B200 (f64, 1024^2 5-point operator): 1.45 ms with its pattern
+// Measured on B200 (f64, 1024^2 5-point operator): 1.22 ms with its pattern
 // check, against 15.6 ms for the general kernel, whose every level (7.6 us) is a chain of
 // dependent loads from L2 and fences.
 // k_ilu0_pattern finds for each of a row's first kPre dependencies where row
