@@ -688,15 +688,10 @@ int BcgPlan<E>::init(const hpb_solver_params* p, int32_t rows, int64_t nnz, cons
     P.g_red = int(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * reduction_occupancy<E>(L))));
     P.g_sp = int(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * 8)));  // grid-stride rows, 8 blocks per SM
     P.g_spd = int(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * 6)));
-    // the update + product's grids on the CSR and on the slots, of which one is
-    // taken when it is known whether there are slots
+    // the update + product's grids follow when it is known whether there are
+    // slots; their partials are sized for as many blocks as any kernel has resident
     auto su_grid = [&](int cap) { return int(std::max<int64_t>(1, std::min<int64_t>(need, int64_t(sms) * cap))); };
-    int g_su_max = 1;
-    for (int j = 0; j < L; ++j) {
-        P.g_su[j] = su_grid(std::min(6, spmv_upd_occupancy<E>(j, L)));
-        g_su_max = std::max(g_su_max, P.g_su[j]);
-        for (int ns : {5, kMaxSlots}) g_su_max = std::max(g_su_max, su_grid(spmv_upd_slots_occupancy<E>(ns, j, L)));
-    }
+    const int g_su_max = su_grid(2048 / kThreads);
     P.g_nrm = int(std::max<int64_t>(
         1, std::min<int64_t>(need, int64_t(sms) * occupancy_of(reinterpret_cast<const void*>(k_norm<E>)))));
     const int g_ew = P.g_ew, g_red = P.g_red, g_sp = P.g_sp, g_spd = P.g_spd;
@@ -736,8 +731,10 @@ int BcgPlan<E>::init(const hpb_solver_params* p, int32_t rows, int64_t nnz, cons
     }
     if (cudaStreamSynchronize(s) != cudaSuccess || make_slots<E>(ws, rows, nnz, rp, ci, val, offs, &P.slots) != HPB_SUCCESS)
         return HPB_ERROR_CUDA;
-    if (P.slots.ns > 0)
-        for (int j = 0; j < L; ++j) P.g_su[j] = su_grid(spmv_upd_slots_occupancy<E>(P.slots.ns, j, L));
+    for (int j = 0; j < L; ++j) {
+        const int occ = P.slots.ns ? spmv_upd_slots_occupancy<E>(P.slots.ns, j, L) : std::min(6, spmv_upd_occupancy<E>(j, L));
+        P.g_su[j] = std::min(g_su_max, su_grid(occ));
+    }
 
     // ---- one cycle as a CUDA graph
     BcgState<S>* st = P.st;
